@@ -1,7 +1,8 @@
 // Per-cell building blocks of the stream-collide kernels and the kernel
-// templates built from them: the one-cell-per-thread kernels (per row and
-// over the flattened lattice), the fine collide with the restriction's child
-// sums fused in, the staged kernel that streams x-rows through shared memory
+// templates built from them: the one-cell-per-thread kernel over the
+// flattened lattice, its form for 16-bit populations with tiles staged through
+// shared memory, the fine collide with the restriction's child sums fused in,
+// the staged kernel that streams x-rows through shared memory
 // with bulk async copies, and the AA-pattern in-place kernels.
 //
 // Physics follows the reference step (src/sim/lbm_core.cu:213-475): per link
@@ -57,35 +58,34 @@ struct CollideArgs {
     const uint2* links;          // pull-link classes per cell (launch_classify), or null
 };
 
-/// Byte offsets of the pulls of an interior cell (no periodic wrap on any
-/// axis), from the cell's own slot in direction slice 0: pull[q] reaches the
-/// source x - c_q in slice q, slice[q] the cell itself in slice q. Passed as
-/// a __grid_constant__ kernel parameter, so each load and store of such a cell
-/// is one 64-bit add of a constant-bank operand to the cell's base pointer
-/// instead of a wrapped 3-D index and a slice product per direction.
-struct PullOffsets {
-    long long pull[kQ];
-    long long slice[kQ];
+/// Slice pointers of one launch, passed as a __grid_constant__ kernel
+/// parameter: pull[q][cell] is the source x - c_q of an interior cell (no
+/// periodic wrap on any axis) in slice q, own[q][cell] the cell itself in
+/// slice q of the source buffer, out[q][cell] in the destination. A load or
+/// store of such a cell is one 32 x 32 + 64-bit multiply-add of the cell index
+/// and a constant-bank pointer, where a wrapped 3-D index, a slice product or
+/// a 64-bit offset added to a base pointer each take more instructions.
+template <class T>
+struct SlicePtrs {
+    const T* pull[kQ];
+    const T* own[kQ];
+    T* out[kQ];
 };
 
 template <class T>
-__host__ PullOffsets pull_offsets(int nx, int ny, long long n) {
-    PullOffsets o;
+__host__ SlicePtrs<T> slice_ptrs(const T* src, T* dst, int nx, int ny, long long n) {
+    SlicePtrs<T> o;
     const long long sx = nx, sxy = static_cast<long long>(nx) * ny;
     for (int q = 0; q < kQ; ++q) {
-        o.slice[q] = q * n * static_cast<long long>(sizeof(T));
-        o.pull[q] = (q * n - (cx(q) + sx * cy(q) + sxy * cz(q))) * static_cast<long long>(sizeof(T));
+        o.own[q] = src + q * n;
+        o.out[q] = dst + q * n;
+        o.pull[q] = src + (q * n - (cx(q) + sx * cy(q) + sxy * cz(q)));
     }
     return o;
 }
 
-template <class T>
-__device__ __forceinline__ const T* byte_add(const T* p, long long b) {
-    return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + b);
-}
-template <class T>
-__device__ __forceinline__ T* byte_add(T* p, long long b) {
-    return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + b);
+__device__ __forceinline__ unsigned smem_addr(const void* p) {
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
 
 /// True when no pull of (x, y, z) wraps around a periodic axis.
@@ -150,41 +150,59 @@ __device__ __forceinline__ void eq19(float rho, float ux, float uy, float uz, fl
 }
 
 // ---- collision bodies ------------------------------------------------------
+// The exact body forms the reference's expressions with fewer operations
+// where the result is the same to the bit: sums start from their first term
+// instead of 0 (only the sign of a zero sum could differ, which nothing below
+// sees), the equilibria of an opposite pair share 0.5 (3 c.u)^2 (3 c.u changes
+// sign exactly), and the TRT halves are taken by scaling the rate
+// (multiplying by 0.5 is exact: omega (0.5 a - 0.5 b) = (0.5 omega)(a - b)).
 __device__ __forceinline__ void collide_exact(float (&f)[kQ], float tau0, float lambda, float smagPre,
                                               float& rhoO, float& uxO, float& uyO, float& uzO) {
-    float rho = 0.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
+    float rho = f[0], jx = f[1], jy = f[3], jz = f[5];
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) {
+    for (int q = 1; q < kQ; ++q) {
         rho += f[q];
-        if (cx(q) != 0) jx = cx(q) > 0 ? jx + f[q] : jx - f[q];
-        if (cy(q) != 0) jy = cy(q) > 0 ? jy + f[q] : jy - f[q];
-        if (cz(q) != 0) jz = cz(q) > 0 ? jz + f[q] : jz - f[q];
+        if (cx(q) != 0 && q != 1) jx = cx(q) > 0 ? jx + f[q] : jx - f[q];
+        if (cy(q) != 0 && q != 3) jy = cy(q) > 0 ? jy + f[q] : jy - f[q];
+        if (cz(q) != 0 && q != 5) jz = cz(q) > 0 ? jz + f[q] : jz - f[q];
     }
     rho = fmaxf(rho, kRhoFloor);
     const float invRho = 1.0f / rho;
     float ux = jx * invRho, uy = jy * invRho, uz = jz * invRho;
-    const float u2 = ux * ux + uy * uy + uz * uz;
+    float u2 = ux * ux + uy * uy + uz * uz;
     if (u2 > kMaxSimSpeed * kMaxSimSpeed) {
         // The hardware reciprocal square root, as the reference's GPU build
         // evaluates rsqrtf (lbm_core.cu:413); its CPU build and the oracle
         // use IEEE 1/sqrtf. Only cells beyond |u| = 0.3 take this branch.
         const float s = kMaxSimSpeed * rsqrtf(u2);
         ux *= s; uy *= s; uz *= s;
+        u2 = ux * ux + uy * uy + uz * uz;
     }
+    const float usq = 1.5f * u2;
     float feq[kQ];
-    eq19(rho, ux, uy, uz, feq);
+    feq[0] = (wgt(0) * rho) * (1.0f - usq);
+#pragma unroll
+    for (int p = 1; p <= 9; ++p) {
+        const int qa = 2 * p - 1, qb = 2 * p;
+        const float cu = 3.0f * dot_c(qa, ux, uy, uz);
+        const float h = 0.5f * cu * cu;
+        const float wr = wgt(qa) * rho;
+        feq[qa] = wr * (1.0f + cu + h - usq);
+        feq[qb] = wr * (1.0f - cu + h - usq);
+    }
     float tauEff = tau0;
     if (smagPre > 0.0f) {
-        float pxx = 0.0f, pyy = 0.0f, pzz = 0.0f, pxy = 0.0f, pxz = 0.0f, pyz = 0.0f;
+        float pxx = f[1] - feq[1], pyy = f[3] - feq[3], pzz = f[5] - feq[5];
+        float pxy = f[7] - feq[7], pxz = f[9] - feq[9], pyz = f[11] - feq[11];
 #pragma unroll
-        for (int q = 0; q < kQ; ++q) {
+        for (int q = 2; q < kQ; ++q) {
             const float fneq = f[q] - feq[q];
             if (cx(q) != 0) pxx += fneq;
-            if (cy(q) != 0) pyy += fneq;
-            if (cz(q) != 0) pzz += fneq;
-            if (cx(q) * cy(q) != 0) pxy = cx(q) * cy(q) > 0 ? pxy + fneq : pxy - fneq;
-            if (cx(q) * cz(q) != 0) pxz = cx(q) * cz(q) > 0 ? pxz + fneq : pxz - fneq;
-            if (cy(q) * cz(q) != 0) pyz = cy(q) * cz(q) > 0 ? pyz + fneq : pyz - fneq;
+            if (cy(q) != 0 && q != 3) pyy += fneq;
+            if (cz(q) != 0 && q != 5) pzz += fneq;
+            if (cx(q) * cy(q) != 0 && q != 7) pxy = cx(q) * cy(q) > 0 ? pxy + fneq : pxy - fneq;
+            if (cx(q) * cz(q) != 0 && q != 9) pxz = cx(q) * cz(q) > 0 ? pxz + fneq : pxz - fneq;
+            if (cy(q) * cz(q) != 0 && q != 11) pyz = cy(q) * cz(q) > 0 ? pyz + fneq : pyz - fneq;
         }
         const float qbar = sqrtf(pxx * pxx + pyy * pyy + pzz * pzz + 2.0f * (pxy * pxy + pxz * pxz + pyz * pyz));
         tauEff = 0.5f * (tau0 + sqrtf(tau0 * tau0 + smagPre * qbar * invRho));
@@ -192,14 +210,14 @@ __device__ __forceinline__ void collide_exact(float (&f)[kQ], float tau0, float 
     const float omP = 1.0f / tauEff;
     const float tauM = 0.5f + lambda / (tauEff - 0.5f);
     const float omM = 1.0f / tauM;
+    const float hP = 0.5f * omP, hM = 0.5f * omM;
     f[0] = f[0] - omP * (f[0] - feq[0]);
 #pragma unroll
     for (int p = 1; p <= 9; ++p) {
         const int qa = 2 * p - 1, qb = 2 * p;
-        const float sym = omP * (0.5f * (f[qa] + f[qb]) - 0.5f * (feq[qa] + feq[qb]));
-        const float asym = omM * (0.5f * (f[qa] - f[qb]) - 0.5f * (feq[qa] - feq[qb]));
-        const float fa = f[qa];
-        f[qa] = fa - sym - asym;
+        const float sym = hP * ((f[qa] + f[qb]) - (feq[qa] + feq[qb]));
+        const float asym = hM * ((f[qa] - f[qb]) - (feq[qa] - feq[qb]));
+        f[qa] = f[qa] - sym - asym;
         f[qb] = f[qb] - sym + asym;
     }
     rhoO = rho; uxO = ux; uyO = uy; uzO = uz;
@@ -401,25 +419,17 @@ __device__ __forceinline__ void gather_bulk(const typename S::T* __restrict__ sr
 /// Bulk fluid cell away from the periodic faces: the same 19 pulls through
 /// the constant offsets.
 template <class S, bool DEV>
-__device__ __forceinline__ void gather_interior(const typename S::T* __restrict__ src, const PullOffsets& o,
-                                                unsigned cell, float (&f)[kQ]) {
-    const typename S::T* base = src + cell;
+__device__ __forceinline__ void gather_interior(const SlicePtrs<typename S::T>& o, unsigned cell, float (&f)[kQ]) {
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) f[q] = Pop<S, DEV>::ld(byte_add(base, o.pull[q]), 0, wgt(q));
+    for (int q = 0; q < kQ; ++q) f[q] = Pop<S, DEV>::ld(o.pull[q], cell, wgt(q));
 }
 
-/// Store the 19 populations of `cell` (slice offsets when given).
+/// Store the 19 populations of `cell` (slice pointers when given).
 template <class S, bool DEV>
 __device__ __forceinline__ void store_cell(typename S::T* __restrict__ dst, const CollideArgs& a, unsigned cell,
-                                           const float (&f)[kQ], const PullOffsets* o) {
-    if (o) {
-        typename S::T* base = dst + cell;
+                                           const float (&f)[kQ], const SlicePtrs<typename S::T>* o) {
 #pragma unroll
-        for (int q = 0; q < kQ; ++q) Pop<S, DEV>::st(byte_add(base, o->slice[q]), 0, f[q], wgt(q));
-    } else {
-#pragma unroll
-        for (int q = 0; q < kQ; ++q) Pop<S, DEV>::st(dst + q * a.n, cell, f[q], wgt(q));
-    }
+    for (int q = 0; q < kQ; ++q) Pop<S, DEV>::st(o ? o->out[q] : dst + q * a.n, cell, f[q], wgt(q));
 }
 
 /// Near-wall fluid cell: the upstream flag picks the (slot, cell) pair per
@@ -502,26 +512,25 @@ __device__ __forceinline__ void gather_wall(const typename S::T* __restrict__ sr
 /// otherwise -- with the same interpolated bounce-back and Ladd terms.
 template <class S, bool WM, bool QL, bool DEV>
 __device__ __forceinline__ void gather_solid_links(const typename S::T* __restrict__ src, const CollideArgs& a,
-                                                   const PullOffsets& o, unsigned cell, int x, int y, int z,
+                                                   const SlicePtrs<typename S::T>& o, unsigned cell, int x, int y, int z,
                                                    unsigned solidMask, float (&f)[kQ]) {
     using P = Pop<S, DEV>;
-    const typename S::T* base = src + cell;
     float uwx = 0.0f, uwy = 0.0f, uwz = 0.0f;
     if constexpr (WM) {
         uwx = __half2float(__ushort_as_half(a.uwx[cell]));
         uwy = __half2float(__ushort_as_half(a.uwy[cell]));
         uwz = __half2float(__ushort_as_half(a.uwz[cell]));
     }
-    f[0] = P::ld(base, 0, wgt(0));
+    f[0] = P::ld(o.own[0], cell, wgt(0));
 #pragma unroll
     for (int q = 1; q < kQ; ++q) {
         const bool solid = (solidMask >> (q - 1)) & 1u;
-        float fq = P::ld(byte_add(base, solid ? o.slice[opp(q)] : o.pull[q]), 0, wgt(q));
+        float fq = P::ld(solid ? o.own[opp(q)] : o.pull[q], cell, wgt(q));
         if (QL && solid) {
             const std::uint8_t qb = a.qFrac[static_cast<long long>(cell) * kQ + q];
             if (qb != 0) {
                 const float qf = static_cast<float>(qb) * (1.0f / 255.0f);
-                const float fOut = P::ld(byte_add(base, o.slice[q]), 0, wgt(q));
+                const float fOut = P::ld(o.own[q], cell, wgt(q));
                 if (qf >= 0.5f) {
                     const float inv2q = 0.5f / qf;
                     fq = inv2q * fOut + (1.0f - inv2q) * fq;
@@ -543,7 +552,7 @@ __device__ __forceinline__ void gather_solid_links(const typename S::T* __restri
 
 template <class S, bool EXACT>
 __device__ __forceinline__ void finish_cell(typename S::T* __restrict__ dst, const CollideArgs& a, unsigned cell,
-                                            float (&f)[kQ], const PullOffsets* o = nullptr) {
+                                            float (&f)[kQ], const SlicePtrs<typename S::T>* o = nullptr) {
     float r, ux, uy, uz;
     collide_body<EXACT>(f, a, r, ux, uy, uz);
     store_cell<S, !EXACT>(dst, a, cell, f, o);
@@ -557,9 +566,9 @@ template <class S, bool WM, bool QL, bool DEV, bool LW = false>
 __device__ __forceinline__ void gather_fluid(const typename S::T* __restrict__ src,
                                              const std::uint8_t* __restrict__ kind, const CollideArgs& a,
                                              std::uint8_t k, unsigned cell, int x, int y, int z, float (&f)[kQ],
-                                             const PullOffsets* o) {
+                                             const SlicePtrs<typename S::T>* o) {
     if (!(k & kNearWall)) {
-        if (o && interior(x, y, z, a)) gather_interior<S, DEV>(src, *o, cell, f);
+        if (o && interior(x, y, z, a)) gather_interior<S, DEV>(*o, cell, f);
         else gather_bulk<S, DEV>(src, a, neighbours(x, y, z, a.nx, a.ny, a.nz), f);
         return;
     }
@@ -584,7 +593,7 @@ __device__ __forceinline__ void gather_fluid(const typename S::T* __restrict__ s
 template <class S, bool WM, bool EXACT, bool QL = false, bool LW = false>
 __device__ __forceinline__ void collide_one(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
                                             const std::uint8_t* __restrict__ kind, const CollideArgs& a, int x, int y,
-                                            int z, const PullOffsets* o = nullptr) {
+                                            int z, const SlicePtrs<typename S::T>* o = nullptr) {
     const unsigned cell = static_cast<unsigned>(x)
                         + static_cast<unsigned>(a.nx) * (static_cast<unsigned>(y) + static_cast<unsigned>(a.ny) * z);
     const std::uint8_t k = kind[cell];
@@ -598,36 +607,161 @@ __device__ __forceinline__ void collide_one(const typename S::T* __restrict__ sr
     finish_cell<S, EXACT>(dst, a, cell, f, o);
 }
 
-// ---- one cell per thread -----------------------------------------------------
-constexpr int kCellBlockX = 128;
+// ---- one cell per thread over the flattened lattice -----------------------------
+// Consecutive threads take consecutive cells across row boundaries, so no
+// warp is cut by a row end. (x, y, z) come from two divisions by invariant
+// integers (FastDiv, d3q19.cuh). HBM-bound with FP32 storage. With codes, a
+// warp of bulk interior cells reads one code byte, brought into L2 ahead of
+// time, in place of 32 kind bytes that stream from HBM before its pulls can
+// start, and needs no coordinates: the 768x320x96 tunnel (23.6 M cells, FP32)
+// runs at 0.552 ms per step, 6.51 TB/s, against 0.591 ms by kind bytes and
+// rows; with every cell taken for bulk without looking it was 0.535 ms.
+constexpr int kCellBlockX = 128;   // the cells of one code word
 
-template <class S, bool WM, bool EXACT, bool QL>
-__global__ void __launch_bounds__(kCellBlockX, S::kCellMinBlocks)
-collide_cell_kernel(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
-                    const std::uint8_t* __restrict__ kind, CollideArgs a, const __grid_constant__ PullOffsets off) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= a.nx) return;
-    collide_one<S, WM, EXACT, QL>(src, dst, kind, a, x, blockIdx.y, blockIdx.z, &off);
+/// Codes of blocks that start a while later into L2: the codes of eight
+/// neighbouring blocks share a sector, and without it all eight wait for HBM.
+constexpr unsigned kCodesAhead = 3072;   // blocks; about one and a half residencies of the GPU
+__device__ __forceinline__ void prefetch_codes(const std::uint32_t* codes) {
+    if ((blockIdx.x & 7) == 0 && threadIdx.x == 0 && blockIdx.x + kCodesAhead < gridDim.x)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(codes + blockIdx.x + kCodesAhead));
 }
 
-// ---- one cell per thread over the flattened lattice -----------------------------
-// For levels whose rows are not a multiple of 32 cells (the 616-cell fine
-// rows of the airfoil patch), a row-per-block launch ends every row with a
-// partly idle warp; here consecutive threads take consecutive cells across
-// row boundaries. (x, y, z) come from two divisions by invariant integers
-// (FastDiv, d3q19.cuh).
+/// One cell, its warp's tile code known.
+template <class S, bool WM, bool EXACT, bool QL>
+__device__ __forceinline__ void collide_coded(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
+                                              const std::uint8_t* __restrict__ kind, int code, const CollideArgs& a,
+                                              const SlicePtrs<typename S::T>& off, unsigned cell, const FastDiv& divX,
+                                              const FastDiv& divY) {
+    if (cell >= static_cast<unsigned>(a.n) || (code == kTileIdle && !a.writeMacro)) return;
+    float f[kQ];
+    if (code == kTileBulk) {
+        gather_interior<S, !EXACT>(off, cell, f);
+    } else {
+        const std::uint8_t k = kind[cell];
+        const unsigned row = fdiv(cell, divX), zu = fdiv(row, divY);
+        const int x = static_cast<int>(cell - row * divX.d), y = static_cast<int>(row - zu * divY.d);
+        const int z = static_cast<int>(zu), flag = k & kFlagMask;
+        if (flag != kFluid) {
+            boundary_cell<S>(src, dst, a, flag, cell, x, y, z);
+            return;
+        }
+        gather_fluid<S, WM, QL, !EXACT>(src, kind, a, k, cell, x, y, z, f, &off);
+    }
+    finish_cell<S, EXACT>(dst, a, cell, f, &off);
+}
+
+template <class S, bool WM, bool EXACT, bool QL, bool CODED>
+__global__ void __launch_bounds__(kCellBlockX, CODED ? S::kCodedMinBlocks : S::kCellMinBlocks)
+collide_flat_kernel(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
+                    const std::uint8_t* __restrict__ kind, const std::uint32_t* __restrict__ codes, CollideArgs a,
+                    const __grid_constant__ SlicePtrs<typename S::T> off, FastDiv divX, FastDiv divY) {
+    const unsigned cell = blockIdx.x * kCellBlockX + threadIdx.x;
+    int code = kTileGeneral;
+    if constexpr (CODED) {
+        prefetch_codes(codes);
+        code = reinterpret_cast<const std::uint8_t*>(codes)[cell >> 5];
+    }
+    collide_coded<S, WM, EXACT, QL>(src, dst, kind, code, a, off, cell, divX, divY);
+}
+
+// ---- tiles staged through shared memory (16-bit populations) --------------------
+// A warp's access to one slice moves 64 bytes at 2 bytes a lane, and it is
+// those small requests that bound the one-cell kernel with FP16 storage: with
+// its collision taken out it ran no faster. Here a block brings the pulls of
+// 128 consecutive cells in by 16-byte asynchronous copies (the 17 aligned
+// chunks around each slice's run) and writes its results back in 16-byte
+// pieces. A block whose cells are not all bulk and off the lattice's faces
+// (walls, faces, inlets, outlets) runs cell by cell.
+constexpr int kTile = 128;
+constexpr int kTileRow = (kTile / 8 + 1) * 16;   // bytes of a slice's run with its misalignment
+constexpr std::uint32_t kTileWordBulk = kTileBulk * 0x01010101u;
+
+/// Per slice: the 16-byte boundary at or below cell 0's element of the reads,
+/// the byte offset of that element in the tile, and cell 0's element of the
+/// writes.
+template <class T>
+struct TileMap {
+    const T* in[kQ];
+    T* out[kQ];
+    unsigned inOff[kQ];
+
+    __host__ void set(int q, const T* i, T* o) {
+        const auto u = reinterpret_cast<std::uintptr_t>(i);
+        in[q] = reinterpret_cast<const T*>(u & ~std::uintptr_t{15});
+        inOff[q] = static_cast<unsigned>(q * kTileRow + (u & 15u));
+        out[q] = o;
+    }
+};
+
+/// Copy the runs of the 128 cells from c0 on (a multiple of 128, all of them
+/// off the faces, so that a run's last chunk ends inside the buffer) into
+/// `tile` and wait for them.
+template <class T>
+__device__ __forceinline__ void tile_in(const TileMap<T>& m, unsigned c0, unsigned tile) {
+    const unsigned t = threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {   // 16 chunks a slice
+        const unsigned i = t + kTile * j, q = i >> 4, c = i & 15;
+        if (q < kQ)
+            asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(tile + q * kTileRow + 16 * c),
+                         "l"(m.in[q] + (c0 + 8 * c))
+                         : "memory");
+    }
+    if (t >= 64 && t < 64 + kQ) {   // and the 17th (the third round left warps 2 and 3 idle)
+        const unsigned q = t - 64;
+        asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(tile + q * kTileRow + 256),
+                     "l"(m.in[q] + (c0 + kTile))
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+}
+
+/// Results of the block's 128 cells to their slots by 16-byte stores through
+/// `tile`, whose contents every thread has read. n a multiple of 8.
+template <class S, bool DEV>
+__device__ __forceinline__ void tile_out(const TileMap<typename S::T>& m, unsigned c0, const float (&f)[kQ],
+                                         unsigned char* tile) {
+    using T = typename S::T;
+    const unsigned t = threadIdx.x;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) Pop<S, DEV>::st(reinterpret_cast<T*>(tile + q * kTileRow), t, f[q], wgt(q));
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const unsigned i = t + kTile * j, q = i >> 4, c = i & 15;
+        if (q < kQ)
+            *reinterpret_cast<uint4*>(m.out[q] + (c0 + 8 * c)) =
+                *reinterpret_cast<const uint4*>(tile + q * kTileRow + 16 * c);
+    }
+}
 
 template <class S, bool WM, bool EXACT, bool QL>
-__global__ void __launch_bounds__(kCellBlockX, S::kCellMinBlocks)
-collide_flat_kernel(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
-                    const std::uint8_t* __restrict__ kind, CollideArgs a, const __grid_constant__ PullOffsets off,
-                    FastDiv divX, FastDiv divY) {
-    const unsigned cell = blockIdx.x * kCellBlockX + threadIdx.x;
-    if (cell >= static_cast<unsigned long long>(a.n)) return;
-    const unsigned row = fdiv(cell, divX);
-    const unsigned z = fdiv(row, divY);
-    collide_one<S, WM, EXACT, QL>(src, dst, kind, a, static_cast<int>(cell - row * divX.d),
-                                  static_cast<int>(row - z * divY.d), static_cast<int>(z), &off);
+__global__ void __launch_bounds__(kTile, S::kTileMinBlocks)
+collide_tile_kernel(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
+                    const std::uint8_t* __restrict__ kind, const std::uint32_t* __restrict__ codes, CollideArgs a,
+                    const __grid_constant__ SlicePtrs<typename S::T> off,
+                    const __grid_constant__ TileMap<typename S::T> map, FastDiv divX, FastDiv divY) {
+    using P = Pop<S, !EXACT>;
+    __shared__ __align__(16) unsigned char tile[kQ * kTileRow];
+    const unsigned c0 = blockIdx.x * kTile, t = threadIdx.x, cell = c0 + t;
+    prefetch_codes(codes);
+    const std::uint32_t word = codes[blockIdx.x];
+    if (word != kTileWordBulk) {
+        collide_coded<S, WM, EXACT, QL>(src, dst, kind, static_cast<int>(word >> (8 * (t >> 5))) & 0xff, a, off, cell,
+                                        divX, divY);
+        return;
+    }
+    const unsigned tb = smem_addr(tile);
+    tile_in(map, c0, tb);
+    float f[kQ], r, ux, uy, uz;
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) f[q] = P::lds(tb + map.inOff[q], t, wgt(q));
+    collide_body<EXACT>(f, a, r, ux, uy, uz);
+    if (a.writeMacro) { a.rho[cell] = r; a.u[cell] = ux; a.v[cell] = uy; a.w[cell] = uz; }
+    if (a.n % 8 == 0) tile_out<S, !EXACT>(map, c0, f, tile);
+    else store_cell<S, !EXACT>(dst, a, cell, f, &off);
 }
 
 // ---- AA-pattern in-place streaming (all-fluid periodic lattices) --------------
@@ -647,6 +781,15 @@ collide_flat_kernel(const typename S::T* __restrict__ src, typename S::T* __rest
 // populations entering each collision are the A/B kernel's, so the results
 // are identical bit for bit. Opposite directions share a weight, so the FP16
 // deviation bytes move between slots unchanged.
+
+template <class T>
+__device__ __forceinline__ const T* byte_add(const T* p, long long b) {
+    return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + b);
+}
+template <class T>
+__device__ __forceinline__ T* byte_add(T* p, long long b) {
+    return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + b);
+}
 
 /// Byte offsets from &A[0][x] of the odd-step read A[opp(q)][x - c_q] of an
 /// interior cell; its write A[q][x + c_q] is the read offset of opp(q).
@@ -819,7 +962,7 @@ template <class S, bool WM, bool EXACT, bool QL>
 __global__ void __launch_bounds__(kFuseX, S::kChildMinBlocks)
 collide_child_kernel(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
                      const std::uint8_t* __restrict__ kind, CollideArgs a, ChildFuse cf,
-                     const __grid_constant__ PullOffsets off) {
+                     const __grid_constant__ SlicePtrs<typename S::T> off) {
     const int x = blockIdx.x * kFuseX + threadIdx.x;
     const bool inX = x < a.nx;
     const bool even = (threadIdx.x & 1) == 0;
@@ -866,10 +1009,8 @@ collide_child_kernel(const typename S::T* __restrict__ src, typename S::T* __res
                     boundary_cell<S>(src, dst, a, flag, cell, x, y, z);
                     if (flag != kSolid) {
                         // Written or untouched, the child average sees what dst holds.
-                        const typename S::T* base = dst + cell;
 #pragma unroll
-                        for (int q = 0; q < kQ; ++q)
-                            v[q] = Pop<S, !EXACT>::ld_coherent(byte_add(base, off.slice[q]), wgt(q));
+                        for (int q = 0; q < kQ; ++q) v[q] = Pop<S, !EXACT>::ld_coherent(off.out[q] + cell, wgt(q));
                         solid = false;
                     }
                 }
@@ -929,7 +1070,7 @@ cudaError_t launch_collide_child_impl(const void* srcv, void* dstv, const std::u
     const T* src = static_cast<const T*>(srcv);
     T* dst = static_cast<T*>(dstv);
     const bool ql = a.qFrac != nullptr;
-    const PullOffsets off = pull_offsets<T>(d.nx, d.ny, a.n);
+    const SlicePtrs<T> off = slice_ptrs<T>(src, dst, d.nx, d.ny, a.n);
     if (slip.active())
         (ql ? collide_child_kernel<S, true, EXACT, true> : collide_child_kernel<S, true, EXACT, false>)
             <<<grid, block, 0, st>>>(src, dst, kind, a, cf, off);
@@ -958,9 +1099,6 @@ constexpr int kStagedThreads = (kConsumerWarps + 1) * 32;
 constexpr int kMaxStages = 8;
 constexpr long long kWaitLimit = 1LL << 18; // try_wait polls (each may sleep ~20 us) before a timeout
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
 __device__ __forceinline__ void mbar_init(std::uint64_t* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
@@ -1232,25 +1370,30 @@ cudaError_t launch_collide_impl(const void* srcv, void* dstv, const std::uint8_t
         kern<<<static_cast<unsigned>(grid), kStagedThreads, plan.smem, st>>>(src, dst, kind, a, plan.stages);
         return cudaGetLastError();
     }
-    const int bx = d.nx >= kCellBlockX ? kCellBlockX : ((d.nx + 31) / 32) * 32;
-    const dim3 grid(static_cast<unsigned>((d.nx + bx - 1) / bx), static_cast<unsigned>(d.ny),
-                    static_cast<unsigned>(d.nz));
-    const PullOffsets off = pull_offsets<T>(d.nx, d.ny, a.n);
-    if (d.nx % 32 != 0 && d.nx >= 2 && d.ny >= 2) {
-        const FastDiv fx = fast_div(static_cast<unsigned>(d.nx)), fy = fast_div(static_cast<unsigned>(d.ny));
-        const unsigned blocks = static_cast<unsigned>((a.n + kCellBlockX - 1) / kCellBlockX);
-        const bool ql = a.qFrac != nullptr;
-        auto kern = wm ? (ql ? collide_flat_kernel<S, true, EXACT, true> : collide_flat_kernel<S, true, EXACT, false>)
-                       : (ql ? collide_flat_kernel<S, false, EXACT, true> : collide_flat_kernel<S, false, EXACT, false>);
-        kern<<<blocks, kCellBlockX, 0, st>>>(src, dst, kind, a, off, fx, fy);
-        return cudaGetLastError();
-    }
-    if (a.qFrac) {
-        if (wm) collide_cell_kernel<S, true, EXACT, true><<<grid, bx, 0, st>>>(src, dst, kind, a, off);
-        else collide_cell_kernel<S, false, EXACT, true><<<grid, bx, 0, st>>>(src, dst, kind, a, off);
+    const SlicePtrs<T> off = slice_ptrs<T>(src, dst, d.nx, d.ny, a.n);
+    const FastDiv fx = fast_div(static_cast<unsigned>(d.nx)), fy = fast_div(static_cast<unsigned>(d.ny));
+    const unsigned blocks = static_cast<unsigned>((a.n + kCellBlockX - 1) / kCellBlockX);
+    const bool ql = a.qFrac != nullptr;
+    // Codes (and the tiles they announce) where the populations stream from
+    // HBM; a lattice that stays in L2 has its kind bytes there too, and the
+    // code is then one more load ahead of the pulls.
+    const bool coded = p.tiles && a.n >= S::kCodedCells;
+    if (coded && (sizeof(T) == 4 || p.kernel == 0)) {
+        if constexpr (sizeof(T) == 2) {
+            TileMap<T> map;
+            for (int q = 0; q < kQ; ++q) map.set(q, off.pull[q], off.out[q]);
+            auto kern = wm ? (ql ? collide_tile_kernel<S, true, EXACT, true> : collide_tile_kernel<S, true, EXACT, false>)
+                           : (ql ? collide_tile_kernel<S, false, EXACT, true> : collide_tile_kernel<S, false, EXACT, false>);
+            kern<<<blocks, kTile, 0, st>>>(src, dst, kind, p.tiles, a, off, map, fx, fy);
+        } else {
+            auto kern = wm ? (ql ? collide_flat_kernel<S, true, EXACT, true, true> : collide_flat_kernel<S, true, EXACT, false, true>)
+                           : (ql ? collide_flat_kernel<S, false, EXACT, true, true> : collide_flat_kernel<S, false, EXACT, false, true>);
+            kern<<<blocks, kCellBlockX, 0, st>>>(src, dst, kind, p.tiles, a, off, fx, fy);
+        }
     } else {
-        if (wm) collide_cell_kernel<S, true, EXACT, false><<<grid, bx, 0, st>>>(src, dst, kind, a, off);
-        else collide_cell_kernel<S, false, EXACT, false><<<grid, bx, 0, st>>>(src, dst, kind, a, off);
+        auto kern = wm ? (ql ? collide_flat_kernel<S, true, EXACT, true, false> : collide_flat_kernel<S, true, EXACT, false, false>)
+                       : (ql ? collide_flat_kernel<S, false, EXACT, true, false> : collide_flat_kernel<S, false, EXACT, false, false>);
+        kern<<<blocks, kCellBlockX, 0, st>>>(src, dst, kind, nullptr, a, off, fx, fy);
     }
     return cudaGetLastError();
 }

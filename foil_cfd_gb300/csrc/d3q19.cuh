@@ -146,10 +146,16 @@ struct StoreF32 {
     using T = float;
     static constexpr int kBytes = 4;
     /// Resident 128-thread blocks per SM the one-cell collide is compiled
-    /// for: a cap of 51 registers, of which ptxas allocates 48 (the
-    /// fine-level launch measured 1.7 % faster than with the compiler's own
-    /// 56).
+    /// for: 48 registers where every cell's kind is read (a lattice in L2;
+    /// 40 ran 2 % faster to 13 % slower on 0.07-0.9 M cells), 40 where the
+    /// warps go by tile codes (0.563 -> 0.550 ms per step of the 768x320x96
+    /// tunnel against 48).
     static constexpr int kCellMinBlocks = 10;
+    static constexpr int kCodedMinBlocks = 12;
+    /// Cells from which the collide goes by tile codes: 1.63 M cells 48 us
+    /// per step with and without them, 3.97 M 103 with and 105 without,
+    /// 7.78 M 190 and 198; 0.33 M 14.6 and 12.6.
+    static constexpr long long kCodedCells = 2500000;
     /// Resident threads per SM the batched collide is compiled for: 64
     /// registers (the FP16 batched polar measured 15 % slower at 1536
     /// threads, 40 registers).
@@ -188,6 +194,14 @@ struct StoreF16 {
     /// A cap of 42 registers, of which ptxas allocates 40: the fine-level
     /// launch measured 7 % faster than at 56.
     static constexpr int kCellMinBlocks = 12;
+    static constexpr int kCodedMinBlocks = kCellMinBlocks;
+    /// The staged tiles at 40 registers: 16 blocks (32 registers) ran 2 %
+    /// slower, 10 blocks 5 %.
+    static constexpr int kTileMinBlocks = 12;
+    /// Cells from which the collide goes by tile codes and stages its tiles:
+    /// 2.62 M cells 52.1 us per step staged and 51.6 cell by cell, 3.97 M 73.6
+    /// and 74.2, 7.78 M 132 and 150.
+    static constexpr long long kCodedCells = 4000000;
     static constexpr int kBatchThreads = 1024;
     static constexpr int kChildMinBlocks = 8;
     __device__ __forceinline__ static float ld(const T* __restrict__ p, long long i, float w) {

@@ -42,6 +42,9 @@ struct CollideParams {
     /// Link classes of each fluid cell's pull neighbours (launch_classify),
     /// or null: the near-wall gather then reads the neighbours' flags.
     const uint2* links = nullptr;
+    /// Tile codes of the level (launch_tile_codes), or null: every cell then
+    /// goes by its kind byte.
+    const std::uint32_t* tiles = nullptr;
 };
 
 /// Half-bit slip field of a level (WallSlipView, lbm_core.cuh:201-208).
@@ -61,6 +64,16 @@ enum class Storage : int { F32 = 0, F16 = 1 };
 /// that are not fluid.
 cudaError_t launch_classify(const std::uint8_t* flags, std::uint8_t* kind,
                             LevelDims d, cudaStream_t st, uint2* links = nullptr);
+/// What a step finds in the 32 consecutive cells of a warp.
+enum : std::uint8_t {
+    kTileIdle = 0,     ///< no cell that a step writes
+    kTileGeneral = 1,  ///< cells to be looked at one by one
+    kTileBulk = 2      ///< all 32 bulk and off the lattice's faces
+};
+/// Tile codes: one word per 128 consecutive cells, byte w the code of its
+/// cells 32 w .. 32 w + 31 (cells past the end count as idle).
+cudaError_t launch_tile_codes(const std::uint8_t* kind, std::uint32_t* tiles, LevelDims d, cudaStream_t st);
+inline size_t tile_code_bytes(long long cells) { return static_cast<size_t>((cells + 127) / 128) * 4; }
 cudaError_t launch_collide(Storage s, const void* src, void* dst,
                            const std::uint8_t* kind, LevelDims d,
                            const CollideParams& p, float* rho, float* u,

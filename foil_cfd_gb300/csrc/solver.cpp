@@ -105,6 +105,7 @@ struct Level {
     std::uint8_t* flags = nullptr;
     std::uint8_t* kind = nullptr;
     uint2* links = nullptr;   // pull-link classes of the fluid cells (8 B per cell)
+    std::uint32_t* tiles = nullptr;   // tile codes (a word per 128 cells)
     int src = 0;
     std::vector<std::uint8_t> hostFlags, surfaceRef;
     std::uint32_t *dLinkCells = nullptr, *dLinkMasks = nullptr;
@@ -128,7 +129,7 @@ struct Level {
     }
 
     void free_all() {
-        dfree(f[0]); dfree(f[1]); dfree(flags); dfree(kind); dfree(links);
+        dfree(f[0]); dfree(f[1]); dfree(flags); dfree(kind); dfree(links); dfree(tiles);
         dfree(dLinkCells); dfree(dLinkMasks); dfree(dPartials);
         dfree(dQFrac); dfree(dFFMask);
         qLinks = qFallback = 0;
@@ -358,6 +359,7 @@ struct fcfd_solver {
         // up to 31 bytes past the last row: pad the allocation.
         if (auto e = dalloc(&L.kind, static_cast<size_t>(L.n) + 64); e != cudaSuccess) return e;
         if (auto e = dalloc(&L.links, static_cast<size_t>(L.n) * sizeof(uint2)); e != cudaSuccess) return e;
+        if (auto e = dalloc(&L.tiles, tile_code_bytes(L.n)); e != cudaSuccess) return e;
         return cudaSuccess;
     }
 
@@ -383,8 +385,9 @@ struct fcfd_solver {
         launches += 1;
         if (auto e = device_flag_classes(L.d, L.flags, stream, cls); e != cudaSuccess) return e;
         L.nReadWrite = cls[0]; L.nInlet = cls[1]; L.nUntouched = cls[2];
-        ++launches;
+        launches += 2;
         if (auto e = launch_classify(L.flags, L.kind, L.d, stream, L.links); e != cudaSuccess) return e;
+        if (auto e = launch_tile_codes(L.kind, L.tiles, L.d, stream); e != cudaSuccess) return e;
         // Compact force-link list of this level (ascending cell order).
         dfree(L.dLinkCells); dfree(L.dLinkMasks); dfree(L.dPartials);
         long long links = 0;
@@ -696,6 +699,7 @@ struct fcfd_solver {
         lp.qFrac = L.dQFrac;
         lp.ffMask = L.dFFMask;
         lp.links = L.links;
+        lp.tiles = L.tiles;
         cudaError_t e;
         if (aa) {
             e = launch_collide_aa(storage, L.f[0], L.d, lp, aaNextOdd, r, uu, vv, ww, stream);

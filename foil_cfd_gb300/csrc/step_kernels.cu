@@ -46,6 +46,27 @@ __global__ void classify_kernel(const std::uint8_t* __restrict__ flags,
     if (links) links[cell] = make_uint2(static_cast<unsigned>(m), static_cast<unsigned>(m >> 32));
 }
 
+/// Tile codes (kernels.h): one warp per 32 cells, so a block writes the
+/// words of its tiles.
+__global__ void __launch_bounds__(256)
+tile_codes_kernel(const std::uint8_t* __restrict__ kind, std::uint8_t* __restrict__ codes, int nx, int ny, int nz,
+                  unsigned n, FastDiv divX, FastDiv divY) {
+    const unsigned cell = blockIdx.x * 256u + threadIdx.x;
+    bool bulk = false, idle = true;
+    if (cell < n) {
+        const int k = kind[cell], flag = k & kFlagMask;
+        idle = !(flag == kFluid || flag == kInlet || flag == kOutlet || flag == kOutletEq);
+        if (k == kFluid) {
+            const unsigned row = fdiv(cell, divX), z = fdiv(row, divY);
+            const int x = static_cast<int>(cell - row * divX.d), y = static_cast<int>(row - z * divY.d);
+            bulk = x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && static_cast<int>(z) < nz - 1;
+        }
+    }
+    const bool all = __all_sync(0xffffffffu, bulk), none = __all_sync(0xffffffffu, idle);
+    if ((threadIdx.x & 31) == 0 && cell / 128 < (n + 127) / 128)
+        codes[cell >> 5] = all ? kTileBulk : (none ? kTileIdle : kTileGeneral);
+}
+
 template <class S>
 __global__ void init_eq_kernel(typename S::T* __restrict__ f, const std::uint8_t* __restrict__ kind,
                                long long n, float uIn) {
@@ -188,6 +209,14 @@ cudaError_t launch_classify(const std::uint8_t* flags, std::uint8_t* kind, Level
                             cudaStream_t st, uint2* links) {
     if (!flags || !kind || d.cells() <= 0) return cudaErrorInvalidValue;
     classify_kernel<<<plane_grid(d, 128), 128, 0, st>>>(flags, kind, d.nx, d.ny, d.nz, links);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tile_codes(const std::uint8_t* kind, std::uint32_t* tiles, LevelDims d, cudaStream_t st) {
+    if (!kind || !tiles || d.cells() <= 0 || d.nx < 2 || d.ny < 2) return cudaErrorInvalidValue;
+    tile_codes_kernel<<<blocks_for(d.cells()), 256, 0, st>>>(
+        kind, reinterpret_cast<std::uint8_t*>(tiles), d.nx, d.ny, d.nz, static_cast<unsigned>(d.cells()),
+        fast_div(static_cast<unsigned>(d.nx)), fast_div(static_cast<unsigned>(d.ny)));
     return cudaGetLastError();
 }
 
