@@ -15,6 +15,7 @@ int batch_occupancy_f16(BatchShape sh) { return batch_occupancy_impl<StoreF16, f
 /// force samples and advance its device-side count.
 __global__ void force_append_kernel(const double* __restrict__ cur, int n3, double* __restrict__ hist, int cap,
                                     int* __restrict__ count) {
+    pdl_wait();
     const int c = *count;
     double* slot = hist + static_cast<long long>(c % cap) * n3;
     for (int i = threadIdx.x; i < n3; i += blockDim.x) slot[i] = cur[i];
@@ -28,6 +29,7 @@ __global__ void force_append_kernel(const double* __restrict__ cur, int n3, doub
 template <class S>
 __global__ void health_kernel(const typename S::T* __restrict__ f, const std::uint8_t* __restrict__ kind, long long n,
                               int* __restrict__ maxSpeedBits, int* __restrict__ nonFinite) {
+    pdl_wait();
     float best = 0.0f;
     int bad = 0;
     for (long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; c < n;
@@ -60,10 +62,10 @@ cudaError_t launch_batch_health(bool fp32, const void* f, const std::uint8_t* ki
                                 int* nonFinite, cudaStream_t st) {
     const unsigned nb = static_cast<unsigned>(std::min<long long>(4096, (n + 255) / 256));
     if (fp32)
-        health_kernel<StoreF32><<<nb, 256, 0, st>>>(static_cast<const float*>(f), kind, n, maxSpeedBits, nonFinite);
-    else
-        health_kernel<StoreF16><<<nb, 256, 0, st>>>(static_cast<const __half*>(f), kind, n, maxSpeedBits, nonFinite);
-    return cudaGetLastError();
+        return launch_pdl(health_kernel<StoreF32>, nb, 256, st, static_cast<const float*>(f), kind, n, maxSpeedBits,
+                          nonFinite);
+    return launch_pdl(health_kernel<StoreF16>, nb, 256, st, static_cast<const __half*>(f), kind, n, maxSpeedBits,
+                      nonFinite);
 }
 
 /// Latch every running tunnel whose health scan found a non-finite cell
@@ -71,6 +73,7 @@ cudaError_t launch_batch_health(bool fp32, const void* f, const std::uint8_t* ki
 /// + t] records the force-sample count at that moment.
 __global__ void batch_latch_kernel(const int* __restrict__ maxSpeedBits, const int* __restrict__ nonFinite, int ntun,
                                    float cap, const int* __restrict__ samples, int* __restrict__ latch) {
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntun || latch[t] != 0) return;
     const int v = nonFinite[t] > 0 ? 1 : (__int_as_float(maxSpeedBits[t]) >= cap ? 2 : 0);
@@ -82,13 +85,11 @@ __global__ void batch_latch_kernel(const int* __restrict__ maxSpeedBits, const i
 
 cudaError_t launch_batch_latch(const int* maxSpeedBits, const int* nonFinite, int ntun, float cap,
                                const int* samples, int* latch, cudaStream_t st) {
-    batch_latch_kernel<<<(ntun + 63) / 64, 64, 0, st>>>(maxSpeedBits, nonFinite, ntun, cap, samples, latch);
-    return cudaGetLastError();
+    return launch_pdl(batch_latch_kernel, (ntun + 63) / 64, 64, st, maxSpeedBits, nonFinite, ntun, cap, samples, latch);
 }
 
 cudaError_t launch_force_append(const double* cur, int n3, double* hist, int cap, int* count, cudaStream_t st) {
-    force_append_kernel<<<1, 256, 0, st>>>(cur, n3, hist, cap, count);
-    return cudaGetLastError();
+    return launch_pdl(force_append_kernel, 1, 256, st, cur, n3, hist, cap, count);
 }
 
 } // namespace fcfd

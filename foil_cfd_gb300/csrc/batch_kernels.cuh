@@ -28,6 +28,7 @@ namespace {
 template <class S, bool EXACT, int BX, int ROWS>
 __global__ void __launch_bounds__(BX, S::kBatchThreads / BX)
 batch_collide_kernel(const __grid_constant__ BatchTable P, unsigned itemBase, unsigned nItems, int parity) {
+    pdl_wait();
     using T = typename S::T;
     // FP32: the near-wall gather reads the cells' link words (batch step
     // 1.054 -> 0.950 ms on the polar); FP16: the same path at the 64-register
@@ -76,8 +77,7 @@ cudaError_t launch_batch_shape(const BatchTable& tab, unsigned itemBase, unsigne
                                cudaStream_t st) {
     const unsigned g = grid > 0 ? std::min<unsigned>(static_cast<unsigned>(grid), nItems) : nItems;
     if (g == 0) return cudaSuccess;
-    batch_collide_kernel<S, EXACT, BX, ROWS><<<g, BX, 0, st>>>(tab, itemBase, nItems, parity);
-    return cudaGetLastError();
+    return launch_pdl(batch_collide_kernel<S, EXACT, BX, ROWS>, g, BX, st, tab, itemBase, nItems, parity);
 }
 
 template <class S, bool EXACT, int BX, int ROWS>

@@ -37,6 +37,7 @@
 #include "child_record.cuh"
 #include "d3q19.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 #include <cuda_runtime.h>
 
@@ -655,6 +656,7 @@ __global__ void __launch_bounds__(kCellBlockX, CODED ? S::kCodedMinBlocks : S::k
 collide_flat_kernel(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
                     const std::uint8_t* __restrict__ kind, const std::uint32_t* __restrict__ codes, CollideArgs a,
                     const __grid_constant__ SlicePtrs<typename S::T> off, FastDiv divX, FastDiv divY) {
+    pdl_wait();
     const unsigned cell = blockIdx.x * kCellBlockX + threadIdx.x;
     int code = kTileGeneral;
     if constexpr (CODED) {
@@ -746,6 +748,7 @@ collide_tile_kernel(const typename S::T* __restrict__ src, typename S::T* __rest
     using P = Pop<S, !EXACT>;
     __shared__ __align__(16) unsigned char tile[kQ * kTileRow];
     const unsigned c0 = blockIdx.x * kTile, t = threadIdx.x, cell = c0 + t;
+    pdl_wait();
     prefetch_codes(codes);
     const std::uint32_t word = codes[blockIdx.x];
     if (word != kTileWordBulk) {
@@ -809,6 +812,7 @@ __host__ AAOffsets aa_offsets(int nx, int ny, long long n) {
 template <class S, bool EXACT, bool ODD>
 __global__ void __launch_bounds__(kCellBlockX, S::kCellMinBlocks)
 collide_aa_kernel(typename S::T* __restrict__ A, CollideArgs a, const __grid_constant__ AAOffsets off) {
+    pdl_wait();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= a.nx) return;
     const int y = blockIdx.y, z = blockIdx.z;
@@ -863,9 +867,8 @@ cudaError_t launch_collide_aa_impl(void* fv, LevelDims d, const CollideParams& p
     const dim3 grid(static_cast<unsigned>((d.nx + bx - 1) / bx), static_cast<unsigned>(d.ny),
                     static_cast<unsigned>(d.nz));
     const AAOffsets off = aa_offsets<T>(d.nx, d.ny, a.n);
-    if (odd) collide_aa_kernel<S, EXACT, true><<<grid, bx, 0, st>>>(f, a, off);
-    else collide_aa_kernel<S, EXACT, false><<<grid, bx, 0, st>>>(f, a, off);
-    return cudaGetLastError();
+    return launch_pdl(odd ? collide_aa_kernel<S, EXACT, true> : collide_aa_kernel<S, EXACT, false>, grid, dim3(bx), st, f,
+                      a, off);
 }
 
 // ---- warm-restart flag edits (applyFlagEditsKernel, lbm_core.cu:644-717) -----
@@ -963,6 +966,7 @@ __global__ void __launch_bounds__(kFuseX, S::kChildMinBlocks)
 collide_child_kernel(const typename S::T* __restrict__ src, typename S::T* __restrict__ dst,
                      const std::uint8_t* __restrict__ kind, CollideArgs a, ChildFuse cf,
                      const __grid_constant__ SlicePtrs<typename S::T> off) {
+    pdl_wait();
     const int x = blockIdx.x * kFuseX + threadIdx.x;
     const bool inX = x < a.nx;
     const bool even = (threadIdx.x & 1) == 0;
@@ -1071,13 +1075,10 @@ cudaError_t launch_collide_child_impl(const void* srcv, void* dstv, const std::u
     T* dst = static_cast<T*>(dstv);
     const bool ql = a.qFrac != nullptr;
     const SlicePtrs<T> off = slice_ptrs<T>(src, dst, d.nx, d.ny, a.n);
-    if (slip.active())
-        (ql ? collide_child_kernel<S, true, EXACT, true> : collide_child_kernel<S, true, EXACT, false>)
-            <<<grid, block, 0, st>>>(src, dst, kind, a, cf, off);
-    else
-        (ql ? collide_child_kernel<S, false, EXACT, true> : collide_child_kernel<S, false, EXACT, false>)
-            <<<grid, block, 0, st>>>(src, dst, kind, a, cf, off);
-    return cudaGetLastError();
+    auto kern = slip.active()
+                    ? (ql ? collide_child_kernel<S, true, EXACT, true> : collide_child_kernel<S, true, EXACT, false>)
+                    : (ql ? collide_child_kernel<S, false, EXACT, true> : collide_child_kernel<S, false, EXACT, false>);
+    return launch_pdl(kern, grid, block, st, src, dst, kind, a, cf, off);
 }
 
 // ---- staged: x-rows through shared memory with bulk async copies -------------
@@ -1384,18 +1385,17 @@ cudaError_t launch_collide_impl(const void* srcv, void* dstv, const std::uint8_t
             for (int q = 0; q < kQ; ++q) map.set(q, off.pull[q], off.out[q]);
             auto kern = wm ? (ql ? collide_tile_kernel<S, true, EXACT, true> : collide_tile_kernel<S, true, EXACT, false>)
                            : (ql ? collide_tile_kernel<S, false, EXACT, true> : collide_tile_kernel<S, false, EXACT, false>);
-            kern<<<blocks, kTile, 0, st>>>(src, dst, kind, p.tiles, a, off, map, fx, fy);
+            return launch_pdl(kern, blocks, kTile, st, src, dst, kind, p.tiles, a, off, map, fx, fy);
         } else {
             auto kern = wm ? (ql ? collide_flat_kernel<S, true, EXACT, true, true> : collide_flat_kernel<S, true, EXACT, false, true>)
                            : (ql ? collide_flat_kernel<S, false, EXACT, true, true> : collide_flat_kernel<S, false, EXACT, false, true>);
-            kern<<<blocks, kCellBlockX, 0, st>>>(src, dst, kind, p.tiles, a, off, fx, fy);
+            return launch_pdl(kern, blocks, kCellBlockX, st, src, dst, kind, p.tiles, a, off, fx, fy);
         }
     } else {
         auto kern = wm ? (ql ? collide_flat_kernel<S, true, EXACT, true, false> : collide_flat_kernel<S, true, EXACT, false, false>)
                        : (ql ? collide_flat_kernel<S, false, EXACT, true, false> : collide_flat_kernel<S, false, EXACT, false, false>);
-        kern<<<blocks, kCellBlockX, 0, st>>>(src, dst, kind, nullptr, a, off, fx, fy);
+        return launch_pdl(kern, blocks, kCellBlockX, st, src, dst, kind, nullptr, a, off, fx, fy);
     }
-    return cudaGetLastError();
 }
 
 } // namespace

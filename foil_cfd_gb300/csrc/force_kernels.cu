@@ -12,6 +12,7 @@
 // block partials in a fixed order, so the result is deterministic run to run.
 #include "d3q19.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 #include <cuda_runtime.h>
 
@@ -52,6 +53,7 @@ force_partial_kernel(const typename S::T* __restrict__ f, long long n,
                      const std::uint16_t* __restrict__ uwyA,
                      const std::uint16_t* __restrict__ uwzA,
                      double* __restrict__ partials) {
+    pdl_wait();
     double fx = 0.0, fy = 0.0, fz = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const std::uint32_t c = cells[i];
@@ -84,6 +86,7 @@ force_partial_kernel(const typename S::T* __restrict__ f, long long n,
 
 __global__ void __launch_bounds__(kForceBlock)
 force_final_kernel(const double* __restrict__ partials, int nblocks, double* __restrict__ out) {
+    pdl_wait();
     double fx = 0.0, fy = 0.0, fz = 0.0;
     for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
         fx += partials[3 * b + 0];
@@ -110,18 +113,18 @@ cudaError_t launch_force(Storage s, const void* f, long long cells, const std::u
     const int nb = force_blocks(count);
     if (count == 0) return cudaMemsetAsync(out, 0, 3 * sizeof(double), st);
     const bool wm = slip.active();
+    cudaError_t e;
     if (s == Storage::F32) {
         auto* p = static_cast<const float*>(f);
-        if (wm) force_partial_kernel<StoreF32, true><<<nb, kForceBlock, 0, st>>>(p, cells, linkCells, linkMasks, count, slip.uwx, slip.uwy, slip.uwz, partials);
-        else force_partial_kernel<StoreF32, false><<<nb, kForceBlock, 0, st>>>(p, cells, linkCells, linkMasks, count, nullptr, nullptr, nullptr, partials);
+        e = launch_pdl(wm ? force_partial_kernel<StoreF32, true> : force_partial_kernel<StoreF32, false>, nb, kForceBlock,
+                       st, p, cells, linkCells, linkMasks, count, slip.uwx, slip.uwy, slip.uwz, partials);
     } else {
         auto* p = static_cast<const __half*>(f);
-        if (wm) force_partial_kernel<StoreF16, true><<<nb, kForceBlock, 0, st>>>(p, cells, linkCells, linkMasks, count, slip.uwx, slip.uwy, slip.uwz, partials);
-        else force_partial_kernel<StoreF16, false><<<nb, kForceBlock, 0, st>>>(p, cells, linkCells, linkMasks, count, nullptr, nullptr, nullptr, partials);
+        e = launch_pdl(wm ? force_partial_kernel<StoreF16, true> : force_partial_kernel<StoreF16, false>, nb, kForceBlock,
+                       st, p, cells, linkCells, linkMasks, count, slip.uwx, slip.uwy, slip.uwz, partials);
     }
-    if (auto e = cudaGetLastError(); e != cudaSuccess) return e;
-    force_final_kernel<<<1, kForceBlock, 0, st>>>(partials, nb, out);
-    return cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_pdl(force_final_kernel, 1, kForceBlock, st, partials, nb, out);
 }
 
 } // namespace fcfd

@@ -28,6 +28,7 @@
 #include "child_record.cuh"
 #include "d3q19.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 #include <cuda_runtime.h>
 
@@ -74,6 +75,7 @@ fill_kernel(const typename S::T* __restrict__ cT0, const typename S::T* __restri
             const std::uint8_t* __restrict__ ckind, typename S::T* __restrict__ ff,
             const std::uint32_t* __restrict__ targets, int count, RefineGeom g, float invFactor,
             float tw, float neqScale, FastDiv divX, FastDiv divXY) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const std::uint32_t t = targets[i];
@@ -170,6 +172,7 @@ template <class S>
 __global__ void __launch_bounds__(kRefineBlock)
 child_avg_kernel(const typename S::T* __restrict__ ff, const std::uint8_t* __restrict__ fkind,
                  RefineGeom g, int rx0, int ry0, int rw, int rh, float* __restrict__ scratch) {
+    pdl_wait();
     const int lx = blockIdx.x * blockDim.x + threadIdx.x;
     if (lx >= rw) return;
     const int ly = blockIdx.y, zc = blockIdx.z;
@@ -204,6 +207,7 @@ restrict_kernel(typename S::T* __restrict__ fc, const std::uint8_t* __restrict__
                 RefineGeom g, int rx0, int ry0, int rw, int rh, float neqScaleInv,
                 const float* __restrict__ scratch, float* __restrict__ mRho,
                 float* __restrict__ mU, float* __restrict__ mV, float* __restrict__ mW) {
+    pdl_wait();
     const int lx = blockIdx.x * kRestrictTX + threadIdx.x;
     const int ly = blockIdx.y * kRestrictTY + threadIdx.y;
     const int zc = blockIdx.z * kRestrictTZ + threadIdx.z;
@@ -280,14 +284,12 @@ cudaError_t launch_fill_c2f(Storage s, const void* cT0, const void* cT1,
     const FastDiv dx = fast_div(static_cast<unsigned>(g.fine.nx));
     const FastDiv dxy = fast_div(static_cast<unsigned>(g.fine.nx) * static_cast<unsigned>(g.fine.ny));
     if (s == Storage::F32)
-        (blend ? fill_kernel<StoreF32, true> : fill_kernel<StoreF32, false>)<<<nb, kRefineBlock, 0, st>>>(
-            static_cast<const float*>(cT0), static_cast<const float*>(cT1), coarseKind,
-            static_cast<float*>(fineF), targets, count, g, invF, timeWeight, neqScale, dx, dxy);
-    else
-        (blend ? fill_kernel<StoreF16, true> : fill_kernel<StoreF16, false>)<<<nb, kRefineBlock, 0, st>>>(
-            static_cast<const __half*>(cT0), static_cast<const __half*>(cT1), coarseKind,
-            static_cast<__half*>(fineF), targets, count, g, invF, timeWeight, neqScale, dx, dxy);
-    return cudaGetLastError();
+        return launch_pdl(blend ? fill_kernel<StoreF32, true> : fill_kernel<StoreF32, false>, nb, kRefineBlock, st,
+                          static_cast<const float*>(cT0), static_cast<const float*>(cT1), coarseKind,
+                          static_cast<float*>(fineF), targets, count, g, invF, timeWeight, neqScale, dx, dxy);
+    return launch_pdl(blend ? fill_kernel<StoreF16, true> : fill_kernel<StoreF16, false>, nb, kRefineBlock, st,
+                      static_cast<const __half*>(cT0), static_cast<const __half*>(cT1), coarseKind,
+                      static_cast<__half*>(fineF), targets, count, g, invF, timeWeight, neqScale, dx, dxy);
 }
 
 long long restrict_scratch_floats(const RefineGeom& g) {
@@ -317,20 +319,20 @@ cudaError_t launch_restrict_f2c(Storage s, const void* fineF, const std::uint8_t
                      static_cast<unsigned>((g.coarse.nz + kRestrictTZ - 1) / kRestrictTZ));
     if (s == Storage::F32) {
         if (!childDone)
-            child_avg_kernel<StoreF32><<<grid, kRefineBlock, 0, st>>>(
-                static_cast<const float*>(fineF), fineKind, g, rx0, ry0, rw, rh, scratch);
-        restrict_kernel<StoreF32><<<rgrid, rblock, 0, st>>>(
-            static_cast<float*>(coarseF), coarseKind, g, rx0, ry0, rw, rh, neqScaleInv, scratch,
-            macro ? rho : nullptr, u, v, w);
-    } else {
-        if (!childDone)
-            child_avg_kernel<StoreF16><<<grid, kRefineBlock, 0, st>>>(
-                static_cast<const __half*>(fineF), fineKind, g, rx0, ry0, rw, rh, scratch);
-        restrict_kernel<StoreF16><<<rgrid, rblock, 0, st>>>(
-            static_cast<__half*>(coarseF), coarseKind, g, rx0, ry0, rw, rh, neqScaleInv, scratch,
-            macro ? rho : nullptr, u, v, w);
+            if (auto e = launch_pdl(child_avg_kernel<StoreF32>, grid, kRefineBlock, st, static_cast<const float*>(fineF),
+                                    fineKind, g, rx0, ry0, rw, rh, scratch);
+                e != cudaSuccess)
+                return e;
+        return launch_pdl(restrict_kernel<StoreF32>, rgrid, rblock, st, static_cast<float*>(coarseF), coarseKind, g, rx0,
+                          ry0, rw, rh, neqScaleInv, scratch, macro ? rho : nullptr, u, v, w);
     }
-    return cudaGetLastError();
+    if (!childDone)
+        if (auto e = launch_pdl(child_avg_kernel<StoreF16>, grid, kRefineBlock, st, static_cast<const __half*>(fineF),
+                                fineKind, g, rx0, ry0, rw, rh, scratch);
+            e != cudaSuccess)
+            return e;
+    return launch_pdl(restrict_kernel<StoreF16>, rgrid, rblock, st, static_cast<__half*>(coarseF), coarseKind, g, rx0,
+                      ry0, rw, rh, neqScaleInv, scratch, macro ? rho : nullptr, u, v, w);
 }
 
 } // namespace fcfd

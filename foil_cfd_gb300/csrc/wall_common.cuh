@@ -27,6 +27,7 @@
 
 #include "d3q19.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 #include "wallnet.cuh"
 
 #include <cuda_runtime.h>
@@ -59,6 +60,7 @@ wall_update_kernel(const typename S::T* __restrict__ f, long long n, WallListDev
                    std::uint16_t* __restrict__ uwx, std::uint16_t* __restrict__ uwy,
                    std::uint16_t* __restrict__ uwz, float nu, float utCut, float ema,
                    WallStatsDev* __restrict__ stats, wallnet::NetDev net) {
+    pdl_wait();
     constexpr bool kNet = METHOD == 2;
     __shared__ float P[kNet ? wallnet::kParams : 1];
     if (kNet) {
@@ -186,8 +188,8 @@ void launch_wall(const void* f, long long cells, WallListDev list, std::uint16_t
                  std::uint16_t* uwz, float nu, float cut, float ema, WallStatsDev* stats, wallnet::NetDev net,
                  cudaStream_t st) {
     const unsigned nb = static_cast<unsigned>((list.count + kWallBlock - 1) / kWallBlock);
-    wall_update_kernel<S, M><<<nb, kWallBlock, 0, st>>>(static_cast<const typename S::T*>(f), cells, list, uwx, uwy,
-                                                        uwz, nu, cut, ema, stats, net);
+    (void)launch_pdl(wall_update_kernel<S, M>, nb, kWallBlock, st, static_cast<const typename S::T*>(f), cells, list,
+                     uwx, uwy, uwz, nu, cut, ema, stats, net);   // the caller reads the launch error
 }
 
 template <class S>
