@@ -28,16 +28,20 @@ __device__ __forceinline__ float rn_mul(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, b); }
 
+// Terms whose lattice coefficient is 0 are left out of the sums below, and
+// sums start from their first term: the same value for finite populations
+// (the sign of a zero aside).
+
 /// Moments of fi with the density floor and the |u| <= 0.3 limiter.
 __device__ __forceinline__ void limited_moments(const float (&fi)[kQ], float& rho, float& ux, float& uy,
                                                 float& uz) {
-    float r = 0.f, jx = 0.f, jy = 0.f, jz = 0.f;
+    float r = fi[0], jx = fi[1], jy = fi[3], jz = fi[5];
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) {
+    for (int q = 1; q < kQ; ++q) {
         r = rn_add(r, fi[q]);
-        jx = rn_add(jx, rn_mul(static_cast<float>(cx(q)), fi[q]));
-        jy = rn_add(jy, rn_mul(static_cast<float>(cy(q)), fi[q]));
-        jz = rn_add(jz, rn_mul(static_cast<float>(cz(q)), fi[q]));
+        if (cx(q) != 0 && q != 1) jx = cx(q) > 0 ? rn_add(jx, fi[q]) : rn_sub(jx, fi[q]);
+        if (cy(q) != 0 && q != 3) jy = cy(q) > 0 ? rn_add(jy, fi[q]) : rn_sub(jy, fi[q]);
+        if (cz(q) != 0 && q != 5) jz = cz(q) > 0 ? rn_add(jz, fi[q]) : rn_sub(jz, fi[q]);
     }
     r = fmaxf(r, kRhoFloor);
     const float inv = 1.0f / r;
@@ -52,14 +56,51 @@ __device__ __forceinline__ void limited_moments(const float (&fi)[kQ], float& rh
     rho = r;
 }
 
-/// Second-order equilibrium (lbm_core.cu:65-73), operations in source order.
-__device__ __forceinline__ float feq_q_rn(int q, float rho, float ux, float uy, float uz, float usq) {
-    const float cdot = rn_add(rn_add(rn_mul(static_cast<float>(cx(q)), ux), rn_mul(static_cast<float>(cy(q)), uy)),
-                              rn_mul(static_cast<float>(cz(q)), uz));
-    const float cu = rn_mul(3.0f, cdot);
-    const float poly = rn_sub(rn_add(rn_add(1.0f, cu), rn_mul(rn_mul(0.5f, cu), cu)), usq);
-    return rn_mul(rn_mul(wgt(q), rho), poly);
+/// c_q . u, the components in the order x, y, z.
+__device__ __forceinline__ float dot_rn(int q, float ux, float uy, float uz) {
+    float d = 0.0f;
+    bool any = false;
+    if (cx(q) != 0) { d = cx(q) > 0 ? ux : -ux; any = true; }
+    if (cy(q) != 0) { const float t = cy(q) > 0 ? uy : -uy; d = any ? rn_add(d, t) : t; any = true; }
+    if (cz(q) != 0) { const float t = cz(q) > 0 ? uz : -uz; d = any ? rn_add(d, t) : t; }
+    return d;
 }
+
+/// Second-order equilibria (lbm_core.cu:65-73), operations in source order;
+/// the two of an opposite pair share 0.5 (3 c.u)^2.
+__device__ __forceinline__ void feq_rn(float rho, float ux, float uy, float uz, float (&feq)[kQ]) {
+    const float usq = rn_mul(1.5f, rn_add(rn_add(rn_mul(ux, ux), rn_mul(uy, uy)), rn_mul(uz, uz)));
+    feq[0] = rn_mul(rn_mul(wgt(0), rho), rn_sub(1.0f, usq));
+#pragma unroll
+    for (int p = 1; p <= 9; ++p) {
+        const int a = 2 * p - 1;
+        const float cu = rn_mul(3.0f, dot_rn(a, ux, uy, uz));
+        const float h = rn_mul(rn_mul(0.5f, cu), cu), wr = rn_mul(wgt(a), rho);
+        feq[a] = rn_mul(wr, rn_sub(rn_add(rn_add(1.0f, cu), h), usq));
+        feq[a + 1] = rn_mul(wr, rn_sub(rn_add(rn_sub(1.0f, cu), h), usq));
+    }
+}
+
+/// The scratch covers the restricted sub-box with a border of one cell in x
+/// and y, so that every neighbour of a cell of the box has a record.
+struct RecordGrid {
+    int w = 0, h = 0;   // of the sub-box
+    __host__ __device__ unsigned index(int lx, int ly, int z) const {
+        return static_cast<unsigned>(lx + 1) + static_cast<unsigned>(w + 2)
+             * (static_cast<unsigned>(ly + 1) + static_cast<unsigned>(h + 2) * static_cast<unsigned>(z));
+    }
+    __host__ __device__ long long count(int nz) const { return static_cast<long long>(w + 2) * (h + 2) * nz; }
+};
+
+/// The planes of the scratch (four or six of them), float4 k of record t at p[k][t].
+struct RecordPlanes {
+    const float4* p[kScratchVals / 4];
+    __host__ static RecordPlanes of(const float* scratch, long long stride) {
+        RecordPlanes r;
+        for (int k = 0; k < kScratchVals / 4; ++k) r.p[k] = reinterpret_cast<const float4*>(scratch) + k * stride;
+        return r;
+    }
+};
 
 /// Layout of a coarse cell's record by storage. FP32 storage: fneq[19] in
 /// FP32, the valid flag, rho, ux, uy, uz -- six float4 (96 B), so the
@@ -67,6 +108,9 @@ __device__ __forceinline__ float feq_q_rn(int q, float rho, float ux, float uy, 
 /// as halves (the precision of the stored deviations), the valid flag and
 /// rho, ux, uy, uz in FP32 -- four float4 (64 B); the restriction's 19
 /// neighbour reads per coarse cell then move 48 B each instead of 80 B.
+/// A record without fluid children, and the border's, holds -0 in fneq and 0
+/// in the flag: adding it changes no sum (x + -0 is x for every x), so the
+/// restriction adds all its neighbours without looking.
 template <class S> struct ChildRecord;
 
 template <> struct ChildRecord<StoreF32> {
@@ -82,55 +126,29 @@ template <> struct ChildRecord<StoreF32> {
         for (int k = 0; k < kVec; ++k) rec[k * st] = make_float4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
     }
     __device__ __forceinline__ static void write_invalid(float4* rec, long long st) {
-        rec[(kScratchValid / 4) * st] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    /// fneq of the record into out; false (out untouched) when not valid.
-    __device__ __forceinline__ static bool load(const float4* rec, long long st, float (&out)[kQ]) {
-        const float4 v4 = __ldg(rec + (kScratchValid / 4) * st);   // fneq[16..18], valid
-        if (v4.w == 0.0f) return false;
-        out[16] = v4.x; out[17] = v4.y; out[18] = v4.z;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 a = __ldg(rec + k * st);
-            out[4 * k] = a.x; out[4 * k + 1] = a.y; out[4 * k + 2] = a.z; out[4 * k + 3] = a.w;
-        }
-        return true;
+        for (int k = 0; k < 4; ++k) rec[k * st] = make_float4(-0.0f, -0.0f, -0.0f, -0.0f);
+        rec[4 * st] = make_float4(-0.0f, -0.0f, -0.0f, 0.0f);
     }
-    /// acc[q] += fneq[q] for every q when the record is valid.
-    __device__ __forceinline__ static bool add(const float4* rec, long long st, float (&acc)[kQ]) {
-        const float4 last = __ldg(rec + (kScratchValid / 4) * st);
-        if (last.w == 0.0f) return false;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 a = __ldg(rec + k * st);
-            acc[4 * k] += a.x; acc[4 * k + 1] += a.y; acc[4 * k + 2] += a.z; acc[4 * k + 3] += a.w;
-        }
-        acc[16] += last.x; acc[17] += last.y; acc[18] += last.z;
-        return true;
-    }
-    __device__ __forceinline__ static float4 moments(const float4* rec, long long st) {
-        return __ldg(rec + (kScratchRho / 4) * st);
-    }
-    /// As add, but every part of the record is read before the valid flag
-    /// decides (a select keeps acc when the record is invalid), so the loads
-    /// of successive neighbours do not wait on each other's flags.
-    __device__ __forceinline__ static bool add_sel(const float4* rec, long long st, float (&acc)[kQ],
-                                                   bool use = true) {
+    /// acc[q] += fneq[q], count += valid flag; SET: the record's own values.
+    template <bool SET>
+    __device__ __forceinline__ static void add(const RecordPlanes& r, unsigned t, float (&acc)[kQ], float& count) {
         float4 a[5];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) a[k] = __ldg(rec + k * st);
-        const bool ok = use && a[4].w != 0.0f;
+        for (int k = 0; k < 5; ++k) a[k] = __ldg(r.p[k] + t);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            acc[4 * k] = ok ? acc[4 * k] + a[k].x : acc[4 * k];
-            acc[4 * k + 1] = ok ? acc[4 * k + 1] + a[k].y : acc[4 * k + 1];
-            acc[4 * k + 2] = ok ? acc[4 * k + 2] + a[k].z : acc[4 * k + 2];
-            acc[4 * k + 3] = ok ? acc[4 * k + 3] + a[k].w : acc[4 * k + 3];
+        for (int k = 0; k < 5; ++k) {
+            const float v[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int q = 4 * k + e;
+                if (q < kQ) acc[q] = SET ? v[e] : acc[q] + v[e];
+                else count = SET ? v[e] : count + v[e];
+            }
         }
-        acc[16] = ok ? acc[16] + a[4].x : acc[16];
-        acc[17] = ok ? acc[17] + a[4].y : acc[17];
-        acc[18] = ok ? acc[18] + a[4].z : acc[18];
-        return ok;
+    }
+    __device__ __forceinline__ static float4 moments(const RecordPlanes& r, unsigned t) {
+        return __ldg(r.p[kScratchRho / 4] + t);
     }
 };
 
@@ -155,65 +173,32 @@ template <> struct ChildRecord<StoreF16> {
         rec[3 * st] = make_float4(rho, ux, uy, uz);
     }
     __device__ __forceinline__ static void write_invalid(float4* rec, long long st) {
-        reinterpret_cast<uint4*>(rec)[2 * st] = make_uint4(0u, 0u, 0u, 0u);
+        uint4* r = reinterpret_cast<uint4*>(rec);
+        constexpr unsigned z = 0x80008000u;   // two halves of -0
+        r[0] = make_uint4(z, z, z, z);
+        r[st] = make_uint4(z, z, z, z);
+        r[2 * st] = make_uint4(z, z, 0u, 0u);
     }
-    __device__ __forceinline__ static bool load(const float4* rec, long long st, float (&out)[kQ]) {
-        const uint4 c2 = __ldg(reinterpret_cast<const uint4*>(rec) + 2 * st);
-        if (__uint_as_float(c2.z) == 0.0f) return false;
-        const float2 p16 = unpack(c2.x), p18 = unpack(c2.y);
-        out[16] = p16.x; out[17] = p16.y; out[18] = p18.x;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const uint4 c = __ldg(reinterpret_cast<const uint4*>(rec) + k * st);
-            const unsigned w[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 p = unpack(w[j]);
-                out[8 * k + 2 * j] = p.x; out[8 * k + 2 * j + 1] = p.y;
-            }
-        }
-        return true;
-    }
-    __device__ __forceinline__ static bool add(const float4* rec, long long st, float (&acc)[kQ]) {
-        const uint4 c2 = __ldg(reinterpret_cast<const uint4*>(rec) + 2 * st);
-        if (__uint_as_float(c2.z) == 0.0f) return false;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const uint4 c = __ldg(reinterpret_cast<const uint4*>(rec) + k * st);
-            const unsigned w[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 p = unpack(w[j]);
-                acc[8 * k + 2 * j] += p.x; acc[8 * k + 2 * j + 1] += p.y;
-            }
-        }
-        const float2 p16 = unpack(c2.x), p18 = unpack(c2.y);
-        acc[16] += p16.x; acc[17] += p16.y; acc[18] += p18.x;
-        return true;
-    }
-    __device__ __forceinline__ static float4 moments(const float4* rec, long long st) { return __ldg(rec + 3 * st); }
-    __device__ __forceinline__ static bool add_sel(const float4* rec, long long st, float (&acc)[kQ],
-                                                   bool use = true) {
+    template <bool SET>
+    __device__ __forceinline__ static void add(const RecordPlanes& r, unsigned t, float (&acc)[kQ], float& count) {
         uint4 c[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) c[k] = __ldg(reinterpret_cast<const uint4*>(rec) + k * st);
-        const bool ok = use && __uint_as_float(c[2].z) != 0.0f;
+        for (int k = 0; k < 3; ++k) c[k] = __ldg(reinterpret_cast<const uint4*>(r.p[k]) + t);
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < 3; ++k) {
             const unsigned w[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float2 p = unpack(w[j]);
-                acc[8 * k + 2 * j] = ok ? acc[8 * k + 2 * j] + p.x : acc[8 * k + 2 * j];
-                acc[8 * k + 2 * j + 1] = ok ? acc[8 * k + 2 * j + 1] + p.y : acc[8 * k + 2 * j + 1];
+                const int q = 8 * k + 2 * j;
+                if (q >= kQ) continue;
+                const float2 v = unpack(w[j]);
+                acc[q] = SET ? v.x : acc[q] + v.x;
+                if (q + 1 < kQ) acc[q + 1] = SET ? v.y : acc[q + 1] + v.y;
             }
         }
-        const float2 p16 = unpack(c[2].x), p18 = unpack(c[2].y);
-        acc[16] = ok ? acc[16] + p16.x : acc[16];
-        acc[17] = ok ? acc[17] + p16.y : acc[17];
-        acc[18] = ok ? acc[18] + p18.x : acc[18];
-        return ok;
+        count = SET ? __uint_as_float(c[2].z) : count + __uint_as_float(c[2].z);
     }
+    __device__ __forceinline__ static float4 moments(const RecordPlanes& r, unsigned t) { return __ldg(r.p[3] + t); }
 };
 
 /// Record of a coarse cell from the sum fi of its nFluid fluid children
@@ -230,10 +215,10 @@ __device__ __forceinline__ void write_child_record(float (&fi)[kQ], int nFluid, 
     for (int q = 0; q < kQ; ++q) fi[q] = DEV ? rn_mul(fi[q], invN) + wgt(q) : rn_mul(fi[q], invN);
     float rho, ux, uy, uz;
     limited_moments(fi, rho, ux, uy, uz);
-    const float usq = rn_mul(1.5f, rn_add(rn_add(rn_mul(ux, ux), rn_mul(uy, uy)), rn_mul(uz, uz)));
     float fneq[kQ];
+    feq_rn(rho, ux, uy, uz, fneq);
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) fneq[q] = rn_sub(fi[q], feq_q_rn(q, rho, ux, uy, uz, usq));
+    for (int q = 0; q < kQ; ++q) fneq[q] = rn_sub(fi[q], fneq[q]);
     ChildRecord<S>::write(rec, st, fneq, rho, ux, uy, uz);
 }
 

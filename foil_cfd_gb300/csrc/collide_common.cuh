@@ -993,50 +993,38 @@ collide_child_kernel(const typename S::T* __restrict__ src, typename S::T* __res
     for (int kz = 0; kz < 2; ++kz)
         for (int jy = 0; jy < 2; ++jy) {
             const int y = 2 * blockIdx.y + jy, z = 2 * blockIdx.z + kz;
+            // A solid child, or none, adds -0 to every sum: no sum changes.
             float v[kQ];
             bool solid = true;
-            if (inX) {
-                const unsigned cell = static_cast<unsigned>(x)
-                                    + static_cast<unsigned>(a.nx) * (static_cast<unsigned>(y) + static_cast<unsigned>(a.ny) * z);
-                const std::uint8_t k = static_cast<std::uint8_t>(kinds >> (8 * (2 * kz + jy)));
-                const int flag = k & kFlagMask;
-                if (flag == kFluid) {
-                    gather_fluid<S, WM, QL, !EXACT>(src, kind, a, k, cell, x, y, z, v, &off);
-                    float rr, ux, uy, uz;
-                    collide_body<EXACT>(v, a, rr, ux, uy, uz);
-                    // FP32: the sums see the stored values exactly. FP16:
-                    // the collided FP32 values (not their half round trip),
-                    // the more accurate child average.
-                    store_cell<S, !EXACT>(dst, a, cell, v, &off);
-                    solid = false;
-                } else {
-                    boundary_cell<S>(src, dst, a, flag, cell, x, y, z);
-                    if (flag != kSolid) {
-                        // Written or untouched, the child average sees what dst holds.
+            const std::uint8_t k = static_cast<std::uint8_t>(kinds >> (8 * (2 * kz + jy)));
+            const int flag = k & kFlagMask;
+            const unsigned cell = static_cast<unsigned>(x)
+                                + static_cast<unsigned>(a.nx) * (static_cast<unsigned>(y) + static_cast<unsigned>(a.ny) * z);
+            if (inX && flag == kFluid) {
+                gather_fluid<S, WM, QL, !EXACT>(src, kind, a, k, cell, x, y, z, v, &off);
+                float rr, ux, uy, uz;
+                collide_body<EXACT>(v, a, rr, ux, uy, uz);
+                // FP32: the sums see the stored values exactly. FP16:
+                // the collided FP32 values (not their half round trip),
+                // the more accurate child average.
+                store_cell<S, !EXACT>(dst, a, cell, v, &off);
+                solid = false;
+            } else {
+                if (inX) boundary_cell<S>(src, dst, a, flag, cell, x, y, z);
+                solid = !inX || flag == kSolid;
+                // Written or untouched, the child average sees what dst holds.
 #pragma unroll
-                        for (int q = 0; q < kQ; ++q) v[q] = Pop<S, !EXACT>::ld_coherent(off.out[q] + cell, wgt(q));
-                        solid = false;
-                    }
-                }
+                for (int q = 0; q < kQ; ++q)
+                    v[q] = solid ? -0.0f : Pop<S, !EXACT>::ld_coherent(off.out[q] + cell, wgt(q));
             }
             if (!solid) ++nFluid;
-            const bool partnerSolid = __shfl_xor_sync(0xffffffffu, static_cast<int>(solid), 1) != 0;
             // Children in order: the even lane's first, then the odd lane's.
-            const bool skipFirst = even ? solid : partnerSolid;
-            const bool skipSecond = even ? partnerSolid : solid;
 #pragma unroll
-            for (int k = 0; k < kSplit; ++k) {
-                const int qo = k + kSplit < kQ ? k + kSplit : kQ - 1;   // odd lane's direction
-                const float send = even ? v[qo] : v[k];
-                const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-                const float own = even ? v[k] : v[qo];
-                const float first = even ? own : recv, second = even ? recv : own;
-                if (k + kSplit < kQ || even) {
-                    float t = acc[k];
-                    if (!skipFirst) t += first;
-                    if (!skipSecond) t += second;
-                    acc[k] = t;
-                }
+            for (int k2 = 0; k2 < kSplit; ++k2) {
+                const int qo = k2 + kSplit < kQ ? k2 + kSplit : kQ - 1;   // odd lane's direction
+                const float recv = __shfl_xor_sync(0xffffffffu, even ? v[qo] : v[k2], 1);
+                const float own = even ? v[k2] : v[qo];
+                acc[k2] = (acc[k2] + (even ? own : recv)) + (even ? recv : own);
             }
         }
     // The even lane gathers the odd lane's sums (directions 10..18) and the
@@ -1048,9 +1036,10 @@ collide_child_kernel(const typename S::T* __restrict__ src, typename S::T* __res
 #pragma unroll
     for (int k = 0; k + kSplit < kQ; ++k) fi[k + kSplit] = __shfl_xor_sync(0xffffffffu, acc[k], 1);
     if (!record || !even) return;
-    const long long t = lx + static_cast<long long>(cf.rw) * (ly + static_cast<long long>(cf.rh) * blockIdx.z);
-    write_child_record<S, !EXACT>(fi, nFluid + nOdd, reinterpret_cast<float4*>(cf.scratch) + t,
-                                  static_cast<long long>(cf.rw) * cf.rh * (a.nz / 2));
+    const RecordGrid rg{cf.rw, cf.rh};
+    write_child_record<S, !EXACT>(fi, nFluid + nOdd,
+                                  reinterpret_cast<float4*>(cf.scratch) + rg.index(lx, ly, static_cast<int>(blockIdx.z)),
+                                  rg.count(a.nz / 2));
 }
 
 template <class S, bool EXACT>

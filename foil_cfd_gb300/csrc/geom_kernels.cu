@@ -19,7 +19,7 @@
 //   the force-link list, the wall-model cell list of buildWallCellList
 //   (src/sim/wall_model.cpp:55-236: pull-solid link mask, vane exclusion,
 //   5^3 occupancy-gradient normal, sample cell along the normal), the
-//   interface-shell list and the non-solid seed list of a refined level.
+//   interface-shell list of a refined level.
 //
 // Built without FMA contraction: the rasteriser's crossings and the wall
 // normals are the host builders' values bit for bit.
@@ -284,16 +284,6 @@ struct ShellPulledPred {
         }
         return 0u;
     }
-    __device__ void emit(long long slot, long long c, int, int, int, std::uint32_t) const {
-        cells[slot] = static_cast<std::uint32_t>(c);
-    }
-};
-
-struct FlagNePred {     // flag != value (non-solid seed list)
-    const std::uint8_t* f;
-    std::uint8_t value;
-    std::uint32_t* cells;
-    __device__ std::uint32_t eval(long long c, int, int, int, int*) const { return f[c] != value ? 1u : 0u; }
     __device__ void emit(long long slot, long long c, int, int, int, std::uint32_t) const {
         cells[slot] = static_cast<std::uint32_t>(c);
     }
@@ -731,10 +721,9 @@ cudaError_t device_force_links(LevelDims d, const std::uint8_t* flags, std::uint
     return compact_into(p, {d.nx, d.ny, d.nz}, cap, count, nullptr, st);
 }
 
-cudaError_t device_cells_where(LevelDims d, const std::uint8_t* flags, std::uint8_t value, bool equal,
-                               std::uint32_t* cells, long long cap, long long* count, cudaStream_t st) {
-    if (equal) return compact_into(FlagEqPred{flags, value, cells}, {d.nx, d.ny, d.nz}, cap, count, nullptr, st);
-    return compact_into(FlagNePred{flags, value, cells}, {d.nx, d.ny, d.nz}, cap, count, nullptr, st);
+cudaError_t device_cells_where(LevelDims d, const std::uint8_t* flags, std::uint8_t value, std::uint32_t* cells,
+                               long long cap, long long* count, cudaStream_t st) {
+    return compact_into(FlagEqPred{flags, value, cells}, {d.nx, d.ny, d.nz}, cap, count, nullptr, st);
 }
 
 cudaError_t device_shell_pulled(LevelDims d, const std::uint8_t* flags, std::uint32_t* cells, long long cap,

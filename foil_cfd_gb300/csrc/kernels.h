@@ -229,6 +229,12 @@ cudaError_t launch_fill_c2f(Storage s, const void* cT0, const void* cT1,
                             const std::uint32_t* targets, int count,
                             const RefineGeom& g, float timeWeight,
                             float neqScale, cudaStream_t st);
+/// Both buffers of the fine level from the coarse state: every cell that is
+/// not solid (the fill of a level that starts), in one pass.
+cudaError_t launch_seed_c2f(Storage s, const void* coarseF, const std::uint8_t* coarseKind, void* fine0, void* fine1,
+                            const std::uint8_t* fineKind, const RefineGeom& g, float neqScale, cudaStream_t st);
+/// A new scratch of the restriction (restrict_scratch_floats) has to be cleared once.
+cudaError_t launch_clear_scratch(Storage s, const RefineGeom& g, float* scratch, cudaStream_t st);
 /// Fine-to-coarse restriction. `scratch` holds 24 floats per coarse cell of
 /// the restricted sub-box (child-averaged fneq[19], rho, ux, uy, uz, valid).
 long long restrict_scratch_floats(const RefineGeom& g);
@@ -271,8 +277,8 @@ bool is_device_pointer(const void* p);
 /// exceeds cap (size with a first call of capacity 0). All synchronise.
 cudaError_t device_force_links(LevelDims d, const std::uint8_t* flags, std::uint32_t* cells, std::uint32_t* masks,
                                long long cap, long long* count, cudaStream_t st);
-cudaError_t device_cells_where(LevelDims d, const std::uint8_t* flags, std::uint8_t value, bool equal,
-                               std::uint32_t* cells, long long cap, long long* count, cudaStream_t st);
+cudaError_t device_cells_where(LevelDims d, const std::uint8_t* flags, std::uint8_t value, std::uint32_t* cells,
+                               long long cap, long long* count, cudaStream_t st);
 /// Interface cells with a fluid or outlet cell among their 18 neighbours
 /// (the shell cells a stream-collide reads), ascending; as device_cells_where.
 cudaError_t device_shell_pulled(LevelDims d, const std::uint8_t* flags, std::uint32_t* cells, long long cap,

@@ -45,44 +45,80 @@ constexpr int kRestrictBlend = 3;  // edge-blend ramp width (coarse cells)
 /// cell outside the coarse domain, so a compare replaces the division.
 __device__ __forceinline__ int wrap1(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 
-/// Latt-Chopard projection of fneq onto the second-order Hermite space.
+/// Latt-Chopard projection of fneq onto the second-order Hermite space
+/// (zero-coefficient terms left out, as in child_record.cuh).
 __device__ __forceinline__ void regularize(float (&fneq)[kQ]) {
-    float pxx = 0.f, pyy = 0.f, pzz = 0.f, pxy = 0.f, pxz = 0.f, pyz = 0.f;
+    float pxx = fneq[1], pyy = fneq[3], pzz = fneq[5], pxy = fneq[7], pxz = fneq[9], pyz = fneq[11];
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) {
+    for (int q = 2; q < kQ; ++q) {
         const float v = fneq[q];
-        pxx += cx(q) * cx(q) * v; pyy += cy(q) * cy(q) * v; pzz += cz(q) * cz(q) * v;
-        pxy += cx(q) * cy(q) * v; pxz += cx(q) * cz(q) * v; pyz += cy(q) * cz(q) * v;
+        if (cx(q) != 0) pxx += v;
+        if (cy(q) != 0 && q != 3) pyy += v;
+        if (cz(q) != 0 && q != 5) pzz += v;
+        if (cx(q) * cy(q) != 0 && q != 7) pxy = cx(q) * cy(q) > 0 ? pxy + v : pxy - v;
+        if (cx(q) * cz(q) != 0 && q != 9) pxz = cx(q) * cz(q) > 0 ? pxz + v : pxz - v;
+        if (cy(q) * cz(q) != 0 && q != 11) pyz = cy(q) * cz(q) > 0 ? pyz + v : pyz - v;
     }
     const float trace = (1.0f / 3.0f) * (pxx + pyy + pzz);
+    fneq[0] = 4.5f * wgt(0) * (0.0f - trace);
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-        const float qpi = cx(q) * cx(q) * pxx + cy(q) * cy(q) * pyy + cz(q) * cz(q) * pzz
-                        + 2.0f * (cx(q) * cy(q) * pxy + cx(q) * cz(q) * pxz + cy(q) * cz(q) * pyz)
-                        - trace;
-        fneq[q] = 4.5f * wgt(q) * qpi;
+    for (int p = 1; p <= 9; ++p) {   // c and -c project alike
+        const int q = 2 * p - 1;
+        float d = 0.0f;
+        bool any = false;
+        if (cx(q) != 0) { d = pxx; any = true; }
+        if (cy(q) != 0) { d = any ? d + pyy : pyy; any = true; }
+        if (cz(q) != 0) d = any ? d + pzz : pzz;
+        if (cx(q) * cy(q) != 0) d = cx(q) * cy(q) > 0 ? d + 2.0f * pxy : d - 2.0f * pxy;
+        if (cx(q) * cz(q) != 0) d = cx(q) * cz(q) > 0 ? d + 2.0f * pxz : d - 2.0f * pxz;
+        if (cy(q) * cz(q) != 0) d = cy(q) * cz(q) > 0 ? d + 2.0f * pyz : d - 2.0f * pyz;
+        fneq[q] = fneq[q + 1] = 4.5f * wgt(q) * (d - trace);
     }
 }
 
+/// Slice pointers of a fill: the coarse level's two time levels and the fine level.
+template <class T>
+struct FillPtrs {
+    const T* t0[kQ];
+    const T* t1[kQ];
+    T* out[kQ];
+    __host__ FillPtrs(const T* c0, const T* c1, T* f, long long cn, long long fn) {
+        for (int q = 0; q < kQ; ++q) {
+            t0[q] = c0 + q * cn;
+            t1[q] = c1 + q * cn;
+            out[q] = f + q * fn;
+        }
+    }
+};
 
 /// BLEND false: a time weight of 0, where s0 + 0 (s1 - s0) is s0 itself
 /// (the sign of a zero sum aside, for which s1 is read), so the second time
 /// level is not read. Identical to the blended form whenever the second
 /// level is finite.
-template <class S, bool BLEND>
+/// The eight corners lie in four pairs of x neighbours (a patch keeps a cell
+/// away from the coarse domain's x and y faces, so only z wraps): four cell
+/// indices, the second of a pair one element on.
+/// EVERY: the targets are all the fine level's cells that are not solid
+/// (`targets` its kind bytes), and the values go to both buffers, `twin`
+/// elements apart.
+template <class S, bool BLEND, bool EVERY>
 __global__ void __launch_bounds__(kRefineBlock)
-fill_kernel(const typename S::T* __restrict__ cT0, const typename S::T* __restrict__ cT1,
-            const std::uint8_t* __restrict__ ckind, typename S::T* __restrict__ ff,
-            const std::uint32_t* __restrict__ targets, int count, RefineGeom g, float invFactor,
-            float tw, float neqScale, FastDiv divX, FastDiv divXY) {
+fill_kernel(const __grid_constant__ FillPtrs<typename S::T> fp, const std::uint8_t* __restrict__ ckind,
+            const void* __restrict__ targets, unsigned count, RefineGeom g, float invFactor, float tw, float neqScale,
+            FastDiv divX, FastDiv divXY, long long twin) {
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    const std::uint32_t t = targets[i];
-    const int zf = static_cast<int>(fdiv(t, divXY));
-    const unsigned rem = t - static_cast<unsigned>(zf) * divXY.d;
-    const int yf = static_cast<int>(fdiv(rem, divX));
-    const int xf = static_cast<int>(rem - static_cast<unsigned>(yf) * divX.d);
+    std::uint32_t t = i;
+    if constexpr (EVERY) {
+        if ((static_cast<const std::uint8_t*>(targets)[i] & kFlagMask) == kSolid) return;
+    } else {
+        t = static_cast<const std::uint32_t*>(targets)[i];
+    }
+    const unsigned zu = fdiv(t, divXY);
+    const unsigned rem = t - zu * divXY.d;
+    const unsigned yu = fdiv(rem, divX);
+    const int zf = static_cast<int>(zu), yf = static_cast<int>(yu), xf = static_cast<int>(rem - yu * divX.d);
 
     const float gx = static_cast<float>(g.boxX0) + (static_cast<float>(xf) + 0.5f) * invFactor - 0.5f;
     const float gy = static_cast<float>(g.boxY0) + (static_cast<float>(yf) + 0.5f) * invFactor - 0.5f;
@@ -100,16 +136,16 @@ fill_kernel(const typename S::T* __restrict__ cT0, const typename S::T* __restri
     w8[5] = tx * (1 - ty) * tz;
     w8[6] = (1 - tx) * ty * tz;
     w8[7] = tx * ty * tz;
-    const int cnx = g.coarse.nx, cny = g.coarse.ny, cnz = g.coarse.nz;
-    std::uint32_t corner[8];
+    const unsigned cnx = g.coarse.nx, cny = g.coarse.ny;
+    std::uint32_t row[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        row[r] = static_cast<unsigned>(ix) + cnx * (static_cast<unsigned>(iy + (r & 1))
+                                                    + cny * static_cast<unsigned>(wrap1(iz + (r >> 1), g.coarse.nz)));
     float wsum = 0.0f;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-        const int X = wrap1(ix + (c & 1), cnx), Y = wrap1(iy + ((c >> 1) & 1), cny);
-        const int Z = wrap1(iz + ((c >> 2) & 1), cnz);
-        corner[c] = static_cast<std::uint32_t>(X) + static_cast<std::uint32_t>(cnx)
-                  * (static_cast<std::uint32_t>(Y) + static_cast<std::uint32_t>(cny) * Z);
-        if ((ckind[corner[c]] & kFlagMask) == kSolid) w8[c] = 0.0f;
+        if ((ckind[row[c >> 1] + (c & 1)] & kFlagMask) == kSolid) w8[c] = 0.0f;
         wsum += w8[c];
     }
     if (wsum < 1e-6f) return; // fully inside a parent solid: leave it
@@ -117,7 +153,6 @@ fill_kernel(const typename S::T* __restrict__ cT0, const typename S::T* __restri
 #pragma unroll
     for (int c = 0; c < 8; ++c) w8[c] *= iws;
 
-    const long long cn = g.coarse.cells(), fn = g.fine.cells();
     float fi[kQ];
     // FP16 storage sums the stored deviations and adds w_q once: with the
     // corner weights summing to one, sum w8 (w_q + g) = w_q + sum w8 g up to
@@ -127,26 +162,25 @@ fill_kernel(const typename S::T* __restrict__ cT0, const typename S::T* __restri
 #pragma unroll
     for (int q = 0; q < kQ; ++q) {
         float s0 = 0.0f, s1 = 0.0f;
-        if constexpr (kDev) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                s0 += w8[c] * S::ld_dev(cT0 + q * cn, corner[c], wgt(q));
-                if constexpr (BLEND) s1 += w8[c] * S::ld_dev(cT1 + q * cn, corner[c], wgt(q));
+        for (int c = 0; c < 8; ++c) {
+            const unsigned e = row[c >> 1];
+            if constexpr (kDev) {
+                s0 += w8[c] * S::ld_dev(fp.t0[q] + e, c & 1, wgt(q));
+                if constexpr (BLEND) s1 += w8[c] * S::ld_dev(fp.t1[q] + e, c & 1, wgt(q));
+            } else {
+                s0 += w8[c] * S::ld(fp.t0[q] + e, c & 1, wgt(q));
+                if constexpr (BLEND) s1 += w8[c] * S::ld(fp.t1[q] + e, c & 1, wgt(q));
             }
+        }
+        if constexpr (kDev) {
             fi[q] = wgt(q) + (BLEND ? s0 + tw * (s1 - s0) : s0);
         } else if constexpr (BLEND) {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                s0 += w8[c] * S::ld(cT0 + q * cn, corner[c], wgt(q));
-                s1 += w8[c] * S::ld(cT1 + q * cn, corner[c], wgt(q));
-            }
             fi[q] = s0 + tw * (s1 - s0);
         } else {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) s0 += w8[c] * S::ld(cT0 + q * cn, corner[c], wgt(q));
             if (s0 == 0.0f) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c) s1 += w8[c] * S::ld(cT1 + q * cn, corner[c], wgt(q));
+                for (int c = 0; c < 8; ++c) s1 += w8[c] * S::ld(fp.t1[q] + row[c >> 1], c & 1, wgt(q));
                 s0 = s0 + tw * (s1 - s0);
             }
             fi[q] = s0;
@@ -154,16 +188,17 @@ fill_kernel(const typename S::T* __restrict__ cT0, const typename S::T* __restri
     }
     float rho, ux, uy, uz;
     limited_moments(fi, rho, ux, uy, uz);
-    const float usq = 1.5f * (ux * ux + uy * uy + uz * uz);
-    float feq[kQ], fneq[kQ];
+    float feq[kQ];
+    feq_rn(rho, ux, uy, uz, feq);
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) fi[q] -= feq[q];
+    regularize(fi);
 #pragma unroll
     for (int q = 0; q < kQ; ++q) {
-        feq[q] = feq_q(q, rho, ux, uy, uz, usq);
-        fneq[q] = fi[q] - feq[q];
+        const float v = feq[q] + neqScale * fi[q];
+        S::st(fp.out[q], t, v, wgt(q));
+        if constexpr (EVERY) S::st(fp.out[q] + twin, t, v, wgt(q));
     }
-    regularize(fneq);
-#pragma unroll
-    for (int q = 0; q < kQ; ++q) S::st(ff + q * fn, t, feq[q] + neqScale * fneq[q], wgt(q));
 }
 
 /// Pass 1: child average of every coarse cell of the restricted sub-box, as
@@ -171,12 +206,11 @@ fill_kernel(const typename S::T* __restrict__ cT0, const typename S::T* __restri
 template <class S>
 __global__ void __launch_bounds__(kRefineBlock)
 child_avg_kernel(const typename S::T* __restrict__ ff, const std::uint8_t* __restrict__ fkind,
-                 RefineGeom g, int rx0, int ry0, int rw, int rh, float* __restrict__ scratch) {
+                 RefineGeom g, int rx0, int ry0, RecordGrid rg, float* __restrict__ scratch) {
     pdl_wait();
     const int lx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lx >= rw) return;
+    if (lx >= rg.w) return;
     const int ly = blockIdx.y, zc = blockIdx.z;
-    const long long t = lx + static_cast<long long>(rw) * (ly + static_cast<long long>(rh) * zc);
     const int m = g.factor;
     const int fx = m * (rx0 + lx - g.boxX0), fy = m * (ry0 + ly - g.boxY0), fz = m * zc;
     const long long fn = g.fine.cells();
@@ -195,8 +229,15 @@ child_avg_kernel(const typename S::T* __restrict__ ff, const std::uint8_t* __res
 #pragma unroll
                 for (int q = 0; q < kQ; ++q) fi[q] += S::ld(ff + q * fn, c, wgt(q));
             }
-    const long long nrec = static_cast<long long>(rw) * rh * g.coarse.nz;
-    write_child_record<S>(fi, nFluid, reinterpret_cast<float4*>(scratch) + t, nrec);
+    write_child_record<S>(fi, nFluid, reinterpret_cast<float4*>(scratch) + rg.index(lx, ly, zc),
+                          rg.count(g.coarse.nz));
+}
+
+/// Every record of a new scratch without fluid children (the border stays so).
+template <class S>
+__global__ void __launch_bounds__(kRefineBlock) clear_records_kernel(float* __restrict__ scratch, unsigned count) {
+    const unsigned t = blockIdx.x * kRefineBlock + threadIdx.x;
+    if (t < count) ChildRecord<S>::write_invalid(reinterpret_cast<float4*>(scratch) + t, count);
 }
 
 constexpr int kRestrictTX = 32, kRestrictTY = 2, kRestrictTZ = 2;
@@ -204,58 +245,59 @@ constexpr int kRestrictTX = 32, kRestrictTY = 2, kRestrictTZ = 2;
 template <class S>
 __global__ void __launch_bounds__(kRestrictTX * kRestrictTY * kRestrictTZ)
 restrict_kernel(typename S::T* __restrict__ fc, const std::uint8_t* __restrict__ ckind,
-                RefineGeom g, int rx0, int ry0, int rw, int rh, float neqScaleInv,
-                const float* __restrict__ scratch, float* __restrict__ mRho,
+                RefineGeom g, int rx0, int ry0, RecordGrid rg, float neqScaleInv,
+                const __grid_constant__ RecordPlanes rec, float* __restrict__ mRho,
                 float* __restrict__ mU, float* __restrict__ mV, float* __restrict__ mW) {
     pdl_wait();
     const int lx = blockIdx.x * kRestrictTX + threadIdx.x;
     const int ly = blockIdx.y * kRestrictTY + threadIdx.y;
     const int zc = blockIdx.z * kRestrictTZ + threadIdx.z;
     const int nz = g.coarse.nz;
-    if (lx >= rw || ly >= rh || zc >= nz) return;
-    const long long t = lx + static_cast<long long>(rw) * (ly + static_cast<long long>(rh) * zc);
+    if (lx >= rg.w || ly >= rg.h || zc >= nz) return;
+    const unsigned t = rg.index(lx, ly, zc);
     const int xc = rx0 + lx, yc = ry0 + ly;
     const long long cn = g.coarse.cells();
     const unsigned cell = static_cast<unsigned>(xc) + static_cast<unsigned>(g.coarse.nx)
                         * (static_cast<unsigned>(yc) + static_cast<unsigned>(g.coarse.ny) * zc);
     if ((ckind[cell] & kFlagMask) != kFluid) return;
-    const float4* rec = reinterpret_cast<const float4*>(scratch);
-    const long long nrec = static_cast<long long>(rw) * rh * nz;
-    float fneq[kQ];
-    if (!ChildRecord<S>::load(rec + t, nrec, fneq)) return;
+    float fneq[kQ], stencil;
+    ChildRecord<S>::template add<true>(rec, t, fneq, stencil);
+    if (stencil == 0.0f) return;
 
-    const int dEdge = min(min(lx, rw - 1 - lx), min(ly, rh - 1 - ly));
+    const int dEdge = min(min(lx, rg.w - 1 - lx), min(ly, rg.h - 1 - ly));
     const float blend = fminf(1.0f, static_cast<float>(dEdge + 1) / static_cast<float>(kRestrictBlend + 1));
 
-    int nStencil = 1;
+    // The neighbours in the reference's order. A record in the border or
+    // without fluid children adds nothing, so no load waits on a test.
+    const int zm = zc == 0 ? nz - 1 : zc - 1, zp = zc == nz - 1 ? 0 : zc + 1;
 #pragma unroll
-    for (int nb = 1; nb < kQ; ++nb) {
-        const int nlx = lx + cx(nb), nly = ly + cy(nb);
-        // A neighbour outside the box reads the cell's own record and is
-        // dropped by the select, so no neighbour's loads wait on a branch.
-        const bool inBox = nlx >= 0 && nlx < rw && nly >= 0 && nly < rh;
-        const int nzw = zc + cz(nb) < 0 ? nz - 1 : (zc + cz(nb) >= nz ? 0 : zc + cz(nb));
-        const long long tn = inBox ? nlx + static_cast<long long>(rw) * (nly + static_cast<long long>(rh) * nzw) : t;
-        // Same per-q accumulation order as summing slot by slot.
-        nStencil += ChildRecord<S>::add_sel(rec + tn, nrec, fneq, inBox) ? 1 : 0;
-    }
-    const float invS = 1.0f / static_cast<float>(nStencil);
+    for (int nb = 1; nb < kQ; ++nb)
+        ChildRecord<S>::template add<false>(
+            rec, rg.index(lx + cx(nb), ly + cy(nb), cz(nb) < 0 ? zm : (cz(nb) > 0 ? zp : zc)), fneq, stencil);
+    const float invS = 1.0f / stencil;
 #pragma unroll
     for (int q = 0; q < kQ; ++q) fneq[q] *= invS;
     regularize(fneq);
-    const float4 m4 = ChildRecord<S>::moments(rec + t, nrec);
-    const float rho = m4.x, ux = m4.y, uy = m4.z, uz = m4.w;
-    const float usq = 1.5f * (ux * ux + uy * uy + uz * uz);
-    float br = 0.f, bjx = 0.f, bjy = 0.f, bjz = 0.f;
+    const float4 m4 = ChildRecord<S>::moments(rec, t);
+    float feq[kQ];
+    feq_rn(m4.x, m4.y, m4.z, m4.w, feq);
+    float b[kQ];
 #pragma unroll
     for (int q = 0; q < kQ; ++q) {
-        const float restricted = feq_q(q, rho, ux, uy, uz, usq) + neqScaleInv * fneq[q];
+        const float restricted = feq[q] + neqScaleInv * fneq[q];
         const float existing = S::ld(fc + q * cn, cell, wgt(q));
-        const float b = existing + blend * (restricted - existing);
-        S::st(fc + q * cn, cell, b, wgt(q));
-        br += b; bjx += cx(q) * b; bjy += cy(q) * b; bjz += cz(q) * b;
+        b[q] = existing + blend * (restricted - existing);
+        S::st(fc + q * cn, cell, b[q], wgt(q));
     }
     if (mRho) {
+        float br = b[0], bjx = b[1], bjy = b[3], bjz = b[5];
+#pragma unroll
+        for (int q = 1; q < kQ; ++q) {
+            br += b[q];
+            if (cx(q) != 0 && q != 1) bjx = cx(q) > 0 ? bjx + b[q] : bjx - b[q];
+            if (cy(q) != 0 && q != 3) bjy = cy(q) > 0 ? bjy + b[q] : bjy - b[q];
+            if (cz(q) != 0 && q != 5) bjz = cz(q) > 0 ? bjz + b[q] : bjz - b[q];
+        }
         br = fmaxf(br, kRhoFloor);
         const float bi = 1.0f / br;
         mRho[cell] = br; mU[cell] = bjx * bi; mV[cell] = bjy * bi; mW[cell] = bjz * bi;
@@ -271,6 +313,21 @@ inline void sub_box(const RefineGeom& g, int& rx0, int& ry0, int& rw, int& rh) {
 
 } // namespace
 
+template <class S, bool EVERY>
+static cudaError_t launch_fill_impl(const void* cT0, const void* cT1, const std::uint8_t* coarseKind, void* fineF,
+                                    const void* targets, long long count, const RefineGeom& g, float timeWeight,
+                                    float neqScale, long long twin, cudaStream_t st) {
+    using T = typename S::T;
+    const FillPtrs<T> fp(static_cast<const T*>(cT0), static_cast<const T*>(cT1), static_cast<T*>(fineF),
+                         g.coarse.cells(), g.fine.cells());
+    const unsigned nb = static_cast<unsigned>((count + kRefineBlock - 1) / kRefineBlock);
+    const FastDiv dx = fast_div(static_cast<unsigned>(g.fine.nx));
+    const FastDiv dxy = fast_div(static_cast<unsigned>(g.fine.nx) * static_cast<unsigned>(g.fine.ny));
+    auto kern = !EVERY && timeWeight != 0.0f ? fill_kernel<S, !EVERY, EVERY> : fill_kernel<S, false, EVERY>;
+    return launch_pdl(kern, nb, kRefineBlock, st, fp, coarseKind, targets, static_cast<unsigned>(count), g,
+                      1.0f / static_cast<float>(g.factor), timeWeight, neqScale, dx, dxy, twin);
+}
+
 cudaError_t launch_fill_c2f(Storage s, const void* cT0, const void* cT1,
                             const std::uint8_t* coarseKind, void* fineF,
                             const std::uint32_t* targets, int count, const RefineGeom& g,
@@ -278,61 +335,79 @@ cudaError_t launch_fill_c2f(Storage s, const void* cT0, const void* cT1,
     if (!cT0 || !cT1 || !coarseKind || !fineF || g.factor < 2 || g.factor > 4)
         return cudaErrorInvalidValue;
     if (count <= 0) return cudaSuccess;
-    const unsigned nb = static_cast<unsigned>((count + kRefineBlock - 1) / kRefineBlock);
-    const float invF = 1.0f / static_cast<float>(g.factor);
-    const bool blend = timeWeight != 0.0f;
-    const FastDiv dx = fast_div(static_cast<unsigned>(g.fine.nx));
-    const FastDiv dxy = fast_div(static_cast<unsigned>(g.fine.nx) * static_cast<unsigned>(g.fine.ny));
-    if (s == Storage::F32)
-        return launch_pdl(blend ? fill_kernel<StoreF32, true> : fill_kernel<StoreF32, false>, nb, kRefineBlock, st,
-                          static_cast<const float*>(cT0), static_cast<const float*>(cT1), coarseKind,
-                          static_cast<float*>(fineF), targets, count, g, invF, timeWeight, neqScale, dx, dxy);
-    return launch_pdl(blend ? fill_kernel<StoreF16, true> : fill_kernel<StoreF16, false>, nb, kRefineBlock, st,
-                      static_cast<const __half*>(cT0), static_cast<const __half*>(cT1), coarseKind,
-                      static_cast<__half*>(fineF), targets, count, g, invF, timeWeight, neqScale, dx, dxy);
+    return (s == Storage::F32 ? launch_fill_impl<StoreF32, false> : launch_fill_impl<StoreF16, false>)(
+        cT0, cT1, coarseKind, fineF, targets, count, g, timeWeight, neqScale, 0, st);
+}
+
+cudaError_t launch_seed_c2f(Storage s, const void* coarseF, const std::uint8_t* coarseKind, void* fine0, void* fine1,
+                            const std::uint8_t* fineKind, const RefineGeom& g, float neqScale, cudaStream_t st) {
+    if (!coarseF || !coarseKind || !fine0 || !fine1 || !fineKind || g.factor < 2 || g.factor > 4)
+        return cudaErrorInvalidValue;
+    const long long bytes = static_cast<char*>(fine1) - static_cast<char*>(fine0);
+    return (s == Storage::F32 ? launch_fill_impl<StoreF32, true> : launch_fill_impl<StoreF16, true>)(
+        coarseF, coarseF, coarseKind, fine0, fineKind, g.fine.cells(), g, 0.0f, neqScale,
+        bytes / (s == Storage::F32 ? 4 : 2), st);
+}
+
+static RecordGrid record_grid(const RefineGeom& g, int& rx0, int& ry0) {
+    RecordGrid rg;
+    sub_box(g, rx0, ry0, rg.w, rg.h);
+    return rg;
 }
 
 long long restrict_scratch_floats(const RefineGeom& g) {
-    int rx0, ry0, rw, rh;
-    sub_box(g, rx0, ry0, rw, rh);
-    if (rw <= 0 || rh <= 0) return 0;
-    return static_cast<long long>(kScratchVals) * rw * rh * g.coarse.nz;
+    int rx0, ry0;
+    const RecordGrid rg = record_grid(g, rx0, ry0);
+    if (rg.w <= 0 || rg.h <= 0) return 0;
+    return kScratchVals * rg.count(g.coarse.nz);
+}
+
+cudaError_t launch_clear_scratch(Storage s, const RefineGeom& g, float* scratch, cudaStream_t st) {
+    int rx0, ry0;
+    const long long n = record_grid(g, rx0, ry0).count(g.coarse.nz);
+    if (!scratch || n <= 0) return cudaErrorInvalidValue;
+    const unsigned nb = static_cast<unsigned>((n + kRefineBlock - 1) / kRefineBlock);
+    if (s == Storage::F32) clear_records_kernel<StoreF32><<<nb, kRefineBlock, 0, st>>>(scratch, static_cast<unsigned>(n));
+    else clear_records_kernel<StoreF16><<<nb, kRefineBlock, 0, st>>>(scratch, static_cast<unsigned>(n));
+    return cudaGetLastError();
 }
 
 void restrict_sub_box(const RefineGeom& g, int& rx0, int& ry0, int& rw, int& rh) { sub_box(g, rx0, ry0, rw, rh); }
+
+template <class S>
+static cudaError_t launch_restrict_impl(const void* fineF, const std::uint8_t* fineKind, void* coarseF,
+                                        const std::uint8_t* coarseKind, const RefineGeom& g, float neqScaleInv,
+                                        float* scratch, float* rho, float* u, float* v, float* w, cudaStream_t st,
+                                        bool childDone) {
+    using T = typename S::T;
+    int rx0, ry0;
+    const RecordGrid rg = record_grid(g, rx0, ry0);
+    if (rg.w <= 0 || rg.h <= 0) return cudaErrorInvalidValue;
+    if (!childDone) {
+        const dim3 grid(static_cast<unsigned>((rg.w + kRefineBlock - 1) / kRefineBlock), static_cast<unsigned>(rg.h),
+                        static_cast<unsigned>(g.coarse.nz));
+        if (auto e = launch_pdl(child_avg_kernel<S>, grid, kRefineBlock, st, static_cast<const T*>(fineF), fineKind, g,
+                                rx0, ry0, rg, scratch);
+            e != cudaSuccess)
+            return e;
+    }
+    const dim3 block(kRestrictTX, kRestrictTY, kRestrictTZ);
+    const dim3 grid(static_cast<unsigned>((rg.w + kRestrictTX - 1) / kRestrictTX),
+                    static_cast<unsigned>((rg.h + kRestrictTY - 1) / kRestrictTY),
+                    static_cast<unsigned>((g.coarse.nz + kRestrictTZ - 1) / kRestrictTZ));
+    return launch_pdl(restrict_kernel<S>, grid, block, st, static_cast<T*>(coarseF), coarseKind, g, rx0, ry0, rg,
+                      neqScaleInv, RecordPlanes::of(scratch, rg.count(g.coarse.nz)), u && v && w ? rho : nullptr, u, v,
+                      w);
+}
 
 cudaError_t launch_restrict_f2c(Storage s, const void* fineF, const std::uint8_t* fineKind,
                                 void* coarseF, const std::uint8_t* coarseKind,
                                 const RefineGeom& g, float neqScaleInv, float* scratch,
                                 float* rho, float* u, float* v, float* w, cudaStream_t st, bool childDone) {
-    int rx0, ry0, rw, rh;
-    sub_box(g, rx0, ry0, rw, rh);
-    if (!fineF || !fineKind || !coarseF || !coarseKind || !scratch || rw <= 0 || rh <= 0
-        || g.factor < 2 || g.factor > 4)
+    if (!fineF || !fineKind || !coarseF || !coarseKind || !scratch || g.factor < 2 || g.factor > 4)
         return cudaErrorInvalidValue;
-    const dim3 grid(static_cast<unsigned>((rw + kRefineBlock - 1) / kRefineBlock),
-                    static_cast<unsigned>(rh), static_cast<unsigned>(g.coarse.nz));
-    const bool macro = rho && u && v && w;
-    const dim3 rblock(kRestrictTX, kRestrictTY, kRestrictTZ);
-    const dim3 rgrid(static_cast<unsigned>((rw + kRestrictTX - 1) / kRestrictTX),
-                     static_cast<unsigned>((rh + kRestrictTY - 1) / kRestrictTY),
-                     static_cast<unsigned>((g.coarse.nz + kRestrictTZ - 1) / kRestrictTZ));
-    if (s == Storage::F32) {
-        if (!childDone)
-            if (auto e = launch_pdl(child_avg_kernel<StoreF32>, grid, kRefineBlock, st, static_cast<const float*>(fineF),
-                                    fineKind, g, rx0, ry0, rw, rh, scratch);
-                e != cudaSuccess)
-                return e;
-        return launch_pdl(restrict_kernel<StoreF32>, rgrid, rblock, st, static_cast<float*>(coarseF), coarseKind, g, rx0,
-                          ry0, rw, rh, neqScaleInv, scratch, macro ? rho : nullptr, u, v, w);
-    }
-    if (!childDone)
-        if (auto e = launch_pdl(child_avg_kernel<StoreF16>, grid, kRefineBlock, st, static_cast<const __half*>(fineF),
-                                fineKind, g, rx0, ry0, rw, rh, scratch);
-            e != cudaSuccess)
-            return e;
-    return launch_pdl(restrict_kernel<StoreF16>, rgrid, rblock, st, static_cast<__half*>(coarseF), coarseKind, g, rx0,
-                      ry0, rw, rh, neqScaleInv, scratch, macro ? rho : nullptr, u, v, w);
+    return (s == Storage::F32 ? launch_restrict_impl<StoreF32> : launch_restrict_impl<StoreF16>)(
+        fineF, fineKind, coarseF, coarseKind, g, neqScaleInv, scratch, rho, u, v, w, st, childDone);
 }
 
 } // namespace fcfd

@@ -231,8 +231,8 @@ struct fcfd_solver {
     bool finerActive = false;
     int finerFactor = 2;
     fcfd_patch_box finerBox{};
-    std::uint32_t *dShellFiner = nullptr, *dSeedFiner = nullptr;
-    int shellCountFiner = 0, seedCountFiner = 0;
+    std::uint32_t* dShellFiner = nullptr;
+    int shellCountFiner = 0;
     std::uint64_t flagsHashCache = 0;   // FNV-1a of coarse.hostFlags
     bool flagsHashValid = false;
     float* dScratchFiner = nullptr;
@@ -241,8 +241,6 @@ struct fcfd_solver {
     // The fine level's fill covers every interface cell while a finer box
     // reaches its outer shell layer (the finer fill gathers from there).
     bool fineShellFull = false;
-    std::uint32_t* dSeed = nullptr;
-    int seedCount = 0;
     float* dScratch = nullptr;
     bool forcesFromFine = false;
 
@@ -417,7 +415,7 @@ struct fcfd_solver {
     /// level while a finer level nests in it, whose fill may gather from
     /// the fine shell) every interface cell.
     cudaError_t shellList(const Level& L, bool full, std::uint32_t** out, int* count) {
-        if (full) return cellList(L, FCFD_FLAG_INTERFACE, true, out, count);
+        if (full) return cellList(L, FCFD_FLAG_INTERFACE, out, count);
         dfree(*out);
         *count = 0;
         long long c = 0;
@@ -433,20 +431,20 @@ struct fcfd_solver {
         return cudaSuccess;
     }
 
-    /// Ascending list of the level's cells whose flag equals (or, with
-    /// equal false, differs from) `value`, into a fresh device array.
-    cudaError_t cellList(const Level& L, std::uint8_t value, bool equal, std::uint32_t** out, int* count) {
+    /// Ascending list of the level's cells whose flag equals `value`, into a
+    /// fresh device array.
+    cudaError_t cellList(const Level& L, std::uint8_t value, std::uint32_t** out, int* count) {
         dfree(*out);
         *count = 0;
         long long c = 0;
         launches += 2;
-        if (auto e = device_cells_where(L.d, L.flags, value, equal, nullptr, 0, &c, stream); e != cudaSuccess)
+        if (auto e = device_cells_where(L.d, L.flags, value, nullptr, 0, &c, stream); e != cudaSuccess)
             return e;
         if (auto e = dalloc(out, static_cast<size_t>(c) * 4); e != cudaSuccess) return e;
         if (c > 0) {
             launches += 3;
             long long again = 0;
-            if (auto e = device_cells_where(L.d, L.flags, value, equal, *out, c, &again, stream); e != cudaSuccess)
+            if (auto e = device_cells_where(L.d, L.flags, value, *out, c, &again, stream); e != cudaSuccess)
                 return e;
         }
         *count = static_cast<int>(c);
@@ -535,36 +533,24 @@ struct fcfd_solver {
     cudaError_t seedFiner() {
         if (!finerActive) return cudaSuccess;
         const float tf = fineTau(effTau(), factor), tr = fineTau(tf, finerFactor);
-        for (int i = 0; i < 2; ++i) {
-            ++launches;
-            if (auto e = launch_fill_c2f(storage, fine.f[fine.src], fine.f[fine.src], fine.kind, finer.f[i],
-                                         dSeedFiner, seedCountFiner, geomFiner(), 0.0f,
-                                         tr / (static_cast<float>(finerFactor) * tf), stream);
-                e != cudaSuccess)
-                return e;
-        }
-        return cudaSuccess;
+        ++launches;
+        return launch_seed_c2f(storage, fine.f[fine.src], fine.kind, finer.f[0], finer.f[1], finer.kind, geomFiner(),
+                               tr / (static_cast<float>(finerFactor) * tf), stream);
     }
 
     void freeFiner() {
         finer.free_all();
-        dfree(dShellFiner); dfree(dSeedFiner); dfree(dScratchFiner);
-        shellCountFiner = seedCountFiner = 0;
+        dfree(dShellFiner); dfree(dScratchFiner);
+        shellCountFiner = 0;
         finerActive = false;
     }
 
     cudaError_t seedFine() {
         if (!fineActive) return cudaSuccess;
         const float tc = effTau(), tf = fineTau(tc, factor);
-        for (int i = 0; i < 2; ++i) {
-            ++launches;
-            if (auto e = launch_fill_c2f(storage, coarse.f[coarse.src], coarse.f[coarse.src], coarse.kind,
-                                         fine.f[i], dSeed, seedCount, geom(), 0.0f,
-                                         tf / (static_cast<float>(factor) * tc), stream);
-                e != cudaSuccess)
-                return e;
-        }
-        return cudaSuccess;
+        ++launches;
+        return launch_seed_c2f(storage, coarse.f[coarse.src], coarse.kind, fine.f[0], fine.f[1], fine.kind, geom(),
+                               tf / (static_cast<float>(factor) * tc), stream);
     }
 
     /// Forces come from the fine level when every coarse solid cell lies in
@@ -583,8 +569,8 @@ struct fcfd_solver {
     void freeFine() {
         freeFiner();  // the finer level nests in the fine one
         fine.free_all();
-        dfree(dShell); dfree(dSeed); dfree(dScratch);
-        shellCount = seedCount = 0;
+        dfree(dShell); dfree(dScratch);
+        shellCount = 0;
         fineShellFull = false;
         fineActive = false;
         forcesFromFine = false;
@@ -1600,13 +1586,14 @@ int fcfd_init_refinement(fcfd_solver* s, const fcfd_patch_box* box, int factor, 
     if (auto e = s->uploadLevelFlags(s->fine, ff); e != cudaSuccess) return fail("fine flag upload failed", e);
     if (auto e = s->shellList(s->fine, false, &s->dShell, &s->shellCount); e != cudaSuccess)
         return fail("shell list failed", e);
-    if (auto e = s->cellList(s->fine, FCFD_FLAG_SOLID, false, &s->dSeed, &s->seedCount); e != cudaSuccess)
-        return fail("seed list failed", e);
     s->fineActive = true;
     const long long sf = restrict_scratch_floats(s->geom());
     if (sf <= 0) return fail("restriction sub-box is empty", cudaErrorInvalidValue);
     if (auto e = dalloc(&s->dScratch, static_cast<size_t>(sf) * 4); e != cudaSuccess)
         return fail("restriction scratch allocation failed", e);
+    ++s->launches;
+    if (auto e = launch_clear_scratch(s->storage, s->geom(), s->dScratch, s->stream); e != cudaSuccess)
+        return fail("restriction scratch set-up failed", e);
     s->updateForcesFromFine();
     if (auto e = s->buildWM(s->fine, kWallSampleFine); e != cudaSuccess) return fail("fine wall list failed", e);
     if (auto e = s->seedFine(); e != cudaSuccess) return fail("fine level seeding failed", e);
@@ -1626,7 +1613,6 @@ int fcfd_set_refined_flags(fcfd_solver* s, const uint8_t* ff, size_t n) {
         return cudaErrorInvalidValue;
     if (auto e = s->uploadLevelFlags(s->fine, ff); e != cudaSuccess) return e;
     if (auto e = s->shellList(s->fine, s->fineShellFull, &s->dShell, &s->shellCount); e != cudaSuccess) return e;
-    if (auto e = s->cellList(s->fine, FCFD_FLAG_SOLID, false, &s->dSeed, &s->seedCount); e != cudaSuccess) return e;
     s->updateForcesFromFine();
     if (auto e = s->buildWM(s->fine, kWallSampleFine); e != cudaSuccess) return e;
     if (auto e = s->seedFine(); e != cudaSuccess) return e;
@@ -1909,8 +1895,7 @@ int fcfd_q_link_info(fcfd_solver* s, int level, int* active, int* links, int* fa
 
 /// Interface-shell and seed lists of the finer level (its flags uploaded).
 static int finer_lists(fcfd_solver* s) {
-    if (auto e = s->shellList(s->finer, false, &s->dShellFiner, &s->shellCountFiner); e != cudaSuccess) return e;
-    return s->cellList(s->finer, FCFD_FLAG_SOLID, false, &s->dSeedFiner, &s->seedCountFiner);
+    return s->shellList(s->finer, false, &s->dShellFiner, &s->shellCountFiner);
 }
 
 int fcfd_init_finer_refinement(fcfd_solver* s, const fcfd_patch_box* box, int factor, const uint8_t* ff,
@@ -1972,6 +1957,9 @@ int fcfd_init_finer_refinement(fcfd_solver* s, const fcfd_patch_box* box, int fa
     if (sf <= 0) return fail("finer restriction sub-box is empty", cudaErrorInvalidValue);
     if (auto e = dalloc(&s->dScratchFiner, static_cast<size_t>(sf) * 4); e != cudaSuccess)
         return fail("finer restriction scratch allocation failed", e);
+    ++s->launches;
+    if (auto e = launch_clear_scratch(s->storage, s->geomFiner(), s->dScratchFiner, s->stream); e != cudaSuccess)
+        return fail("finer restriction scratch set-up failed", e);
     if (auto e = s->buildWM(s->finer, kWallSampleFine); e != cudaSuccess) return fail("finer wall list failed", e);
     if (auto e = s->seedFiner(); e != cudaSuccess) return fail("finer level seeding failed", e);
     if (auto e = cudaStreamSynchronize(s->stream); e != cudaSuccess) return fail("finer level seeding failed", e);
