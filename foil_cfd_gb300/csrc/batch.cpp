@@ -4,7 +4,7 @@
 // launch-shape autotuner.
 //
 // Per tunnel the set-up follows the single-tunnel solver: flags -> kind
-// bytes (launch_classify), compact force-link list (device compaction),
+// bytes and compact force-link list (build_level_tables),
 // uniform-flow reset feq(1, u) + the reference's speck perturbation
 // (src/sim/lbm_solver.cpp:49, 896-935) on both buffers.
 #include "../../include/foilcfd_batch.h"
@@ -344,6 +344,7 @@ int fcfd_batch_init(fcfd_batch* b, const fcfd_batch_tunnel* tunnels, int count, 
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t esz = b->storage == Storage::F32 ? 4 : 2;
     int maxLinks = 0;
+    GeomScratch scratch;   // of the flag tables; one tunnel after the other on the batch's stream
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < count && e == cudaSuccess; ++i) {
         const fcfd_batch_tunnel& in = tunnels[i];
@@ -352,6 +353,7 @@ int fcfd_batch_init(fcfd_batch* b, const fcfd_batch_tunnel* tunnels, int count, 
         x.n = x.d.cells();
         if (x.d.nx < 3 || x.d.ny < 3 || x.d.nz < 1 || !in.flags || x.n >= (1LL << 31) / 19) {
             set_err(err, errlen, "bad tunnel dims or flags");
+            scratch.release();
             b->freeAll();
             return cudaErrorInvalidValue;
         }
@@ -370,16 +372,19 @@ int fcfd_batch_init(fcfd_batch* b, const fcfd_batch_tunnel* tunnels, int count, 
         if (e == cudaSuccess)
             e = cudaMemcpy(y.flags, in.flags, static_cast<size_t>(y.n),
                            is_device_pointer(in.flags) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = launch_classify(y.flags, y.kind, y.d, b->stream, y.links);
-        long long links = 0, again = 0;
-        if (e == cudaSuccess) e = device_force_links(y.d, y.flags, nullptr, nullptr, 0, &links, b->stream);
-        y.linkCount = static_cast<int>(links);
-        maxLinks = std::max(maxLinks, y.linkCount);
-        if (e == cudaSuccess) e = cudaMalloc(&y.linkCells, std::max<size_t>(4, static_cast<size_t>(links) * 4));
-        if (e == cudaSuccess) e = cudaMalloc(&y.linkMasks, std::max<size_t>(4, static_cast<size_t>(links) * 4));
-        if (e == cudaSuccess && links > 0)
-            e = device_force_links(y.d, y.flags, y.linkCells, y.linkMasks, links, &again, b->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);   // a device copy does not wait, and the batch has its own stream
+        if (e == cudaSuccess) {
+            LevelTables t;
+            t.kind = y.kind;
+            t.links = y.links;
+            e = build_level_tables(y.d, y.flags, t, scratch, b->stream);
+            y.linkCells = t.linkCells;
+            y.linkMasks = t.linkMasks;
+            y.linkCount = static_cast<int>(t.linkCount);
+            maxLinks = std::max(maxLinks, y.linkCount);
+        }
     }
+    scratch.release();
     if (e == cudaSuccess) e = cudaMalloc(&b->dPartials, std::max(1, force_blocks(maxLinks)) * 3 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->dForceCur, 3 * count * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->dHist, static_cast<size_t>(kHistCapacity) * 3 * count * sizeof(double));

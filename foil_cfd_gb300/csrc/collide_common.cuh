@@ -56,7 +56,7 @@ struct CollideArgs {
     int* status; // staged kernel: nonzero when a pipeline wait timed out
     const std::uint8_t* qFrac;   // q-LIBB cut bytes [cell * 19 + q], or null
     const std::uint32_t* ffMask; // q-LIBB two-node bits [cell]
-    const uint2* links;          // pull-link classes per cell (launch_classify), or null
+    const uint2* links;          // pull-link classes per cell (build_level_tables), or null
 };
 
 /// Slice pointers of one launch, passed as a __grid_constant__ kernel

@@ -14,12 +14,17 @@
 //   so the pass is out of place without a copy) and the interface shell.
 // * Patch box (derivePatchBox, voxelizer.cpp:265-301): a min/max reduction
 //   of the solid cells' x and y.
-// * Cell lists in ascending cell order (ordered stream compaction: per-tile
-//   counts, one scan over the tiles, a scatter that re-evaluates the tile):
-//   the force-link list, the wall-model cell list of buildWallCellList
-//   (src/sim/wall_model.cpp:55-236: pull-solid link mask, vane exclusion,
-//   5^3 occupancy-gradient normal, sample cell along the normal), the
-//   interface-shell list of a refined level.
+// * Bit planes: one bit per cell and property (solid, fluid, ...), 32 cells of
+//   a row per word, built once per flag field. What depends on a cell's
+//   neighbours is then word arithmetic on 32 cells at a time.
+// * Level tables: kind bytes, pull-link classes, tile codes, cell classes and
+//   the solid bounding box of a level.
+// * Cell lists in ascending cell order: selection words, one scan over the
+//   tiles of 256 words, the selected cells, then one thread per entry for what
+//   an entry holds: the force-link list, the wall-model cell list of
+//   buildWallCellList (src/sim/wall_model.cpp:55-236: pull-solid link mask,
+//   vane exclusion, 5^3 occupancy-gradient normal, sample cell along the
+//   normal) and the interface-shell list of a refined level.
 //
 // Built without FMA contraction: the rasteriser's crossings and the wall
 // normals are the host builders' values bit for bit.
@@ -37,9 +42,6 @@ constexpr std::uint8_t kFluidB = 0, kSolidB = 1, kInletB = 2, kOutletB = 3, kSli
 constexpr std::uint8_t kInterfaceB = 8, kOutletEqB = 9;
 constexpr int kMaxCrossings = 64;      // per lattice row; more sets the error flag
 constexpr int kRowWarps = 4;           // rows per block of the rasteriser
-constexpr int kTileThreads = 256;      // compaction tile: 256 threads x 16 cells
-constexpr int kTileRun = 16;
-constexpr int kTileCells = kTileThreads * kTileRun;
 
 /// Periodic index for any offset (a sample search can step several
 /// periods on a thin span); equals the single wrap wherever that is in range.
@@ -177,284 +179,325 @@ __global__ void build_flags_kernel(FlagBuild b, std::uint8_t* __restrict__ out, 
     if (bal && (threadIdx.x & 31) == 0) atomicAdd(closed, __popc(bal));
 }
 
-// ---- solid bounding box -------------------------------------------------------
+// ---- bit planes -----------------------------------------------------------------
+// The old builders tested 18 neighbour bytes per cell, a thread running through
+// 16 cells one after the other: 0.56 ms per pass over a 42 M-cell patch. A word
+// of a plane holds 32 cells of a row, so the same test is about 20 loads and
+// 60 operations for 32 cells, and the planes of that patch (5.3 MB each) stay
+// in L2.
 
-__global__ void solid_bbox_kernel(const std::uint8_t* __restrict__ f, int nx, int ny, long long n,
-                                  int* __restrict__ box) {
-    int x0 = nx, x1 = -1, y0 = ny, y1 = -1;
-    for (long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; c < n;
-         c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        if (f[c] != kSolidB) continue;
-        const int x = static_cast<int>(c % nx);
-        const int y = static_cast<int>((c / nx) % ny);
-        x0 = min(x0, x); x1 = max(x1, x); y0 = min(y0, y); y1 = max(y1, y);
+struct BitGrid {
+    int nx, ny, nz, words;   // words per row
+    __host__ __device__ unsigned total() const {
+        return static_cast<unsigned>(words) * static_cast<unsigned>(ny) * static_cast<unsigned>(nz);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        x0 = min(x0, __shfl_xor_sync(0xffffffffu, x0, o));
-        x1 = max(x1, __shfl_xor_sync(0xffffffffu, x1, o));
-        y0 = min(y0, __shfl_xor_sync(0xffffffffu, y0, o));
-        y1 = max(y1, __shfl_xor_sync(0xffffffffu, y1, o));
-    }
-    if ((threadIdx.x & 31) == 0 && x1 >= 0) {
-        atomicMin(box + 0, x0); atomicMax(box + 2, x1);
-        atomicMin(box + 1, y0); atomicMax(box + 3, y1);
-    }
+};
+BitGrid bit_grid(LevelDims d) { return BitGrid{d.nx, d.ny, d.nz, (d.nx + 31) / 32}; }
+
+enum Plane { kPSolid, kPFluid, kPSlip, kPInlet, kPOutlet, kPInter, kPlanes };
+struct Planes {
+    std::uint32_t* p[kPlanes];   // null: not wanted
+};
+
+/// Four cells' matches of one byte value as four bits.
+__device__ __forceinline__ std::uint32_t match4(std::uint32_t cells, std::uint32_t value) {
+    return ((__vcmpeq4(cells, value * 0x01010101u) & 0x01010101u) * 0x10204080u) >> 28;
 }
 
-// ---- flag classes -------------------------------------------------------------
+/// One thread per word. ALIGN: bytes a row's words start on (16, 4 or 1).
+/// keep: the bits of a flag byte that count (the step looks at the low four).
+template <int ALIGN>
+__global__ void __launch_bounds__(256)
+planes_kernel(const std::uint8_t* __restrict__ flags, BitGrid g, Planes P, std::uint32_t keep) {
+    const unsigned wi = blockIdx.x * 256u + threadIdx.x;
+    if (wi >= g.total()) return;
+    const unsigned row = wi / g.words, x0 = 32u * (wi - row * g.words);
+    const std::uint8_t* f = flags + static_cast<size_t>(row) * g.nx + x0;
+    const int valid = min(32, g.nx - static_cast<int>(x0));
+    std::uint32_t c[8];
+    if (ALIGN == 16 && valid == 32) {
+        const uint4 a = reinterpret_cast<const uint4*>(f)[0], b = reinterpret_cast<const uint4*>(f)[1];
+        c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
+        c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            c[k] = 0xffffffffu;
+            if (ALIGN >= 4 && 4 * k + 4 <= valid) {
+                c[k] = reinterpret_cast<const std::uint32_t*>(f)[k];
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (4 * k + e < valid)
+                        c[k] = (c[k] & ~(0xffu << (8 * e))) | (static_cast<std::uint32_t>(f[4 * k + e]) << (8 * e));
+            }
+        }
+    }
+    std::uint32_t w[kPlanes] = {};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        c[k] &= keep;
+        w[kPSolid] |= match4(c[k], kSolidB) << (4 * k);
+        w[kPFluid] |= match4(c[k], kFluidB) << (4 * k);
+        w[kPInlet] |= match4(c[k], kInletB) << (4 * k);
+        w[kPOutlet] |= (match4(c[k], kOutletB) | match4(c[k], kOutletEqB)) << (4 * k);
+        w[kPInter] |= match4(c[k], kInterfaceB) << (4 * k);
+        w[kPSlip] |= match4(c[k] & 0xfcfcfcfcu, kSlipTopB) << (4 * k);   // 4..7
+    }
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p)
+        if (P.p[p]) P.p[p][wi] = w[p];
+}
 
-__global__ void flag_classes_kernel(const std::uint8_t* __restrict__ f, long long n,
-                                    unsigned long long* __restrict__ counts) {
-    unsigned long long rw = 0, in = 0, un = 0;
-    for (long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; c < n;
-         c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const std::uint8_t v = f[c];
-        if (v == kFluidB || v == kOutletB || v == kOutletEqB) ++rw;
-        else if (v == kInletB) ++in;
-        else ++un;
+/// Word w of row (y, z) of a plane with its neighbours x - 1 and x + 1.
+/// WRAPX: periodic in x; otherwise nothing beyond the faces.
+struct Word3 {
+    std::uint32_t mid, xm, xp;   // bit i: cell 32 w + i, the cell before it, the cell after it
+};
+template <bool WRAPX, class F>
+__device__ __forceinline__ Word3 word3(const F& at, const BitGrid& g, unsigned rowWord, int w) {
+    Word3 r;
+    r.mid = at(rowWord + w);
+    const int last = g.words - 1, valid = min(32, g.nx - 32 * w);
+    std::uint32_t before = 0, after = 0;
+    if (w > 0) before = at(rowWord + w - 1) >> 31;
+    else if (WRAPX) before = (at(rowWord + last) >> ((g.nx - 1) & 31)) & 1u;
+    if (w < last) after = at(rowWord + w + 1) & 1u;
+    else if (WRAPX) after = at(rowWord) & 1u;
+    r.xm = (r.mid << 1) | before;
+    r.xp = (r.mid >> 1) | (after << (valid - 1));
+    return r;
+}
+
+/// Cells of word w of row (y, z) with a set cell among their 18 neighbours.
+/// WRAPXY: periodic in x and y; otherwise nothing beyond those faces. z is
+/// periodic.
+template <bool WRAPXY, class F>
+__device__ __forceinline__ std::uint32_t near18(const F& at, const BitGrid& g, int w, int y, int z) {
+    std::uint32_t any = 0;
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz) {
+        const int Z = wrapi(z + dz, g.nz);
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy) {
+            int Y = y + dy;
+            if (WRAPXY) Y = wrapi(Y, g.ny);
+            else if (Y < 0 || Y >= g.ny) continue;
+            const unsigned rw = (static_cast<unsigned>(Z) * g.ny + Y) * g.words;
+            if (dy != 0 && dz != 0) {
+                any |= at(rw + w);
+            } else {
+                const Word3 r = word3<WRAPXY>(at, g, rw, w);
+                any |= r.xm | r.xp | (dy != 0 || dz != 0 ? r.mid : 0u);
+            }
+        }
+    }
+    return any;
+}
+
+struct OnePlane {
+    const std::uint32_t* p;
+    __device__ __forceinline__ std::uint32_t operator()(unsigned i) const { return __ldg(p + i); }
+};
+struct OrPlanes {
+    const std::uint32_t *p, *q;
+    __device__ __forceinline__ std::uint32_t operator()(unsigned i) const { return __ldg(p + i) | __ldg(q + i); }
+};
+struct AndNotPlanes {
+    const std::uint32_t *p, *q;
+    __device__ __forceinline__ std::uint32_t operator()(unsigned i) const { return __ldg(p + i) & ~__ldg(q + i); }
+};
+
+__device__ __forceinline__ void word_of(const BitGrid& g, unsigned wi, int& w, int& y, int& z) {
+    const unsigned row = wi / g.words;
+    w = static_cast<int>(wi - row * g.words);
+    z = static_cast<int>(row / g.ny);
+    y = static_cast<int>(row - static_cast<unsigned>(z) * g.ny);
+}
+
+// ---- classes and bounding box ------------------------------------------------------
+
+/// counts: cells read and written by a step, inlets, the others' complement is
+/// formed by the host; box: min/max of the solid cells' x and y.
+__global__ void __launch_bounds__(256)
+classes_kernel(Planes P, BitGrid g, unsigned long long* __restrict__ counts, int* __restrict__ box) {
+    unsigned long long rw = 0, in = 0;
+    int x0 = g.nx, x1 = -1, y0 = g.ny, y1 = -1;
+    for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < g.total(); i += gridDim.x * 256u) {
+        if (counts) {
+            rw += __popc(P.p[kPFluid][i]) + __popc(P.p[kPOutlet][i]);
+            in += __popc(P.p[kPInlet][i]);
+        }
+        const std::uint32_t s = P.p[kPSolid][i];
+        if (s) {
+            int w, y, z;
+            word_of(g, i, w, y, z);
+            x0 = min(x0, 32 * w + __ffs(static_cast<int>(s)) - 1);
+            x1 = max(x1, 32 * w + 31 - __clz(static_cast<int>(s)));
+            y0 = min(y0, y);
+            y1 = max(y1, y);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         rw += __shfl_xor_sync(0xffffffffu, rw, o);
         in += __shfl_xor_sync(0xffffffffu, in, o);
-        un += __shfl_xor_sync(0xffffffffu, un, o);
+        x0 = min(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+        x1 = max(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+        y0 = min(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+        y1 = max(y1, __shfl_xor_sync(0xffffffffu, y1, o));
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(counts + 0, rw); atomicAdd(counts + 1, in); atomicAdd(counts + 2, un);
+        if (counts && rw) atomicAdd(counts + 0, rw);
+        if (counts && in) atomicAdd(counts + 1, in);
+        if (x1 >= 0) {
+            atomicMin(box + 0, x0); atomicMax(box + 2, x1);
+            atomicMin(box + 1, y0); atomicMax(box + 3, y1);
+        }
     }
 }
 
-// ---- ordered compaction --------------------------------------------------------
+// ---- kind bytes, pull-link classes, tile codes -------------------------------------
 
-struct Grid3 {
-    int nx, ny, nz;
-};
-
-// Force links: fluid cells with a solid neighbour at x + c_q (x, y, z wrapped).
-struct ForceLinkPred {
-    Grid3 g;
-    const std::uint8_t* f;
-    std::uint32_t* cells;
-    std::uint32_t* masks;
-    __device__ std::uint32_t eval(long long c, int x, int y, int z, int* /*stats*/) const {
-        if (f[c] != kFluidB) return 0;
-        std::uint32_t m = 0;
+/// kind = flag | kNearWall for fluid cells with a solid or slip pull
+/// neighbour; links (when given): the classes of those cells' 18 pull links
+/// (kernels.h; the other cells' words are read by nothing and not written).
+/// One thread per word; the links of a word by its warp, one cell per lane.
+template <int ALIGN>
+__global__ void __launch_bounds__(256)
+classify_kernel(const std::uint8_t* __restrict__ flags, Planes P, BitGrid g, std::uint8_t* __restrict__ kind,
+                uint2* __restrict__ links) {
+    const unsigned wi = blockIdx.x * 256u + threadIdx.x, lane = threadIdx.x & 31;
+    std::uint32_t near = 0;
+    if (wi < g.total()) {
+        int w, y, z;
+        word_of(g, wi, w, y, z);
+        const std::uint32_t fluid = P.p[kPFluid][wi];
+        if (fluid) near = fluid & near18<true>(OrPlanes{P.p[kPSolid], P.p[kPSlip]}, g, w, y, z);
+        const size_t c0 = (static_cast<size_t>(z) * g.ny + y) * g.nx + 32u * w;
+        const int valid = min(32, g.nx - 32 * w);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const std::uint32_t add = ((((near >> (4 * k)) & 15u) * 0x00204081u) & 0x01010101u) << 7;
+            if (ALIGN >= 4 && 4 * k + 4 <= valid) {
+                reinterpret_cast<std::uint32_t*>(kind + c0)[k] =
+                    (reinterpret_cast<const std::uint32_t*>(flags + c0)[k] & 0x0f0f0f0fu) | add;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (4 * k + e < valid)
+                        kind[c0 + 4 * k + e] =
+                            static_cast<std::uint8_t>((flags[c0 + 4 * k + e] & kFlagMask) | (add >> (8 * e)));
+            }
+        }
+    }
+    if (!links) return;
+    for (unsigned todo = __ballot_sync(0xffffffffu, near != 0); todo; todo &= todo - 1) {
+        const int src = __ffs(static_cast<int>(todo)) - 1;
+        const std::uint32_t nw = __shfl_sync(0xffffffffu, near, src);
+        if (!(nw >> lane & 1u)) continue;
+        int w, y, z;
+        word_of(g, wi - lane + src, w, y, z);
+        const int x = 32 * w + static_cast<int>(lane);
+        unsigned long long m = 0;
 #pragma unroll
         for (int q = 1; q < kQ; ++q) {
-            const int X = wrapi(x + cx(q), g.nx), Y = wrapi(y + cy(q), g.ny), Z = wrapi(z + cz(q), g.nz);
-            const unsigned nb = static_cast<unsigned>(X)
-                              + static_cast<unsigned>(g.nx) * (static_cast<unsigned>(Y) + static_cast<unsigned>(g.ny) * Z);
-            if (f[nb] == kSolidB) m |= 1u << q;
+            const int X = wrapi(x - cx(q), g.nx), Y = wrapi(y - cy(q), g.ny), Z = wrapi(z - cz(q), g.nz);
+            const int nf = flags[(static_cast<size_t>(Z) * g.ny + Y) * g.nx + X] & kFlagMask;
+            if (nf == kSolid) m |= 1ull << (q - 1);
+            if (is_slip_y(nf)) m |= 1ull << (17 + q);
+            if (is_slip_z(nf)) m |= 1ull << (35 + q);
         }
-        return m;
+        links[(static_cast<size_t>(z) * g.ny + y) * g.nx + x] =
+            make_uint2(static_cast<unsigned>(m), static_cast<unsigned>(m >> 32));
     }
-    __device__ void emit(long long slot, long long c, int, int, int, std::uint32_t m) const {
-        cells[slot] = static_cast<std::uint32_t>(c);
-        masks[slot] = m;
-    }
-};
+}
 
-struct FlagEqPred {     // flag == value (interface-shell list)
-    const std::uint8_t* f;
-    std::uint8_t value;
-    std::uint32_t* cells;
-    __device__ std::uint32_t eval(long long c, int, int, int, int*) const { return f[c] == value ? 1u : 0u; }
-    __device__ void emit(long long slot, long long c, int, int, int, std::uint32_t) const {
-        cells[slot] = static_cast<std::uint32_t>(c);
-    }
-};
-
-// Interface cells a step reads: the shell cells with a fluid or outlet cell
-// among their 18 neighbours (wrapped). The stream-collide reaches no
-// further than one cell, so the rest of a 2-cell shell is read by nothing.
-struct ShellPulledPred {
-    Grid3 g;
-    const std::uint8_t* f;
-    std::uint32_t* cells;
-    __device__ std::uint32_t eval(long long c, int x, int y, int z, int*) const {
-        if (f[c] != kInterfaceB) return 0;
-#pragma unroll
-        for (int q = 1; q < kQ; ++q) {
-            const int X = wrapi(x + cx(q), g.nx), Y = wrapi(y + cy(q), g.ny), Z = wrapi(z + cz(q), g.nz);
-            const std::uint8_t nf = f[static_cast<unsigned>(X)
-                                      + static_cast<unsigned>(g.nx) * (static_cast<unsigned>(Y)
-                                                                       + static_cast<unsigned>(g.ny) * Z)];
-            if (nf == kFluidB || nf == kOutletB || nf == kOutletEqB) return 1u;
+/// Tile codes (kernels.h), one thread per 32 cells of the flattened lattice;
+/// `kind` has 64 bytes after its last cell.
+__global__ void __launch_bounds__(256)
+tile_codes_kernel(const std::uint8_t* __restrict__ kind, std::uint8_t* __restrict__ codes, int nx, int ny, int nz,
+                  unsigned n, unsigned ncodes) {
+    const unsigned i = blockIdx.x * 256u + threadIdx.x, c0 = 32 * i;
+    if (i >= ncodes) return;
+    std::uint8_t code = kTileIdle;
+    if (c0 < n) {
+        const uint4 a = reinterpret_cast<const uint4*>(kind + c0)[0], b = reinterpret_cast<const uint4*>(kind + c0)[1];
+        const bool full = c0 + 32 <= n;
+        const unsigned row = c0 / nx, z = row / ny;
+        const int x = static_cast<int>(c0 - row * nx), y = static_cast<int>(row - z * ny);
+        if (full && (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) == 0) {
+            const bool inner = x > 0 && x + 31 < nx - 1 && y > 0 && y < ny - 1 && z > 0 && static_cast<int>(z) < nz - 1;
+            code = inner ? kTileBulk : kTileGeneral;
+            if (!inner) {   // the run may cross a row's end
+                bool all = true;
+                unsigned xx = x, yy = y, zz = z;
+                for (int k = 0; k < 32; ++k) {
+                    all = all && xx > 0 && static_cast<int>(xx) < nx - 1 && yy > 0 && static_cast<int>(yy) < ny - 1
+                          && zz > 0 && static_cast<int>(zz) < nz - 1;
+                    if (static_cast<int>(++xx) == nx) { xx = 0; if (static_cast<int>(++yy) == ny) { yy = 0; ++zz; } }
+                }
+                if (all) code = kTileBulk;
+            }
+        } else {
+            const std::uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            for (int k = 0; k < 32 && c0 + k < n; ++k) {
+                const int flag = static_cast<int>(v[k >> 2] >> (8 * (k & 3))) & kFlagMask;
+                if (flag == kFluid || flag == kInlet || flag == kOutlet || flag == kOutletEq) { code = kTileGeneral; break; }
+            }
         }
-        return 0u;
     }
-    __device__ void emit(long long slot, long long c, int, int, int, std::uint32_t) const {
-        cells[slot] = static_cast<std::uint32_t>(c);
-    }
-};
+    codes[i] = code;
+}
 
-// Wall-model cell list (wall_model.cpp:55-236), in two compactions so that
-// the 5^3 occupancy gradient runs one candidate per thread instead of on
-// the one lane of a warp that meets a wall cell:
-//  1. WallCandPred over the lattice: fluid cells with a pull link that is
-//     solid in the active field and none that is solid only there (a vane
-//     link: the cell is excluded and counted);
-//  2. WallListPred over the candidate list: the gradient normal (degenerate
-//     ones dropped and counted), the sample cell along it, the entry.
-// Both compactions keep order, so the entries are in ascending cell order,
-// as the host builder's.
-struct WallGeom {
-    Grid3 g;
-    const std::uint8_t* active;
-    const std::uint8_t* clean;
-    __device__ __forceinline__ unsigned at(int x, int y, int z) const {
-        return static_cast<unsigned>(x) + static_cast<unsigned>(g.nx) * (static_cast<unsigned>(y)
-                                                                         + static_cast<unsigned>(g.ny) * z);
-    }
-    // Solid with x/y out of range = not solid, z periodic.
-    __device__ __forceinline__ bool solid(const std::uint8_t* f, int x, int y, int z) const {
-        if (x < 0 || x >= g.nx || y < 0 || y >= g.ny) return false;
-        return f[at(x, y, wrapi(z, g.nz))] == kSolidB;
-    }
-    __device__ __forceinline__ void gradient(int x, int y, int z, float& gx, float& gy, float& gz) const {
-        gx = gy = gz = 0.0f;
-        for (int dz = -2; dz <= 2; ++dz)
-            for (int dy = -2; dy <= 2; ++dy)
-#pragma unroll
-                for (int dx = -2; dx <= 2; ++dx)
-                    if (solid(clean, x + dx, y + dy, z + dz)) {
-                        gx += static_cast<float>(dx);
-                        gy += static_cast<float>(dy);
-                        gz += static_cast<float>(dz);
+// ---- ordered lists ------------------------------------------------------------------
+
+constexpr int kSelTile = 256;   // words per tile
+
+enum SelectOp { kSelForce, kSelShell, kSelInter, kSelWall };
+
+/// Selection words of a list and the number of cells in each tile.
+/// kSelWall: `C` are the planes of the clean field, stats[1] counts the cells
+/// left out for a link that is solid in the active field only.
+template <int OP>
+__global__ void __launch_bounds__(kSelTile)
+select_kernel(Planes P, Planes C, BitGrid g, std::uint32_t* __restrict__ sel, int* __restrict__ tileCount,
+              int* __restrict__ stats) {
+    const unsigned wi = blockIdx.x * kSelTile + threadIdx.x;
+    std::uint32_t s = 0;
+    int vanes = 0;
+    if (wi < g.total()) {
+        int w, y, z;
+        word_of(g, wi, w, y, z);
+        if (OP == kSelInter) {
+            s = P.p[kPInter][wi];
+        } else {
+            s = P.p[OP == kSelShell ? kPInter : kPFluid][wi];
+            if (s) {
+                if (OP == kSelForce) s &= near18<true>(OnePlane{P.p[kPSolid]}, g, w, y, z);
+                if (OP == kSelShell) s &= near18<true>(OrPlanes{P.p[kPFluid], P.p[kPOutlet]}, g, w, y, z);
+                if (OP == kSelWall) {
+                    s &= near18<false>(OnePlane{P.p[kPSolid]}, g, w, y, z);
+                    if (s && C.p[kPSolid] != P.p[kPSolid]) {
+                        const std::uint32_t v = s & near18<false>(AndNotPlanes{P.p[kPSolid], C.p[kPSolid]}, g, w, y, z);
+                        vanes = __popc(v);
+                        s &= ~v;
                     }
-    }
-};
-
-struct WallCandPred {
-    WallGeom w;
-    std::uint32_t *cells, *masks;
-    // 0 = not a candidate; otherwise the link mask. stats (count pass only):
-    // [1] vane-excluded.
-    __device__ std::uint32_t eval(long long c, int x, int y, int z, int* stats) const {
-        if (w.active[c] != kFluidB) return 0;
-        std::uint32_t m = 0;
-        bool vgOnly = false;
-#pragma unroll
-        for (int q = 1; q < kQ; ++q) {
-            const int sx = x - cx(q), sy = y - cy(q), sz = z - cz(q);
-            if (!w.solid(w.active, sx, sy, sz)) continue;
-            m |= 1u << q;
-            if (!w.solid(w.clean, sx, sy, sz)) vgOnly = true;
+                }
+            }
         }
-        if (m == 0) return 0;
-        if (vgOnly) {
-            if (stats) atomicAdd(stats + 1, 1);
-            return 0;
-        }
-        return m;
+        sel[wi] = s;
     }
-    __device__ void emit(long long slot, long long c, int, int, int, std::uint32_t m) const {
-        cells[slot] = static_cast<std::uint32_t>(c);
-        masks[slot] = m;
-    }
-};
-
-struct WallListPred {
-    WallGeom w;
-    int sampleCells;
-    const std::uint32_t *candCell, *candMask;
-    std::uint32_t *cell, *sample, *mask;
-    float *nX, *nY, *nZ, *ys;
-
-    __device__ __forceinline__ void decode(std::uint32_t c, int& x, int& y, int& z) const {
-        const unsigned nxy = static_cast<unsigned>(w.g.nx) * static_cast<unsigned>(w.g.ny);
-        z = static_cast<int>(c / nxy);
-        const unsigned r = c - static_cast<unsigned>(z) * nxy;
-        y = static_cast<int>(r / static_cast<unsigned>(w.g.nx));
-        x = static_cast<int>(r - static_cast<unsigned>(y) * static_cast<unsigned>(w.g.nx));
-    }
-    // i = candidate index. 0 = dropped; otherwise the link mask. stats
-    // (count pass only): [0] listed, [2] degenerate normal.
-    __device__ std::uint32_t eval(long long i, int, int, int, int* stats) const {
-        int x, y, z;
-        decode(candCell[i], x, y, z);
-        float gx, gy, gz;
-        w.gradient(x, y, z, gx, gy, gz);
-        const float gm = sqrtf(gx * gx + gy * gy + gz * gz);
-        if (gm < 1e-3f) {
-            if (stats) atomicAdd(stats + 2, 1);
-            return 0;
-        }
-        if (stats) atomicAdd(stats + 0, 1);
-        return candMask[i];
-    }
-    __device__ void emit(long long slot, long long i, int, int, int, std::uint32_t m) const {
-        const std::uint32_t c = candCell[i];
-        int x, y, z;
-        decode(c, x, y, z);
-        float gx, gy, gz;
-        w.gradient(x, y, z, gx, gy, gz);
-        const float gm = sqrtf(gx * gx + gy * gy + gz * gz);
-        const float nx_ = -gx / gm, ny_ = -gy / gm, nz_ = -gz / gm;
-        std::uint32_t s = c;
-        int sx = x, sy = y, sz = z;
-        for (int k = sampleCells; k >= 1; --k) {
-            const int tx = x + static_cast<int>(lroundf(nx_ * static_cast<float>(k)));
-            const int ty = y + static_cast<int>(lroundf(ny_ * static_cast<float>(k)));
-            const int tz = wrapi(z + static_cast<int>(lroundf(nz_ * static_cast<float>(k))), w.g.nz);
-            if (tx < 0 || tx >= w.g.nx || ty < 0 || ty >= w.g.ny) continue;
-            const std::uint32_t cand = w.at(tx, ty, tz);
-            if (w.active[cand] != kFluidB) continue;
-            s = cand; sx = tx; sy = ty; sz = tz;
-            break;
-        }
-        int dzw = sz - z;
-        if (dzw > w.g.nz / 2) dzw -= w.g.nz;
-        if (dzw < -w.g.nz / 2) dzw += w.g.nz;
-        const float proj = static_cast<float>(sx - x) * nx_ + static_cast<float>(sy - y) * ny_
-                         + static_cast<float>(dzw) * nz_;
-        cell[slot] = c;
-        sample[slot] = s;
-        nX[slot] = nx_; nY[slot] = ny_; nZ[slot] = nz_;
-        ys[slot] = 0.5f + fmaxf(proj, 0.0f);
-        mask[slot] = m;
-    }
-};
-
-template <class P>
-__device__ __forceinline__ std::uint32_t tile_eval(const P& p, const Grid3& g, long long n, int* stats,
-                                                   std::uint32_t (&vals)[kTileRun], int& cnt) {
-    const long long first = static_cast<long long>(blockIdx.x) * kTileCells + static_cast<long long>(threadIdx.x) * kTileRun;
-    cnt = 0;
-    std::uint32_t sel = 0;
-    if (first >= n) return 0;
-    int x = static_cast<int>(first % g.nx);
-    const long long r = first / g.nx;
-    int y = static_cast<int>(r % g.ny);
-    int z = static_cast<int>(r / g.ny);
-#pragma unroll 1
-    for (int k = 0; k < kTileRun; ++k) {
-        const long long c = first + k;
-        if (c >= n) break;
-        const std::uint32_t v = p.eval(c, x, y, z, stats);
-        vals[k] = v;
-        if (v) { sel |= 1u << k; ++cnt; }
-        if (++x == g.nx) { x = 0; if (++y == g.ny) { y = 0; ++z; } }
-    }
-    return sel;
-}
-
-template <class P>
-__global__ void __launch_bounds__(kTileThreads) compact_count_kernel(P p, Grid3 g, long long n, int* tileCount,
-                                                                     int* stats) {
-    std::uint32_t vals[kTileRun];
-    int cnt;
-    tile_eval(p, g, n, stats, vals, cnt);
-    __shared__ int warpSum[kTileThreads / 32];
-    int v = cnt;
+    __shared__ int warpSum[kSelTile / 32];
+    int v = __popc(s);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) warpSum[threadIdx.x >> 5] = v;
+    if (OP == kSelWall && vanes) atomicAdd(stats + 1, vanes);
     __syncthreads();
     if (threadIdx.x == 0) {
         int t = 0;
-        for (int w = 0; w < kTileThreads / 32; ++w) t += warpSum[w];
+        for (int k = 0; k < kSelTile / 32; ++k) t += warpSum[k];
         tileCount[blockIdx.x] = t;
     }
 }
@@ -497,15 +540,10 @@ __global__ void __launch_bounds__(1024) tile_scan_kernel(int* counts, int tiles,
     if (threadIdx.x == 0) *total = carry;
 }
 
-template <class P>
-__global__ void __launch_bounds__(kTileThreads) compact_scatter_kernel(P p, Grid3 g, long long n,
-                                                                       const int* tileOffset, long long cap,
-                                                                       int* overflow) {
-    std::uint32_t vals[kTileRun];
-    int cnt;
-    const std::uint32_t sel = tile_eval(p, g, n, nullptr, vals, cnt);
-    // Exclusive scan of the thread counts across the block.
-    __shared__ int warpSum[kTileThreads / 32];
+/// First list slot of this thread's selected cells: the tile's plus an
+/// exclusive scan over the block of `cnt`.
+__device__ __forceinline__ long long first_slot(int cnt, const int* __restrict__ tileOffset) {
+    __shared__ int warpSum[kSelTile / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int inc = cnt;
 #pragma unroll
@@ -515,103 +553,244 @@ __global__ void __launch_bounds__(kTileThreads) compact_scatter_kernel(P p, Grid
     }
     if (lane == 31) warpSum[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-        const int w = lane < kTileThreads / 32 ? warpSum[lane] : 0;
-        int wi = w;
+    int before = 0;
+    for (int k = 0; k < warp; ++k) before += warpSum[k];
+    return static_cast<long long>(tileOffset[blockIdx.x]) + before + inc - cnt;
+}
+
+/// Selected cells into the list, ascending.
+__global__ void __launch_bounds__(kSelTile)
+scatter_kernel(const std::uint32_t* __restrict__ sel, BitGrid g, const int* __restrict__ tileOffset,
+               std::uint32_t* __restrict__ cells) {
+    const unsigned wi = blockIdx.x * kSelTile + threadIdx.x;
+    std::uint32_t s = wi < g.total() ? sel[wi] : 0;
+    long long slot = first_slot(__popc(s), tileOffset);
+    if (!s) return;
+    const unsigned row = wi / g.words, c0 = row * static_cast<unsigned>(g.nx) + 32u * (wi - row * g.words);
+    for (; s; s &= s - 1) cells[slot++] = c0 + static_cast<unsigned>(__ffs(static_cast<int>(s)) - 1);
+}
+
+/// Cell coordinates from its index.
+__device__ __forceinline__ void coords(const BitGrid& g, std::uint32_t c, int& x, int& y, int& z) {
+    const unsigned row = c / static_cast<unsigned>(g.nx);
+    x = static_cast<int>(c - row * static_cast<unsigned>(g.nx));
+    z = static_cast<int>(row / static_cast<unsigned>(g.ny));
+    y = static_cast<int>(row - static_cast<unsigned>(z) * static_cast<unsigned>(g.ny));
+}
+
+/// Solid links of the listed cells, bit q: FORCE the neighbours at + c_q,
+/// everything periodic; otherwise the pull neighbours at - c_q, nothing
+/// beyond the x and y faces.
+template <bool FORCE>
+__global__ void __launch_bounds__(128)
+link_mask_kernel(const std::uint8_t* __restrict__ flags, BitGrid g, const std::uint32_t* __restrict__ cells, unsigned n,
+                 std::uint32_t* __restrict__ masks) {
+    const unsigned i = blockIdx.x * 128u + threadIdx.x;
+    if (i >= n) return;
+    int x, y, z;
+    coords(g, cells[i], x, y, z);
+    std::uint32_t m = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += t;
+    for (int q = 1; q < kQ; ++q) {
+        int X = x + (FORCE ? cx(q) : -cx(q)), Y = y + (FORCE ? cy(q) : -cy(q));
+        const int Z = wrapi(z + (FORCE ? cz(q) : -cz(q)), g.nz);
+        if (FORCE) {
+            X = wrapi(X, g.nx);
+            Y = wrapi(Y, g.ny);
+        } else if (X < 0 || X >= g.nx || Y < 0 || Y >= g.ny) {
+            continue;
         }
-        if (lane < kTileThreads / 32) warpSum[lane] = wi - w;
+        if (flags[(static_cast<size_t>(Z) * g.ny + Y) * g.nx + X] == kSolidB) m |= 1u << q;
     }
-    __syncthreads();
-    long long slot = static_cast<long long>(tileOffset[blockIdx.x]) + warpSum[warp] + inc - cnt;
-    if (!sel) return;
-    const long long first = static_cast<long long>(blockIdx.x) * kTileCells + static_cast<long long>(threadIdx.x) * kTileRun;
-    int x = static_cast<int>(first % g.nx);
-    const long long r = first / g.nx;
-    int y = static_cast<int>(r % g.ny);
-    int z = static_cast<int>(r / g.ny);
-#pragma unroll 1
-    for (int k = 0; k < kTileRun; ++k) {
-        if (sel >> k & 1u) {
-            if (slot < cap) p.emit(slot, first + k, x, y, z, vals[k]);
-            else atomicExch(overflow, 1);
-            ++slot;
+    masks[i] = m;
+}
+
+// ---- wall-model list --------------------------------------------------------------
+// Two lists: the candidates over the lattice (fluid cells with a pull link that
+// is solid and none that is solid in the active field only), then the ones
+// among them whose occupancy gradient gives a normal. Both keep the order, so
+// the entries ascend by cell, as the host builder's.
+
+/// Sum of (dx, dy, dz) over the solid cells of the 5^3 block around (x, y, z):
+/// nothing solid beyond the x and y faces, z periodic. Whole numbers, so the
+/// order of the sum does not matter.
+__device__ __forceinline__ void occupancy_gradient(const std::uint32_t* __restrict__ solid, const BitGrid& g, int x, int y,
+                                                   int z, int& gx, int& gy, int& gz) {
+    gx = gy = gz = 0;
+    const int w = x >> 5, b = x & 31, last = g.words - 1;
+    for (int dz = -2; dz <= 2; ++dz) {
+        const int Z = wrapi(z + dz, g.nz);
+        for (int dy = -2; dy <= 2; ++dy) {
+            const int Y = y + dy;
+            if (Y < 0 || Y >= g.ny) continue;
+            const std::uint32_t* r = solid + (static_cast<size_t>(Z) * g.ny + Y) * g.words;
+            // Bits x - 2 .. x + 2 (the row's words hold nothing beyond nx).
+            std::uint32_t v = b >= 2 ? __ldg(r + w) >> (b - 2) : __ldg(r + w) << (2 - b);
+            if (b < 2 && w > 0) v |= __ldg(r + w - 1) >> (30 + b);
+            if (b > 29 && w < last) v |= __ldg(r + w + 1) << (34 - b);
+            v &= 31u;
+            const int n = __popc(v);
+            gx += static_cast<int>((v >> 3) & 1u) + 2 * static_cast<int>((v >> 4) & 1u) - static_cast<int>((v >> 1) & 1u)
+                - 2 * static_cast<int>(v & 1u);
+            gy += dy * n;
+            gz += dz * n;
         }
-        if (++x == g.nx) { x = 0; if (++y == g.ny) { y = 0; ++z; } }
     }
 }
 
-/// Stream-ordered scratch of the compaction (tile counts, total, stats).
-struct CompactScratch {
-    int* tiles = nullptr;
-    long long* total = nullptr;
-    int* stats = nullptr;
-    int* overflow = nullptr;
-    void* block = nullptr;
-    cudaError_t alloc(long long nTiles, cudaStream_t st) {
-        const size_t bytes = static_cast<size_t>(nTiles) * 4 + 64;
-        if (auto e = cudaMallocAsync(&block, bytes, st); e != cudaSuccess) return e;
-        auto* b = static_cast<char*>(block);
-        total = reinterpret_cast<long long*>(b);
-        stats = reinterpret_cast<int*>(b + 8);
-        overflow = reinterpret_cast<int*>(b + 20);
-        tiles = reinterpret_cast<int*>(b + 64);
-        return cudaMemsetAsync(block, 0, 64, st);
+/// Candidates with a normal: their number per tile of 256, and in stats
+/// [0] listed, [2] without a normal.
+__global__ void __launch_bounds__(kSelTile)
+normal_count_kernel(const std::uint32_t* __restrict__ solid, BitGrid g, const std::uint32_t* __restrict__ cand, unsigned n,
+                    int* __restrict__ tileCount, int* __restrict__ stats) {
+    const unsigned i = blockIdx.x * kSelTile + threadIdx.x;
+    bool ok = false;
+    if (i < n) {
+        int x, y, z, gx, gy, gz;
+        coords(g, cand[i], x, y, z);
+        occupancy_gradient(solid, g, x, y, z, gx, gy, gz);
+        ok = gx != 0 || gy != 0 || gz != 0;   // the host's |gradient| >= 1e-3
     }
-    void release(cudaStream_t st) {
-        if (block) cudaFreeAsync(block, st);
-        block = nullptr;
+    const int c = __syncthreads_count(ok);
+    if (threadIdx.x == 0) {
+        const int here = static_cast<int>(min(static_cast<unsigned>(kSelTile), n - blockIdx.x * kSelTile));
+        tileCount[blockIdx.x] = c;
+        if (c) atomicAdd(stats + 0, c);
+        if (here - c) atomicAdd(stats + 2, here - c);
+    }
+}
+
+__global__ void __launch_bounds__(kSelTile)
+wall_entry_kernel(const std::uint32_t* __restrict__ solid, const std::uint8_t* __restrict__ active, BitGrid g,
+                  int sampleCells, const std::uint32_t* __restrict__ cand, const std::uint32_t* __restrict__ masks,
+                  unsigned n, const int* __restrict__ tileOffset, WallListOut o) {
+    const unsigned i = blockIdx.x * kSelTile + threadIdx.x;
+    int x = 0, y = 0, z = 0, ix = 0, iy = 0, iz = 0;
+    std::uint32_t c = 0;
+    if (i < n) {
+        c = cand[i];
+        coords(g, c, x, y, z);
+        occupancy_gradient(solid, g, x, y, z, ix, iy, iz);
+    }
+    const bool ok = ix != 0 || iy != 0 || iz != 0;
+    const long long slot = first_slot(ok ? 1 : 0, tileOffset);
+    if (!ok) return;
+    const float gx = static_cast<float>(ix), gy = static_cast<float>(iy), gz = static_cast<float>(iz);
+    const float gm = sqrtf(gx * gx + gy * gy + gz * gz);
+    const float nx_ = -gx / gm, ny_ = -gy / gm, nz_ = -gz / gm;
+    std::uint32_t s = c;
+    int sx = x, sy = y, sz = z;
+    for (int k = sampleCells; k >= 1; --k) {
+        const int tx = x + static_cast<int>(lroundf(nx_ * static_cast<float>(k)));
+        const int ty = y + static_cast<int>(lroundf(ny_ * static_cast<float>(k)));
+        const int tz = wrapi(z + static_cast<int>(lroundf(nz_ * static_cast<float>(k))), g.nz);
+        if (tx < 0 || tx >= g.nx || ty < 0 || ty >= g.ny) continue;
+        const std::uint32_t t = static_cast<std::uint32_t>(tx)
+                              + static_cast<std::uint32_t>(g.nx) * (static_cast<std::uint32_t>(ty)
+                                                                    + static_cast<std::uint32_t>(g.ny) * tz);
+        if (active[t] != kFluidB) continue;
+        s = t; sx = tx; sy = ty; sz = tz;
+        break;
+    }
+    int dzw = sz - z;
+    if (dzw > g.nz / 2) dzw -= g.nz;
+    if (dzw < -g.nz / 2) dzw += g.nz;
+    const float proj = static_cast<float>(sx - x) * nx_ + static_cast<float>(sy - y) * ny_
+                     + static_cast<float>(dzw) * nz_;
+    o.cell[slot] = c;
+    o.sample[slot] = s;
+    o.nX[slot] = nx_; o.nY[slot] = ny_; o.nZ[slot] = nz_;
+    o.ys[slot] = 0.5f + fmaxf(proj, 0.0f);
+    o.mask[slot] = masks[i];
+}
+
+// ---- host side of the tables ---------------------------------------------------------
+
+inline unsigned blocks_of(unsigned long long n, unsigned b) { return static_cast<unsigned>((n + b - 1) / b); }
+
+/// What the host reads back of a build: one copy.
+struct Readback {
+    unsigned long long counts[2];
+    long long total[2];    // of the force-link (or wall candidate) and the shell list
+    int stats[4];
+    int box[4];
+};
+
+/// A build's device memory, cut from one scratch block.
+struct Carver {
+    char* p;
+    size_t used = 0;
+    template <class T> T* take(size_t n) {
+        T* r = reinterpret_cast<T*>(p + used);
+        used += (n * sizeof(T) + 255) & ~size_t{255};
+        return r;
     }
 };
 
-long long tiles_for(long long n) { return (n + kTileCells - 1) / kTileCells; }
+struct TableScratch {
+    Readback* rb;
+    Planes planes{}, clean{};
+    std::uint32_t* sel[2] = {};
+    int* tiles[2] = {};
+    /// Lays the parts out at `base` (null: only counts the bytes).
+    size_t lay(char* base, const BitGrid& g, unsigned wanted, bool cleanSolid, int lists) {
+        Carver c{base};
+        rb = c.take<Readback>(1);
+        const size_t words = g.total();
+        for (int k = 0; k < kPlanes; ++k) planes.p[k] = (wanted >> k & 1u) ? c.take<std::uint32_t>(words) : nullptr;
+        clean = Planes{};
+        clean.p[kPSolid] = cleanSolid ? c.take<std::uint32_t>(words) : planes.p[kPSolid];
+        for (int k = 0; k < lists; ++k) {
+            sel[k] = c.take<std::uint32_t>(words);
+            tiles[k] = c.take<int>(words / kSelTile + 1);
+        }
+        return c.used;
+    }
+};
 
-/// Count pass + scan: *count <- number of selected cells (synchronises).
-template <class P>
-cudaError_t compact_count(const P& p, Grid3 g, CompactScratch& ws, long long* count, int statsOut[3],
-                          cudaStream_t st) {
-    const long long n = static_cast<long long>(g.nx) * g.ny * g.nz;
-    const long long tiles = tiles_for(n);
-    compact_count_kernel<P><<<static_cast<unsigned>(tiles), kTileThreads, 0, st>>>(p, g, n, ws.tiles, ws.stats);
-    tile_scan_kernel<<<1, 1024, 0, st>>>(ws.tiles, static_cast<int>(tiles), ws.total);
-    if (auto e = cudaGetLastError(); e != cudaSuccess) return e;
-    long long tot = 0;
-    int sts[3] = {0, 0, 0};
-    if (auto e = cudaMemcpyAsync(&tot, ws.total, sizeof(tot), cudaMemcpyDeviceToHost, st); e != cudaSuccess) return e;
-    if (auto e = cudaMemcpyAsync(sts, ws.stats, sizeof(sts), cudaMemcpyDeviceToHost, st); e != cudaSuccess) return e;
-    if (auto e = cudaStreamSynchronize(st); e != cudaSuccess) return e;
-    *count = tot;
-    if (statsOut) { statsOut[0] = sts[0]; statsOut[1] = sts[1]; statsOut[2] = sts[2]; }
-    return cudaSuccess;
-}
-
-template <class P>
-cudaError_t compact_scatter(const P& p, Grid3 g, CompactScratch& ws, long long cap, cudaStream_t st) {
-    const long long n = static_cast<long long>(g.nx) * g.ny * g.nz;
-    const long long tiles = tiles_for(n);
-    compact_scatter_kernel<P><<<static_cast<unsigned>(tiles), kTileThreads, 0, st>>>(p, g, n, ws.tiles, cap,
-                                                                                     ws.overflow);
+cudaError_t build_planes(const std::uint8_t* flags, const BitGrid& g, const Planes& P, cudaStream_t st,
+                         std::uint32_t keep = 0xffffffffu) {
+    const unsigned nb = blocks_of(g.total(), 256);
+    const auto a = reinterpret_cast<std::uintptr_t>(flags);
+    if (g.nx % 16 == 0 && a % 16 == 0) planes_kernel<16><<<nb, 256, 0, st>>>(flags, g, P, keep);
+    else if (g.nx % 4 == 0 && a % 4 == 0) planes_kernel<4><<<nb, 256, 0, st>>>(flags, g, P, keep);
+    else planes_kernel<1><<<nb, 256, 0, st>>>(flags, g, P, keep);
     return cudaGetLastError();
 }
 
-/// Both passes into caller buffers of capacity cap; *count <- selected cells.
-/// When *count > cap nothing is written (a caller sizes its buffers with a
-/// first call of capacity 0).
-template <class P>
-cudaError_t compact_into(const P& p, Grid3 g, long long cap, long long* count, int stats[3], cudaStream_t st) {
-    const long long n = static_cast<long long>(g.nx) * g.ny * g.nz;
-    if (n <= 0 || n >= (1LL << 31) || !count) return cudaErrorInvalidValue;
-    CompactScratch ws;
-    cudaError_t e = ws.alloc(tiles_for(n), st);
-    if (e == cudaSuccess) e = compact_count(p, g, ws, count, stats, st);
-    if (e == cudaSuccess && *count > 0 && *count <= cap) e = compact_scatter(p, g, ws, cap, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    ws.release(st);
-    return e;
+cudaError_t reset_readback(Readback* rb, const BitGrid& g, cudaStream_t st) {
+    Readback init{};
+    init.box[0] = g.nx; init.box[1] = g.ny; init.box[2] = init.box[3] = -1;
+    return cudaMemcpyAsync(rb, &init, sizeof init, cudaMemcpyHostToDevice, st);
 }
+
+template <int OP>
+void select_list(const TableScratch& ts, int list, const BitGrid& g, cudaStream_t st) {
+    const unsigned tiles = blocks_of(g.total(), kSelTile);
+    select_kernel<OP><<<tiles, kSelTile, 0, st>>>(ts.planes, ts.clean, g, ts.sel[list], ts.tiles[list], ts.rb->stats);
+    tile_scan_kernel<<<1, 1024, 0, st>>>(ts.tiles[list], static_cast<int>(tiles), &ts.rb->total[list]);
+}
+
+void scatter_list(const TableScratch& ts, int list, const BitGrid& g, std::uint32_t* cells, cudaStream_t st) {
+    scatter_kernel<<<blocks_of(g.total(), kSelTile), kSelTile, 0, st>>>(ts.sel[list], g, ts.tiles[list], cells);
+}
+
+cudaError_t read_back(const TableScratch& ts, Readback& h, cudaStream_t st) {
+    if (auto e = cudaGetLastError(); e != cudaSuccess) return e;
+    if (auto e = cudaMemcpyAsync(&h, ts.rb, sizeof h, cudaMemcpyDeviceToHost, st); e != cudaSuccess) return e;
+    return cudaStreamSynchronize(st);
+}
+
+/// Stream-ordered scratch of a call without a GeomScratch of its own.
+struct CallScratch {
+    void* p = nullptr;
+    cudaStream_t st;
+    explicit CallScratch(cudaStream_t s) : st(s) {}
+    ~CallScratch() { if (p) cudaFreeAsync(p, st); }
+    cudaError_t alloc(size_t bytes) { return cudaMallocAsync(&p, bytes, st); }
+};
+
+constexpr unsigned bit(Plane p) { return 1u << p; }
 
 } // namespace
 
@@ -676,99 +855,198 @@ cudaError_t device_build_flags(LevelDims d, int base, const std::uint8_t* in, co
     return e;
 }
 
-cudaError_t device_solid_bbox(LevelDims d, const std::uint8_t* flags, cudaStream_t st, int box[4]) {
-    const long long n = d.cells();
-    if (n <= 0 || !flags) return cudaErrorInvalidValue;
-    int* dbox = nullptr;
-    if (auto e = cudaMallocAsync(reinterpret_cast<void**>(&dbox), 16, st); e != cudaSuccess) return e;
-    const int init[4] = {d.nx, d.ny, -1, -1};
-    cudaError_t e = cudaMemcpyAsync(dbox, init, 16, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) {
-        const long long blocks = (n + 255) / 256;
-        solid_bbox_kernel<<<static_cast<unsigned>(blocks < 152 * 16 ? blocks : 152 * 16), 256, 0, st>>>(flags, d.nx,
-                                                                                                    d.ny, n, dbox);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(box, dbox, 16, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFreeAsync(dbox, st);
-    return e;
+cudaError_t GeomScratch::ensure(size_t bytes) {
+    if (bytes <= size) return cudaSuccess;
+    release();
+    if (auto e = cudaMalloc(&p, bytes); e != cudaSuccess) { p = nullptr; return e; }
+    size = bytes;
+    return cudaSuccess;
+}
+void GeomScratch::release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    size = 0;
 }
 
-cudaError_t device_flag_classes(LevelDims d, const std::uint8_t* flags, cudaStream_t st, long long out[3]) {
+cudaError_t device_solid_bbox(LevelDims d, const std::uint8_t* flags, cudaStream_t st, int box[4]) {
+    if (d.cells() <= 0 || d.cells() >= (1LL << 31) || !flags) return cudaErrorInvalidValue;
+    const BitGrid g = bit_grid(d);
+    TableScratch ts;
+    CallScratch cs(st);
+    if (auto e = cs.alloc(ts.lay(nullptr, g, bit(kPSolid), false, 0)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(cs.p), g, bit(kPSolid), false, 0);
+    if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
+    if (auto e = build_planes(flags, g, ts.planes, st); e != cudaSuccess) return e;
+    classes_kernel<<<min(blocks_of(g.total(), 256), 152u * 8u), 256, 0, st>>>(ts.planes, g, nullptr, ts.rb->box);
+    Readback h;
+    if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
+    for (int k = 0; k < 4; ++k) box[k] = h.box[k];
+    return cudaSuccess;
+}
+
+cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTables& t, GeomScratch& scratch,
+                               cudaStream_t st) {
     const long long n = d.cells();
-    if (n <= 0 || !flags) return cudaErrorInvalidValue;
-    unsigned long long* dc = nullptr;
-    if (auto e = cudaMallocAsync(reinterpret_cast<void**>(&dc), 24, st); e != cudaSuccess) return e;
-    cudaError_t e = cudaMemsetAsync(dc, 0, 24, st);
-    if (e == cudaSuccess) {
-        const long long blocks = (n + 255) / 256;
-        flag_classes_kernel<<<static_cast<unsigned>(blocks < 152 * 16 ? blocks : 152 * 16), 256, 0, st>>>(flags, n,
-                                                                                                      dc);
-        e = cudaGetLastError();
+    if (n <= 0 || n >= (1LL << 31) || !flags || !t.kind) return cudaErrorInvalidValue;
+    const BitGrid g = bit_grid(d);
+    const unsigned wanted = bit(kPSolid) | bit(kPFluid) | bit(kPSlip) | bit(kPInlet) | bit(kPOutlet);
+    TableScratch ts;
+    if (auto e = scratch.ensure(ts.lay(nullptr, g, wanted, false, 1)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(scratch.p), g, wanted, false, 1);
+    if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
+    if (auto e = build_planes(flags, g, ts.planes, st, 0x0f0f0f0fu); e != cudaSuccess) return e;
+    classes_kernel<<<min(blocks_of(g.total(), 256), 152u * 8u), 256, 0, st>>>(ts.planes, g, ts.rb->counts, ts.rb->box);
+    const unsigned nb = blocks_of(g.total(), 256);
+    const auto a = reinterpret_cast<std::uintptr_t>(flags) | reinterpret_cast<std::uintptr_t>(t.kind);
+    if (d.nx % 4 == 0 && a % 4 == 0) classify_kernel<4><<<nb, 256, 0, st>>>(flags, ts.planes, g, t.kind, t.links);
+    else classify_kernel<1><<<nb, 256, 0, st>>>(flags, ts.planes, g, t.kind, t.links);
+    if (t.tiles) {
+        const unsigned nc = static_cast<unsigned>(tile_code_bytes(n));
+        tile_codes_kernel<<<blocks_of(nc, 256), 256, 0, st>>>(t.kind, reinterpret_cast<std::uint8_t*>(t.tiles), d.nx,
+                                                             d.ny, d.nz, static_cast<unsigned>(n), nc);
     }
-    unsigned long long h[3] = {0, 0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, dc, 24, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFreeAsync(dc, st);
-    for (int i = 0; i < 3; ++i) out[i] = static_cast<long long>(h[i]);
-    return e;
+    select_list<kSelForce>(ts, 0, g, st);
+    Readback h;
+    if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
+    t.classes[0] = static_cast<long long>(h.counts[0]);
+    t.classes[1] = static_cast<long long>(h.counts[1]);
+    t.classes[2] = n - t.classes[0] - t.classes[1];
+    for (int k = 0; k < 4; ++k) t.box[k] = h.box[k];
+    t.linkCount = h.total[0];
+    t.linkCells = t.linkMasks = nullptr;
+    const size_t bytes = static_cast<size_t>(t.linkCount > 0 ? t.linkCount : 1) * 4;
+    if (auto e = cudaMalloc(&t.linkCells, bytes); e != cudaSuccess) return e;
+    if (auto e = cudaMalloc(&t.linkMasks, bytes); e != cudaSuccess) {
+        cudaFree(t.linkCells);
+        t.linkCells = nullptr;
+        return e;
+    }
+    if (t.linkCount > 0) {
+        const unsigned m = static_cast<unsigned>(t.linkCount);
+        scatter_list(ts, 0, g, t.linkCells, st);
+        link_mask_kernel<true><<<blocks_of(m, 128), 128, 0, st>>>(flags, g, t.linkCells, m, t.linkMasks);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, std::uint32_t** cells, long long* count,
+                             GeomScratch& scratch, cudaStream_t st) {
+    if (d.cells() <= 0 || d.cells() >= (1LL << 31) || !flags || !cells || !count) return cudaErrorInvalidValue;
+    *cells = nullptr;
+    *count = 0;
+    const BitGrid g = bit_grid(d);
+    const unsigned wanted = full ? bit(kPInter) : bit(kPInter) | bit(kPFluid) | bit(kPOutlet);
+    TableScratch ts;
+    if (auto e = scratch.ensure(ts.lay(nullptr, g, wanted, false, 1)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(scratch.p), g, wanted, false, 1);
+    if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
+    if (auto e = build_planes(flags, g, ts.planes, st); e != cudaSuccess) return e;
+    if (full) select_list<kSelInter>(ts, 0, g, st);
+    else select_list<kSelShell>(ts, 0, g, st);
+    Readback h;
+    if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
+    if (auto e = cudaMalloc(cells, static_cast<size_t>(h.total[0] > 0 ? h.total[0] : 1) * 4); e != cudaSuccess) return e;
+    *count = h.total[0];
+    if (h.total[0] > 0) scatter_list(ts, 0, g, *cells, st);
+    return cudaGetLastError();
 }
 
 cudaError_t device_force_links(LevelDims d, const std::uint8_t* flags, std::uint32_t* cells, std::uint32_t* masks,
                                long long cap, long long* count, cudaStream_t st) {
-    ForceLinkPred p{{d.nx, d.ny, d.nz}, flags, cells, masks};
-    return compact_into(p, {d.nx, d.ny, d.nz}, cap, count, nullptr, st);
+    if (d.cells() <= 0 || d.cells() >= (1LL << 31) || !flags || !count) return cudaErrorInvalidValue;
+    const BitGrid g = bit_grid(d);
+    const unsigned wanted = bit(kPSolid) | bit(kPFluid);
+    TableScratch ts;
+    CallScratch cs(st);
+    if (auto e = cs.alloc(ts.lay(nullptr, g, wanted, false, 1)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(cs.p), g, wanted, false, 1);
+    if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
+    if (auto e = build_planes(flags, g, ts.planes, st); e != cudaSuccess) return e;
+    select_list<kSelForce>(ts, 0, g, st);
+    Readback h;
+    if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
+    *count = h.total[0];
+    if (*count <= 0 || *count > cap) return cudaSuccess;
+    const unsigned m = static_cast<unsigned>(*count);
+    scatter_list(ts, 0, g, cells, st);
+    link_mask_kernel<true><<<blocks_of(m, 128), 128, 0, st>>>(flags, g, cells, m, masks);
+    if (auto e = cudaGetLastError(); e != cudaSuccess) return e;
+    return cudaStreamSynchronize(st);
 }
 
-cudaError_t device_cells_where(LevelDims d, const std::uint8_t* flags, std::uint8_t value, std::uint32_t* cells,
-                               long long cap, long long* count, cudaStream_t st) {
-    return compact_into(FlagEqPred{flags, value, cells}, {d.nx, d.ny, d.nz}, cap, count, nullptr, st);
+// The wall list in two parts, so that its owner can allocate the entries once
+// their number is known.
+cudaError_t WallListBuild::find(LevelDims dims, const std::uint8_t* activeF, const std::uint8_t* clean, long long* count,
+                                int stats[3], cudaStream_t st) {
+    if (dims.cells() <= 0 || dims.cells() >= (1LL << 31) || !activeF || !count) return cudaErrorInvalidValue;
+    d = dims;
+    active = activeF;
+    *count = n = candidates = 0;
+    if (stats) stats[0] = stats[1] = stats[2] = 0;
+    const BitGrid g = bit_grid(d);
+    const bool own = clean && clean != activeF;
+    const unsigned wanted = bit(kPSolid) | bit(kPFluid);
+    TableScratch ts;
+    if (auto e = cudaMallocAsync(&block, ts.lay(nullptr, g, wanted, own, 1), st); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(block), g, wanted, own, 1);
+    if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
+    if (auto e = build_planes(activeF, g, ts.planes, st); e != cudaSuccess) return e;
+    if (own)
+        if (auto e = build_planes(clean, g, ts.clean, st); e != cudaSuccess) return e;
+    select_list<kSelWall>(ts, 0, g, st);
+    Readback h;
+    if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
+    if (stats) stats[1] = h.stats[1];
+    candidates = h.total[0];
+    if (candidates == 0) return cudaSuccess;
+    // Candidates, their link masks and the tiles of the second list.
+    const unsigned nc = static_cast<unsigned>(candidates), tiles = blocks_of(nc, kSelTile);
+    Carver c{nullptr};
+    for (int pass = 0; pass < 2; ++pass) {
+        c.used = 0;
+        cand = c.take<std::uint32_t>(nc);
+        masks = c.take<std::uint32_t>(nc);
+        offsets = c.take<int>(tiles);
+        if (pass == 0) {
+            if (auto e = cudaMallocAsync(&block2, c.used, st); e != cudaSuccess) return e;
+            c.p = static_cast<char*>(block2);
+        }
+    }
+    solid = ts.clean.p[kPSolid];
+    scatter_list(ts, 0, g, cand, st);
+    link_mask_kernel<false><<<blocks_of(nc, 128), 128, 0, st>>>(activeF, g, cand, nc, masks);
+    normal_count_kernel<<<tiles, kSelTile, 0, st>>>(solid, g, cand, nc, offsets, ts.rb->stats);
+    tile_scan_kernel<<<1, 1024, 0, st>>>(offsets, static_cast<int>(tiles), &ts.rb->total[1]);
+    if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
+    *count = n = h.total[1];
+    if (stats) { stats[0] = h.stats[0]; stats[2] = h.stats[2]; }
+    return cudaSuccess;
 }
 
-cudaError_t device_shell_pulled(LevelDims d, const std::uint8_t* flags, std::uint32_t* cells, long long cap,
-                                long long* count, cudaStream_t st) {
-    return compact_into(ShellPulledPred{{d.nx, d.ny, d.nz}, flags, cells}, {d.nx, d.ny, d.nz}, cap, count, nullptr,
-                        st);
+cudaError_t WallListBuild::emit(int sampleCells, const WallListOut& out, cudaStream_t st) const {
+    if (n <= 0) return cudaSuccess;
+    const unsigned nc = static_cast<unsigned>(candidates);
+    wall_entry_kernel<<<blocks_of(nc, kSelTile), kSelTile, 0, st>>>(solid, active, bit_grid(d), sampleCells, cand, masks,
+                                                                   nc, offsets, out);
+    return cudaGetLastError();
+}
+
+void WallListBuild::release(cudaStream_t st) {
+    if (block) cudaFreeAsync(block, st);
+    if (block2) cudaFreeAsync(block2, st);
+    block = block2 = nullptr;
 }
 
 cudaError_t device_wall_list(LevelDims d, const std::uint8_t* active, const std::uint8_t* clean, int sampleCells,
                              const WallListOut& out, long long cap, long long* count, int stats[3],
                              cudaStream_t st) {
-    const Grid3 g{d.nx, d.ny, d.nz};
-    const long long n = d.cells();
-    if (n <= 0 || n >= (1LL << 31) || !count || !active) return cudaErrorInvalidValue;
-    const WallGeom w{g, active, clean ? clean : active};
-    // 1. Candidates, in cell order.
-    WallCandPred p1{w, nullptr, nullptr};
-    CompactScratch ws;
-    long long nc = 0;
-    int s1[3] = {0, 0, 0};
-    cudaError_t e = ws.alloc(tiles_for(n), st);
-    if (e == cudaSuccess) e = compact_count(p1, g, ws, &nc, s1, st);
-    void* cand = nullptr;
-    if (e == cudaSuccess && nc > 0) e = cudaMallocAsync(&cand, static_cast<size_t>(nc) * 8, st);
-    if (e == cudaSuccess && nc > 0) {
-        p1.cells = static_cast<std::uint32_t*>(cand);
-        p1.masks = p1.cells + nc;
-        e = compact_scatter(p1, g, ws, nc, st);
+    WallListBuild b;
+    cudaError_t e = b.find(d, active, clean, count, stats, st);
+    if (e == cudaSuccess && *count > 0 && *count <= cap) {
+        e = b.emit(sampleCells, out, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
-    ws.release(st);
-    // 2. The listed entries among them.
-    int s2[3] = {0, 0, 0};
-    if (e == cudaSuccess) {
-        if (nc > 0) {
-            const std::uint32_t* cc = static_cast<const std::uint32_t*>(cand);
-            WallListPred p2{w, sampleCells, cc, cc + nc, out.cell, out.sample, out.mask, out.nX, out.nY, out.nZ,
-                            out.ys};
-            e = compact_into(p2, {static_cast<int>(nc), 1, 1}, cap, count, s2, st);
-        } else {
-            *count = 0;
-        }
-    }
-    if (cand) cudaFreeAsync(cand, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (stats) { stats[0] = s2[0]; stats[1] = s1[1]; stats[2] = s2[2]; }
+    b.release(st);
     return e;
 }
 

@@ -39,10 +39,10 @@ struct CollideParams {
     /// cut bytes [cell * 19 + q] (q = byte / 255) and two-node bits [cell].
     const std::uint8_t* qFrac = nullptr;
     const std::uint32_t* ffMask = nullptr;
-    /// Link classes of each fluid cell's pull neighbours (launch_classify),
+    /// Link classes of each fluid cell's pull neighbours (build_level_tables),
     /// or null: the near-wall gather then reads the neighbours' flags.
     const uint2* links = nullptr;
-    /// Tile codes of the level (launch_tile_codes), or null: every cell then
+    /// Tile codes of the level (build_level_tables), or null: every cell then
     /// goes by its kind byte.
     const std::uint32_t* tiles = nullptr;
 };
@@ -58,12 +58,9 @@ struct SlipField {
 enum class Storage : int { F32 = 0, F16 = 1 };
 
 // ---- step kernels (step_kernels.cu) ---------------------------------------
-/// Kind bytes, and (links not null) per fluid cell the classes of its 18
-/// pull links x - c_q as one 64-bit word (low half in .x): bit q - 1 solid,
-/// bit 17 + q free-slip y wall, bit 35 + q free-slip z wall; 0 for cells
-/// that are not fluid.
-cudaError_t launch_classify(const std::uint8_t* flags, std::uint8_t* kind,
-                            LevelDims d, cudaStream_t st, uint2* links = nullptr);
+// The level's tables (build_level_tables): kind bytes, and per near-wall fluid
+// cell the classes of its 18 pull links x - c_q as one 64-bit word (low half in
+// .x): bit q - 1 solid, bit 17 + q free-slip y wall, bit 35 + q free-slip z wall.
 /// What a step finds in the 32 consecutive cells of a warp.
 enum : std::uint8_t {
     kTileIdle = 0,     ///< no cell that a step writes
@@ -72,7 +69,6 @@ enum : std::uint8_t {
 };
 /// Tile codes: one word per 128 consecutive cells, byte w the code of its
 /// cells 32 w .. 32 w + 31 (cells past the end count as idle).
-cudaError_t launch_tile_codes(const std::uint8_t* kind, std::uint32_t* tiles, LevelDims d, cudaStream_t st);
 inline size_t tile_code_bytes(long long cells) { return static_cast<size_t>((cells + 127) / 128) * 4; }
 cudaError_t launch_collide(Storage s, const void* src, void* dst,
                            const std::uint8_t* kind, LevelDims d,
@@ -269,20 +265,57 @@ cudaError_t device_build_flags(LevelDims d, int base, const std::uint8_t* in, co
                                int shell, std::uint8_t* out, cudaStream_t st, int* closedOut);
 /// Solid bounding box {x0, y0, x1, y1} (inclusive; x1 < 0 when no solid).
 cudaError_t device_solid_bbox(LevelDims d, const std::uint8_t* flags, cudaStream_t st, int box[4]);
-/// Cells whose flag is read and written / inlet / neither.
-cudaError_t device_flag_classes(LevelDims d, const std::uint8_t* flags, cudaStream_t st, long long out[3]);
 /// True for a pointer into device memory (cudaPointerGetAttributes).
 bool is_device_pointer(const void* p);
-/// Ordered cell lists. *count <- the list length; nothing is written when it
-/// exceeds cap (size with a first call of capacity 0). All synchronise.
+/// Scratch of the table builders, kept by its owner between calls (grows,
+/// given back by release). One stream at a time.
+struct GeomScratch {
+    void* p = nullptr;
+    size_t size = 0;
+    cudaError_t ensure(size_t bytes);
+    void release();
+};
+/// What a level derives from its flags. kind (with 64 bytes after the last
+/// cell), links and tiles are the owner's arrays, the last two may be null;
+/// the link list is allocated here (cudaMalloc), ascending, bit q of a mask set
+/// when the neighbour at +c_q is solid.
+struct LevelTables {
+    std::uint8_t* kind = nullptr;
+    uint2* links = nullptr;
+    std::uint32_t* tiles = nullptr;
+    long long classes[3] = {0, 0, 0};   ///< cells read and written by a step / inlet / neither
+    int box[4] = {0, 0, -1, -1};        ///< solid bounding box, as device_solid_bbox
+    std::uint32_t *linkCells = nullptr, *linkMasks = nullptr;
+    long long linkCount = 0;
+};
+/// Synchronises once (the list's length); the tables are ready in stream order.
+cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTables& t, GeomScratch& scratch,
+                               cudaStream_t st);
+/// Interface cells of a refined level, ascending: those with a fluid or outlet
+/// cell among their 18 neighbours (the ones a stream-collide reads), or with
+/// `full` every one. Allocated here; synchronises once.
+cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, std::uint32_t** cells, long long* count,
+                             GeomScratch& scratch, cudaStream_t st);
+/// The wall-model list: find counts the entries (and synchronises), emit writes
+/// them, release gives the working memory back (stream-ordered).
+struct WallListBuild {
+    LevelDims d;
+    const std::uint8_t* active = nullptr;
+    long long n = 0, candidates = 0;
+    void *block = nullptr, *block2 = nullptr;
+    std::uint32_t *cand = nullptr, *masks = nullptr;
+    const std::uint32_t* solid = nullptr;
+    int* offsets = nullptr;
+    cudaError_t find(LevelDims dims, const std::uint8_t* activeF, const std::uint8_t* clean, long long* count,
+                     int stats[3], cudaStream_t st);
+    cudaError_t emit(int sampleCells, const WallListOut& out, cudaStream_t st) const;
+    void release(cudaStream_t st);
+};
+/// Lists into the caller's buffers. *count <- the list length; nothing is
+/// written when it exceeds cap (size with a first call of capacity 0). Both
+/// synchronise.
 cudaError_t device_force_links(LevelDims d, const std::uint8_t* flags, std::uint32_t* cells, std::uint32_t* masks,
                                long long cap, long long* count, cudaStream_t st);
-cudaError_t device_cells_where(LevelDims d, const std::uint8_t* flags, std::uint8_t value, std::uint32_t* cells,
-                               long long cap, long long* count, cudaStream_t st);
-/// Interface cells with a fluid or outlet cell among their 18 neighbours
-/// (the shell cells a stream-collide reads), ascending; as device_cells_where.
-cudaError_t device_shell_pulled(LevelDims d, const std::uint8_t* flags, std::uint32_t* cells, long long cap,
-                                long long* count, cudaStream_t st);
 cudaError_t device_wall_list(LevelDims d, const std::uint8_t* active, const std::uint8_t* clean, int sampleCells,
                              const WallListOut& out, long long cap, long long* count, int stats[3],
                              cudaStream_t st);

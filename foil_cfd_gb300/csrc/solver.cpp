@@ -121,6 +121,7 @@ struct Level {
     // only) and cells it leaves untouched (solid, slip, interface; the kind
     // byte is still read).
     long long nReadWrite = 0, nInlet = 0, nUntouched = 0;
+    int solidBox[4] = {0, 0, -1, -1};   // bounding box of the solid cells (x1 < 0: none)
 
     double collideBytes(Storage s) const {
         const double pop = s == Storage::F32 ? 4.0 : 2.0;
@@ -243,6 +244,8 @@ struct fcfd_solver {
     bool fineShellFull = false;
     float* dScratch = nullptr;
     bool forcesFromFine = false;
+
+    GeomScratch geomScratch;   // of the flag-field tables, kept between flag changes
 
     // ---- macroscopic fields + readbacks ----
     float *rho = nullptr, *u = nullptr, *v = nullptr, *w = nullptr;
@@ -379,31 +382,22 @@ struct fcfd_solver {
             if (auto e = cudaMemcpyAsync(L.flags, flags, nb, cudaMemcpyHostToDevice, stream); e != cudaSuccess)
                 return e;
         }
-        long long cls[3];
-        launches += 1;
-        if (auto e = device_flag_classes(L.d, L.flags, stream, cls); e != cudaSuccess) return e;
-        L.nReadWrite = cls[0]; L.nInlet = cls[1]; L.nUntouched = cls[2];
-        launches += 2;
-        if (auto e = launch_classify(L.flags, L.kind, L.d, stream, L.links); e != cudaSuccess) return e;
-        if (auto e = launch_tile_codes(L.kind, L.tiles, L.d, stream); e != cudaSuccess) return e;
-        // Compact force-link list of this level (ascending cell order).
         dfree(L.dLinkCells); dfree(L.dLinkMasks); dfree(L.dPartials);
-        long long links = 0;
-        launches += 2;
-        if (auto e = device_force_links(L.d, L.flags, nullptr, nullptr, 0, &links, stream); e != cudaSuccess) return e;
-        L.linkCount = static_cast<int>(links);
-        if (auto e = dalloc(&L.dLinkCells, static_cast<size_t>(links) * 4); e != cudaSuccess) return e;
-        if (auto e = dalloc(&L.dLinkMasks, static_cast<size_t>(links) * 4); e != cudaSuccess) return e;
+        LevelTables t;
+        t.kind = L.kind;
+        t.links = L.links;
+        t.tiles = L.tiles;
+        launches += 8;
+        const cudaError_t te = build_level_tables(L.d, L.flags, t, geomScratch, stream);
+        L.dLinkCells = t.linkCells;
+        L.dLinkMasks = t.linkMasks;
+        L.linkCount = static_cast<int>(t.linkCount);
+        if (te != cudaSuccess) return te;
+        L.nReadWrite = t.classes[0]; L.nInlet = t.classes[1]; L.nUntouched = t.classes[2];
+        for (int k = 0; k < 4; ++k) L.solidBox[k] = t.box[k];
         if (auto e = dalloc(&L.dPartials, static_cast<size_t>(force_blocks(L.linkCount)) * 3 * sizeof(double));
             e != cudaSuccess)
             return e;
-        if (links > 0) {
-            launches += 3;
-            long long again = 0;
-            if (auto e = device_force_links(L.d, L.flags, L.dLinkCells, L.dLinkMasks, links, &again, stream);
-                e != cudaSuccess)
-                return e;
-        }
         return cudaStreamSynchronize(stream);
     }
 
@@ -415,40 +409,13 @@ struct fcfd_solver {
     /// level while a finer level nests in it, whose fill may gather from
     /// the fine shell) every interface cell.
     cudaError_t shellList(const Level& L, bool full, std::uint32_t** out, int* count) {
-        if (full) return cellList(L, FCFD_FLAG_INTERFACE, out, count);
         dfree(*out);
         *count = 0;
         long long c = 0;
-        launches += 2;
-        if (auto e = device_shell_pulled(L.d, L.flags, nullptr, 0, &c, stream); e != cudaSuccess) return e;
-        if (auto e = dalloc(out, static_cast<size_t>(c) * 4); e != cudaSuccess) return e;
-        if (c > 0) {
-            launches += 3;
-            long long again = 0;
-            if (auto e = device_shell_pulled(L.d, L.flags, *out, c, &again, stream); e != cudaSuccess) return e;
-        }
+        launches += 4;
+        const cudaError_t e = build_shell_list(L.d, L.flags, full, out, &c, geomScratch, stream);
         *count = static_cast<int>(c);
-        return cudaSuccess;
-    }
-
-    /// Ascending list of the level's cells whose flag equals `value`, into a
-    /// fresh device array.
-    cudaError_t cellList(const Level& L, std::uint8_t value, std::uint32_t** out, int* count) {
-        dfree(*out);
-        *count = 0;
-        long long c = 0;
-        launches += 2;
-        if (auto e = device_cells_where(L.d, L.flags, value, nullptr, 0, &c, stream); e != cudaSuccess)
-            return e;
-        if (auto e = dalloc(out, static_cast<size_t>(c) * 4); e != cudaSuccess) return e;
-        if (c > 0) {
-            launches += 3;
-            long long again = 0;
-            if (auto e = device_cells_where(L.d, L.flags, value, *out, c, &again, stream); e != cudaSuccess)
-                return e;
-        }
-        *count = static_cast<int>(c);
-        return cudaSuccess;
+        return e;
     }
 
     cudaError_t buildWM(Level& L, int sampleCells) {
@@ -465,12 +432,12 @@ struct fcfd_solver {
         }
         long long n = 0;
         int st[3] = {0, 0, 0};
-        WallListOut none;
-        launches += 2;
-        if (e == cudaSuccess)
-            e = device_wall_list(L.d, L.flags, dClean ? dClean : L.flags, sampleCells, none, 0, &n, st, stream);
+        WallListBuild wb;
+        launches += 6;
+        if (e == cudaSuccess) e = wb.find(L.d, L.flags, dClean ? dClean : L.flags, &n, st, stream);
         L.wm.build.listed = st[0]; L.wm.build.excludedVG = st[1]; L.wm.build.degenerate = st[2];
         if (e != cudaSuccess || n == 0) {
+            wb.release(stream);
             dfree(dClean);
             return e;
         }
@@ -485,10 +452,10 @@ struct fcfd_solver {
             WallListOut o;
             o.cell = m.dCell; o.sample = m.dSample; o.mask = m.dMask;
             o.nX = m.dNx; o.nY = m.dNy; o.nZ = m.dNz; o.ys = m.dYs;
-            long long again = 0;
-            launches += 3;
-            e = device_wall_list(L.d, L.flags, dClean ? dClean : L.flags, sampleCells, o, n, &again, st, stream);
+            ++launches;
+            e = wb.emit(sampleCells, o, stream);
         }
+        wb.release(stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(m.dUTau, 0, nn * 4, stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(m.dUwx, 0, cells * 2, stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(m.dUwy, 0, cells * 2, stream);
@@ -560,9 +527,7 @@ struct fcfd_solver {
         if (!fineActive) return;
         const int x0 = box.x0 + kRestrictBandHost, x1 = box.x1 - kRestrictBandHost;
         const int y0 = box.y0 + kRestrictBandHost, y1 = box.y1 - kRestrictBandHost;
-        int b[4];
-        ++launches;
-        if (device_solid_bbox(coarse.d, coarse.flags, stream, b) != cudaSuccess) return;
+        const int* b = coarse.solidBox;
         forcesFromFine = b[2] < 0 || (b[0] >= x0 && b[2] < x1 && b[1] >= y0 && b[3] < y1);
     }
 
@@ -656,6 +621,7 @@ struct fcfd_solver {
         freeStaged();
         freeFine();
         coarse.free_all();
+        geomScratch.release();
         dfree(aaSlice);
         dfree(rho); dfree(u); dfree(v); dfree(w); dfree(dForce); dfree(dNan); dfree(dStatus);
         dfree(dNetW);

@@ -1,5 +1,4 @@
-// Per-level kernels around the stream-collide: cell-kind and pull-link
-// classification, equilibrium / speck / macroscopic initialisation, the NaN
+// Per-level kernels around the stream-collide: equilibrium / speck / macroscopic initialisation, the NaN
 // watchdog, FP32 <-> storage conversion, the AA layout's conversions, and the
 // FP16-storage stream-collide (the deviation collision body of
 // collide_common.cuh; the FP32 storage collide lives in collide_f32.cu,
@@ -15,57 +14,6 @@ namespace fcfd {
 namespace {
 
 constexpr int kBlock1D = 256;
-
-/// kind = flag | kNearWall for fluid cells with a solid/slip pull neighbour;
-/// links (when given): the classes of the 18 pull links (kernels.h).
-__global__ void classify_kernel(const std::uint8_t* __restrict__ flags,
-                                std::uint8_t* __restrict__ kind, int nx, int ny, int nz,
-                                uint2* __restrict__ links) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= nx) return;
-    const int y = blockIdx.y, z = blockIdx.z;
-    const long long cell = x + static_cast<long long>(nx) * (y + static_cast<long long>(ny) * z);
-    const std::uint8_t fl = flags[cell] & kFlagMask;
-    std::uint8_t out = fl;
-    unsigned long long m = 0;
-    if (fl == kFluid) {
-#pragma unroll
-        for (int q = 1; q < kQ; ++q) {
-            int xs = x - cx(q), ys = y - cy(q), zs = z - cz(q);
-            xs = xs < 0 ? xs + nx : (xs >= nx ? xs - nx : xs);
-            ys = ys < 0 ? ys + ny : (ys >= ny ? ys - ny : ys);
-            zs = zs < 0 ? zs + nz : (zs >= nz ? zs - nz : zs);
-            const int nf = flags[xs + static_cast<long long>(nx) * (ys + static_cast<long long>(ny) * zs)] & kFlagMask;
-            if (nf == kSolid) m |= 1ull << (q - 1);
-            if (is_slip_y(nf)) m |= 1ull << (17 + q);
-            if (is_slip_z(nf)) m |= 1ull << (35 + q);
-        }
-        if (m != 0) out |= kNearWall;
-    }
-    kind[cell] = out;
-    if (links) links[cell] = make_uint2(static_cast<unsigned>(m), static_cast<unsigned>(m >> 32));
-}
-
-/// Tile codes (kernels.h): one warp per 32 cells, so a block writes the
-/// words of its tiles.
-__global__ void __launch_bounds__(256)
-tile_codes_kernel(const std::uint8_t* __restrict__ kind, std::uint8_t* __restrict__ codes, int nx, int ny, int nz,
-                  unsigned n, FastDiv divX, FastDiv divY) {
-    const unsigned cell = blockIdx.x * 256u + threadIdx.x;
-    bool bulk = false, idle = true;
-    if (cell < n) {
-        const int k = kind[cell], flag = k & kFlagMask;
-        idle = !(flag == kFluid || flag == kInlet || flag == kOutlet || flag == kOutletEq);
-        if (k == kFluid) {
-            const unsigned row = fdiv(cell, divX), z = fdiv(row, divY);
-            const int x = static_cast<int>(cell - row * divX.d), y = static_cast<int>(row - z * divY.d);
-            bulk = x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && static_cast<int>(z) < nz - 1;
-        }
-    }
-    const bool all = __all_sync(0xffffffffu, bulk), none = __all_sync(0xffffffffu, idle);
-    if ((threadIdx.x & 31) == 0 && cell / 128 < (n + 127) / 128)
-        codes[cell >> 5] = all ? kTileBulk : (none ? kTileIdle : kTileGeneral);
-}
 
 template <class S>
 __global__ void init_eq_kernel(typename S::T* __restrict__ f, const std::uint8_t* __restrict__ kind,
@@ -204,21 +152,6 @@ inline dim3 plane_grid(const LevelDims& d, int bx) {
 }
 
 } // namespace
-
-cudaError_t launch_classify(const std::uint8_t* flags, std::uint8_t* kind, LevelDims d,
-                            cudaStream_t st, uint2* links) {
-    if (!flags || !kind || d.cells() <= 0) return cudaErrorInvalidValue;
-    classify_kernel<<<plane_grid(d, 128), 128, 0, st>>>(flags, kind, d.nx, d.ny, d.nz, links);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_tile_codes(const std::uint8_t* kind, std::uint32_t* tiles, LevelDims d, cudaStream_t st) {
-    if (!kind || !tiles || d.cells() <= 0 || d.nx < 2 || d.ny < 2) return cudaErrorInvalidValue;
-    tile_codes_kernel<<<blocks_for(d.cells()), 256, 0, st>>>(
-        kind, reinterpret_cast<std::uint8_t*>(tiles), d.nx, d.ny, d.nz, static_cast<unsigned>(d.cells()),
-        fast_div(static_cast<unsigned>(d.nx)), fast_div(static_cast<unsigned>(d.ny)));
-    return cudaGetLastError();
-}
 
 cudaError_t launch_collide(Storage s, const void* src, void* dst, const std::uint8_t* kind, LevelDims d,
                            const CollideParams& p, float* rho, float* u, float* v, float* w, SlipField slip,
