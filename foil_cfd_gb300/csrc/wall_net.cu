@@ -4,18 +4,17 @@
 // seed + one correction). Extends the reference's wall model
 // (src/sim/lbm_wallmodel.cu:31-196), which has no learned part.
 //
-// Training: one thread per sample runs the forward pass (BF16 weights,
-// FP32 arithmetic) and back-propagates the squared error of the normalised
-// log u_tau; the per-sample activations and deltas go to shared memory, and
-// the block then reduces them into its partial gradient (one entry per
-// thread-pass, samples summed in a fixed order). The last block of the launch
-// to finish sums the block partials in block order -- training is
-// deterministic for a given seed -- updates the FP32 master weights (Adam)
-// and rounds them to BF16 for the next step: one launch per training step. The network is ~2.3 kFLOP per sample: CUDA-core FP32 FMAs from
-// shared-memory weights; a 2M-sample epoch is a fraction of a millisecond of
-// arithmetic, so the training is launch-bound, not FLOP-bound.
+// Training: a block takes 64 samples with 512 threads, eight per sample, four
+// units of each layer per thread; the layers' values pass through shared
+// memory, and the block reduces its partial gradient (samples summed in a
+// fixed order). A second kernel sums the block partials in block order --
+// training is deterministic for a given seed -- updates the FP32 master weights
+// (Adam) and rounds them to BF16 for the next step. The network is ~2.3 kFLOP
+// per sample and a step of 2048 samples a chain of short dependent phases on
+// 32 SMs: latency bounds it.
 #include "../../include/foilcfd_wallnet.h"
 #include "kernels.h"
+#include "pdl.cuh"
 #include "wallnet.cuh"
 
 #include <cuda_runtime.h>
@@ -31,10 +30,12 @@ using namespace fcfd::wallnet;
 namespace {
 
 constexpr int kTrainBlock = 64;            // samples per training block
+constexpr int kTrainThreads = 512;         // its threads: eight per sample
 constexpr int kMaxTrainBlocks = 1024;      // => at most 65,536 samples per step
 constexpr int kPartialStride = kParams + 1; // gradient + loss
 constexpr int kSolveBlock = 128;
-constexpr int kRowPad = kH + 1;            // shared rows padded against bank conflicts
+constexpr int kSampleRow = kH + 4;         // a sample's values over the units, in float4s without bank conflicts
+constexpr int kAdamBlock = 64;             // parameters per block of the Adam step
 
 std::uint16_t f32_to_bf16_bits(float f) {
     std::uint32_t u;
@@ -73,137 +74,221 @@ struct AdamStep {
     float* v = nullptr;
     float lr = 0.0f, beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f, bc1 = 1.0f, bc2 = 1.0f;
     float* lossOut = nullptr;      // nullable: the step's mean loss
-    unsigned* ticket = nullptr;    // block-completion counter, zero between steps
 };
 
-/// Adam update of parameter p from the block partials, summed in block order.
-__device__ __forceinline__ void adam_update(const float* __restrict__ partials, int nb, int p, const AdamStep& a,
-                                            float invCount, std::uint16_t* __restrict__ wbf) {
+/// The Adam step: each thread sums its parameter's (the last one the loss's)
+/// block partials in block order, sixteen loads in flight, and updates it. A
+/// kernel of its own: the last block of the gradient launch doing this read
+/// 156 KB through one SM and took 3.5 of that step's 11.5 us.
+__global__ void __launch_bounds__(kAdamBlock)
+adam_kernel(const float* __restrict__ partials, int nb, AdamStep a, float invCount, std::uint16_t* __restrict__ wbf) {
+    const int p = blockIdx.x * kAdamBlock + threadIdx.x;
+    const bool own = p < kParams;
+    // The state is the previous Adam step's, complete before the gradient
+    // launch in between began its work.
+    const float m = own ? __ldcg(a.m + p) : 0.0f, v = own ? __ldcg(a.v + p) : 0.0f;
+    const float w0 = own ? __ldcg(a.master + p) : 0.0f;
+    pdl_wait();
+    asm volatile("griddepcontrol.launch_dependents;");
+    if (p > kParams) return;
     float g = 0.0f;
-    for (int b = 0; b < nb; ++b) g += __ldcg(partials + static_cast<size_t>(b) * kPartialStride + p);
-    if (p == kParams) {
+    for (int b0 = 0; b0 < nb; b0 += 16) {
+        float x[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            x[k] = b0 + k < nb ? __ldcg(partials + static_cast<size_t>(b0 + k) * kPartialStride + p) : -0.0f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) g += x[k];   // + -0 changes nothing
+    }
+    if (!own) {
         if (a.lossOut) *a.lossOut = g * invCount;
         return;
     }
-    const float mm = a.beta1 * a.m[p] + (1.0f - a.beta1) * g;
-    const float vv = a.beta2 * a.v[p] + (1.0f - a.beta2) * g * g;
+    const float mm = __fmaf_rn(1.0f - a.beta1, g, __fmul_rn(a.beta1, m));
+    const float vv = __fmaf_rn(__fmul_rn(1.0f - a.beta2, g), g, __fmul_rn(a.beta2, v));
     a.m[p] = mm;
     a.v[p] = vv;
-    const float w = a.master[p] - a.lr * (mm / a.bc1) / (sqrtf(vv / a.bc2) + a.eps);
+    const float w = w0 - a.lr * (mm / a.bc1) / (sqrtf(vv / a.bc2) + a.eps);
     a.master[p] = w;
     wbf[p] = f32_to_bf16_dev(w);
 }
 
+/// dst += w . src over four consecutive indices.
+__device__ __forceinline__ float fma4(const float4& w, const float4& src, float dst) {
+    return __fmaf_rn(w.w, src.w, __fmaf_rn(w.z, src.z, __fmaf_rn(w.y, src.y, __fmaf_rn(w.x, src.x, dst))));
+}
+
 /// Forward + backward of one block of samples; writes the block's partial
 /// gradient (sum over its samples of dL/dp, L = invCount * sum err^2) and
-/// partial loss (sum err^2) to partials[blockIdx.x]. With ADAM, the block
-/// that finishes last (ticket counter) then sums all partials in block order
-/// and applies the Adam step, so one launch is one training step and the
-/// result does not depend on block scheduling.
-template <bool ADAM>
-__global__ void __launch_bounds__(kTrainBlock)
-grad_kernel(std::uint16_t* __restrict__ wbf, Norm nm, SampleView S, unsigned long long permA,
+/// partial loss (sum err^2) to partials[blockIdx.x].
+///
+/// A warp holds 32 samples and four units of a layer: weights are read as
+/// broadcasts, a sample's values in float4s. Every sum runs over its terms in
+/// index order in one thread. With one thread per sample (64 threads a block,
+/// 18 parameter sums each) a step of 2048 samples took 49.7 us; this one and
+/// the Adam step take 7.4 us, of 256 samples 6.7.
+/// `early`: the samples may be read before the previous launch has completed.
+__global__ void __launch_bounds__(kTrainThreads)
+grad_kernel(const std::uint16_t* __restrict__ wbf, Norm nm, SampleView S, unsigned long long permA,
             unsigned long long permC, unsigned long long pos0, int count, float invCount,
-            float* __restrict__ partials, AdamStep adam) {
-    __shared__ float P[kParams];
-    __shared__ float h1s[kTrainBlock][kRowPad];
-    __shared__ float h2s[kTrainBlock][kRowPad];
-    __shared__ float dz1s[kTrainBlock][kRowPad];
-    __shared__ float dz2s[kTrainBlock][kRowPad];
-    __shared__ float xs[kTrainBlock][4];
-    __shared__ float dys[kTrainBlock];
-    __shared__ float errs[kTrainBlock];
-    load_params(wbf, P);
-    __syncthreads();
-
-    const int t = threadIdx.x;
-    const int local = blockIdx.x * kTrainBlock + t;
+            float* __restrict__ partials, int early) {
+    __shared__ __align__(16) float P[kParams + 7];
+    __shared__ __align__(16) float h1s[kTrainBlock][kSampleRow], h2s[kTrainBlock][kSampleRow];
+    __shared__ __align__(16) float dz1s[kTrainBlock][kSampleRow], dz2s[kTrainBlock][kSampleRow];
+    __shared__ float xs[kTrainBlock][5], tns[kTrainBlock], dys[kTrainBlock], errs[kTrainBlock];
+    const int t = threadIdx.x, warp = t >> 5;
+    const int s = 32 * (warp & 1) + (t & 31), u0 = 4 * (warp >> 1);   // sample, first unit
+    const int local = blockIdx.x * kTrainBlock + s;
     const bool valid = local < count;
-    float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f, tn = 0.0f;
-    if (valid) {
-        const unsigned long long idx = (permA * (pos0 + static_cast<unsigned long long>(local)) + permC) % S.n;
-        const float ut = S.ut[idx], ys = S.ys[idx], nu = S.nu[idx], tau = S.tau[idx];
-        net_inputs(nm, ut, ys, nu, x0, x1, x2);
-        tn = (logf(tau) - logf(ut) - nm.outMean) / nm.outStd;
+    auto load_sample = [&] {
+        float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f, tn = 0.0f;
+        if (valid) {
+            const unsigned long long idx = (permA * (pos0 + static_cast<unsigned long long>(local)) + permC) % S.n;
+            const float ut = S.ut[idx], ys = S.ys[idx], nu = S.nu[idx], tau = S.tau[idx];
+            net_inputs(nm, ut, ys, nu, x0, x1, x2);
+            tn = (logf(tau) - logf(ut) - nm.outMean) / nm.outStd;
+        }
+        xs[s][0] = x0; xs[s][1] = x1; xs[s][2] = x2;
+        tns[s] = tn;
+    };
+    if (early && u0 == 0) load_sample();
+    pdl_wait();
+    // The next launch may come up now, on the SMs this one leaves idle.
+    asm volatile("griddepcontrol.launch_dependents;");
+    if (!early && u0 == 0) load_sample();
+    // Parameters, eight per thread (the array starts on 16 bytes).
+    if (t < kParams / 8) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(wbf) + t);
+        const std::uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            P[8 * t + 2 * k] = __uint_as_float(w[k] << 16);
+            P[8 * t + 2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+        }
+    } else if (t < kParams / 8 + kParams % 8) {
+        const int p = kParams / 8 * 8 + t - kParams / 8;
+        P[p] = bf16_bits_to_f32(__ldcg(wbf + p));
     }
-    // Forward: h1 stays in registers, h2 goes to shared memory as it is made.
-    float h1[kH];
-#pragma unroll
-    for (int j = 0; j < kH; ++j)
-        h1[j] = tanhf(P[kOffB1 + j] + P[kOffW1 + 3 * j] * x0 + P[kOffW1 + 3 * j + 1] * x1
-                      + P[kOffW1 + 3 * j + 2] * x2);
-    float y = P[kOffB3];
-#pragma unroll 2
-    for (int j = 0; j < kH; ++j) {
-        float z = P[kOffB2 + j];
-#pragma unroll
-        for (int k = 0; k < kH; ++k) z += P[kOffW2 + kH * j + k] * h1[k];
-        const float h2 = tanhf(z);
-        h2s[t][j] = h2;
-        y += P[kOffW3 + j] * h2;
-    }
-    const float err = valid ? y - tn : 0.0f;
-    const float dy = 2.0f * err * invCount;
-
-    // Backward: dz2 = dy W3 (1 - h2^2); dh1 = W2^T dz2; dz1 = dh1 (1 - h1^2).
-    float dh1[kH];
-#pragma unroll
-    for (int k = 0; k < kH; ++k) dh1[k] = 0.0f;
-#pragma unroll 2
-    for (int j = 0; j < kH; ++j) {
-        const float h2 = h2s[t][j];
-        const float dz2 = dy * P[kOffW3 + j] * (1.0f - h2 * h2);
-        dz2s[t][j] = dz2;
-#pragma unroll
-        for (int k = 0; k < kH; ++k) dh1[k] += P[kOffW2 + kH * j + k] * dz2;
-    }
-#pragma unroll
-    for (int k = 0; k < kH; ++k) {
-        h1s[t][k] = h1[k];
-        dz1s[t][k] = dh1[k] * (1.0f - h1[k] * h1[k]);
-    }
-    xs[t][0] = x0; xs[t][1] = x1; xs[t][2] = x2;
-    dys[t] = dy;
-    errs[t] = err * err;
     __syncthreads();
 
-    // Block reduction: parameter p summed over the block's samples in order.
-    float* out = partials + static_cast<size_t>(blockIdx.x) * kPartialStride;
-    for (int p = t; p < kPartialStride; p += kTrainBlock) {
-        float acc = 0.0f;
-        if (p < kOffB1) {
-            const int j = p / 3, i = p % 3;
-            for (int s = 0; s < kTrainBlock; ++s) acc += dz1s[s][j] * xs[s][i];
-        } else if (p < kOffW2) {
-            const int j = p - kOffB1;
-            for (int s = 0; s < kTrainBlock; ++s) acc += dz1s[s][j];
-        } else if (p < kOffB2) {
-            const int j = (p - kOffW2) / kH, k = (p - kOffW2) % kH;
-            for (int s = 0; s < kTrainBlock; ++s) acc += dz2s[s][j] * h1s[s][k];
-        } else if (p < kOffW3) {
-            const int j = p - kOffB2;
-            for (int s = 0; s < kTrainBlock; ++s) acc += dz2s[s][j];
-        } else if (p < kOffB3) {
-            const int j = p - kOffW3;
-            for (int s = 0; s < kTrainBlock; ++s) acc += dys[s] * h2s[s][j];
-        } else if (p == kOffB3) {
-            for (int s = 0; s < kTrainBlock; ++s) acc += dys[s];
-        } else {
-            for (int s = 0; s < kTrainBlock; ++s) acc += errs[s];
-        }
-        out[p] = acc;
+    // Layer 1.
+    const float x0 = xs[s][0], x1 = xs[s][1], x2 = xs[s][2];
+    float h1[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int j = u0 + e;
+        h1[e] = tanhf(__fmaf_rn(P[kOffW1 + 3 * j + 2], x2,
+                                __fmaf_rn(P[kOffW1 + 3 * j + 1], x1, __fmaf_rn(P[kOffW1 + 3 * j], x0, P[kOffB1 + j]))));
     }
-    if (ADAM) {
-        __shared__ bool last;
-        __threadfence();
-        __syncthreads();
-        if (t == 0) last = atomicAdd(adam.ticket, 1u) == gridDim.x - 1;
-        __syncthreads();
-        if (!last) return;
-        __threadfence();
-        for (int p = t; p < kPartialStride; p += kTrainBlock)
-            adam_update(partials, gridDim.x, p, adam, invCount, wbf);
-        if (t == 0) *adam.ticket = 0u;
+    *reinterpret_cast<float4*>(&h1s[s][u0]) = make_float4(h1[0], h1[1], h1[2], h1[3]);
+    __syncthreads();
+
+    // Layer 2.
+    float h2[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h2[e] = P[kOffB2 + u0 + e];
+#pragma unroll
+    for (int k = 0; k < kH; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(&h1s[s][k]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            h2[e] = fma4(*reinterpret_cast<const float4*>(P + kOffW2 + kH * (u0 + e) + k), a, h2[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h2[e] = tanhf(h2[e]);
+    *reinterpret_cast<float4*>(&h2s[s][u0]) = make_float4(h2[0], h2[1], h2[2], h2[3]);
+    __syncthreads();
+
+    // Output and error (every thread of a sample forms them), dz2 = dy W3 (1 - h2^2).
+    float y = P[kOffB3];
+#pragma unroll
+    for (int j = 0; j < kH; j += 4)
+        y = fma4(*reinterpret_cast<const float4*>(P + kOffW3 + j), *reinterpret_cast<const float4*>(&h2s[s][j]), y);
+    const float err = valid ? y - tns[s] : 0.0f;
+    const float dy = 2.0f * err * invCount;
+    float d[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        d[e] = __fmul_rn(__fmul_rn(dy, P[kOffW3 + u0 + e]), __fmaf_rn(-h2[e], h2[e], 1.0f));
+    *reinterpret_cast<float4*>(&dz2s[s][u0]) = make_float4(d[0], d[1], d[2], d[3]);
+    if (u0 == 0) {
+        dys[s] = dy;
+        errs[s] = err * err;
+    }
+    __syncthreads();
+
+    // dh1 = W2^T dz2, dz1 = dh1 (1 - h1^2).
+    float dh1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int j = 0; j < kH; j += 4) {
+        const float4 z = *reinterpret_cast<const float4*>(&dz2s[s][j]);
+        const float zj[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 w = *reinterpret_cast<const float4*>(P + kOffW2 + kH * (j + i) + u0);
+            dh1[0] = __fmaf_rn(w.x, zj[i], dh1[0]);
+            dh1[1] = __fmaf_rn(w.y, zj[i], dh1[1]);
+            dh1[2] = __fmaf_rn(w.z, zj[i], dh1[2]);
+            dh1[3] = __fmaf_rn(w.w, zj[i], dh1[3]);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) d[e] = __fmul_rn(dh1[e], __fmaf_rn(-h1[e], h1[e], 1.0f));
+    *reinterpret_cast<float4*>(&dz1s[s][u0]) = make_float4(d[0], d[1], d[2], d[3]);
+    __syncthreads();
+
+    // The block's sums over its samples, in their order: four warps take W2,
+    // 2 x 4 entries a thread; the others one entry of the rest a thread.
+    float* out = partials + static_cast<size_t>(blockIdx.x) * kPartialStride;
+    constexpr int kW2Threads = 128;
+    if (t < kW2Threads) {
+        const int j = 2 * (t >> 3), k = 4 * (t & 7);
+        float a[2][4] = {};
+#pragma unroll 8
+        for (int i = 0; i < kTrainBlock; ++i) {
+            const float2 z = *reinterpret_cast<const float2*>(&dz2s[i][j]);
+            const float4 h = *reinterpret_cast<const float4*>(&h1s[i][k]);
+            a[0][0] = __fmaf_rn(z.x, h.x, a[0][0]);
+            a[0][1] = __fmaf_rn(z.x, h.y, a[0][1]);
+            a[0][2] = __fmaf_rn(z.x, h.z, a[0][2]);
+            a[0][3] = __fmaf_rn(z.x, h.w, a[0][3]);
+            a[1][0] = __fmaf_rn(z.y, h.x, a[1][0]);
+            a[1][1] = __fmaf_rn(z.y, h.y, a[1][1]);
+            a[1][2] = __fmaf_rn(z.y, h.z, a[1][2]);
+            a[1][3] = __fmaf_rn(z.y, h.w, a[1][3]);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) out[kOffW2 + kH * (j + r) + k + e] = a[r][e];
+    } else {
+        const int p = t - kW2Threads;
+        float acc = 0.0f;
+        if (p < 3 * kH) {                         // W1
+#pragma unroll 8
+            for (int i = 0; i < kTrainBlock; ++i) acc = __fmaf_rn(dz1s[i][p / 3], xs[i][p % 3], acc);
+            out[kOffW1 + p] = acc;
+        } else if (p < 4 * kH) {                  // b1
+#pragma unroll 8
+            for (int i = 0; i < kTrainBlock; ++i) acc += dz1s[i][p - 3 * kH];
+            out[kOffB1 + p - 3 * kH] = acc;
+        } else if (p < 5 * kH) {                  // b2
+#pragma unroll 8
+            for (int i = 0; i < kTrainBlock; ++i) acc += dz2s[i][p - 4 * kH];
+            out[kOffB2 + p - 4 * kH] = acc;
+        } else if (p < 6 * kH) {                  // W3
+#pragma unroll 8
+            for (int i = 0; i < kTrainBlock; ++i) acc = __fmaf_rn(dys[i], h2s[i][p - 5 * kH], acc);
+            out[kOffW3 + p - 5 * kH] = acc;
+        } else if (p == 6 * kH) {                 // b3
+#pragma unroll 8
+            for (int i = 0; i < kTrainBlock; ++i) acc += dys[i];
+            out[kOffB3] = acc;
+        } else if (p == 6 * kH + 32) {            // loss, in another warp
+#pragma unroll 8
+            for (int i = 0; i < kTrainBlock; ++i) acc += errs[i];
+            out[kParams] = acc;
+        }
     }
 }
 
@@ -337,7 +422,6 @@ struct fcfd_wallnet {
     float* dLoss = nullptr;
     int* dCounters = nullptr;
     unsigned long long* dIters = nullptr;
-    unsigned* dTicket = nullptr;
     long long adamStep = 0;
     bool ok = false;
 
@@ -389,8 +473,6 @@ fcfd_wallnet* fcfd_wallnet_create(void) {
     ok = ok && cudaMalloc(&n->dLoss, 4) == cudaSuccess;
     ok = ok && cudaMalloc(&n->dCounters, 2 * sizeof(int)) == cudaSuccess;
     ok = ok && cudaMalloc(&n->dIters, sizeof(unsigned long long)) == cudaSuccess;
-    ok = ok && cudaMalloc(&n->dTicket, sizeof(unsigned)) == cudaSuccess;
-    ok = ok && cudaMemset(n->dTicket, 0, sizeof(unsigned)) == cudaSuccess;
     n->ok = ok;
     fcfd_wallnet_norm unit{{0, 0, 0}, {1, 1, 1}, 0, 1};
     n->setNorm(unit);
@@ -405,7 +487,7 @@ fcfd_wallnet* fcfd_wallnet_create(void) {
 void fcfd_wallnet_destroy(fcfd_wallnet* n) {
     if (!n) return;
     cudaFree(n->dMaster); cudaFree(n->dM); cudaFree(n->dV); cudaFree(n->dW); cudaFree(n->dPartials);
-    cudaFree(n->dAcc); cudaFree(n->dLoss); cudaFree(n->dCounters); cudaFree(n->dIters); cudaFree(n->dTicket);
+    cudaFree(n->dAcc); cudaFree(n->dLoss); cudaFree(n->dCounters); cudaFree(n->dIters);
     delete n;
 }
 
@@ -486,9 +568,8 @@ int fcfd_wallnet_gradient(fcfd_wallnet* n, const float* ut, const float* ys, con
     for (int pos = 0; pos < count; pos += chunk) {
         const int c = std::min(chunk, count - pos);
         const int nb = (c + kTrainBlock - 1) / kTrainBlock;
-        grad_kernel<false><<<nb, kTrainBlock, 0, st>>>(n->dW, n->norm, S, 1ULL, 0ULL,
-                                                       static_cast<unsigned long long>(pos), c, inv, n->dPartials,
-                                                       AdamStep{});
+        grad_kernel<<<nb, kTrainThreads, 0, st>>>(n->dW, n->norm, S, 1ULL, 0ULL, static_cast<unsigned long long>(pos), c,
+                                                  inv, n->dPartials, 0);
         accumulate_kernel<<<(kPartialStride + 255) / 256, 256, 0, st>>>(n->dPartials, nb, n->dAcc);
     }
     std::vector<double> h(kPartialStride);
@@ -545,11 +626,22 @@ int fcfd_wallnet_train(fcfd_wallnet* n, const float* ut, const float* ys, const 
             as.bc1 = static_cast<float>(1.0 - std::pow(static_cast<double>(o->beta1), n->adamStep));
             as.bc2 = static_cast<float>(1.0 - std::pow(static_cast<double>(o->beta2), n->adamStep));
             as.lossOut = sidx == stepsPerEpoch - 1 ? dHist + ep : nullptr;
-            as.ticket = n->dTicket;
-            grad_kernel<true><<<nb, kTrainBlock, 0, st>>>(n->dW, n->norm, S, a, c, static_cast<unsigned long long>(pos),
-                                                          cnt, inv, n->dPartials, as);
+            // The first gradient launch is an ordinary one: whatever made the
+            // samples and the weights is complete before it, and so before
+            // every later launch.
+            if (t == 0) {
+                grad_kernel<<<nb, kTrainThreads, 0, st>>>(n->dW, n->norm, S, a, c, static_cast<unsigned long long>(pos),
+                                                          cnt, inv, n->dPartials, 0);
+                e = cudaGetLastError();
+            } else {
+                e = launch_pdl(grad_kernel, nb, kTrainThreads, st, n->dW, n->norm, S, a, c,
+                               static_cast<unsigned long long>(pos), cnt, inv, n->dPartials, 1);
+            }
+            if (e == cudaSuccess)
+                e = launch_pdl(adam_kernel, (kPartialStride + kAdamBlock - 1) / kAdamBlock, kAdamBlock, st, n->dPartials,
+                               nb, as, inv, n->dW);
+            if (e != cudaSuccess) break;
         }
-        e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(hist.data(), dHist, o->epochs * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
