@@ -125,6 +125,29 @@ def test_learned_seed_accuracy_and_gain(wn, wo, trained):
     assert sn["newton_iterations"] < sj["newton_iterations"], (sj, sn)
 
 
+@pytest.mark.parametrize("n", [1, 255, 257, 4099])
+@pytest.mark.parametrize("method", ["NEWTON64", "LEARNED", "NEWTON64_NET"])
+def test_solves_without_statistics_match_the_counted_ones(wn, trained, method, n):
+    """The short FP64 solve, with sizes around a block, y+ far outside the trained
+    range and numbers that FP32 Newton cannot follow. Both stop at a step of 1e-8,
+    so two results round to the same or to neighbouring floats."""
+    r = np.random.default_rng(n)
+    ut = np.exp(r.uniform(np.log(1e-6), np.log(10.0), n)).astype(np.float32)
+    ys = np.exp(r.uniform(np.log(1e-3), np.log(1e3), n)).astype(np.float32)
+    nu = np.exp(r.uniform(np.log(1e-9), np.log(1.0), n)).astype(np.float32)
+    if n > 1:
+        ut[:9] = [0.0, -1.0, 1.0, 1e-30, 1e30, np.inf, np.nan, 1.0, 1e-38]
+        ys[:9] = [1.0, 1.0, 1e25, 1.0, 1.0, 1.0, 1.0, 1e-30, 0.5]
+        nu[:9] = [1e-3, 1e-3, 1e-25, 1e-3, 1e-3, 1e-3, 1e-3, 1e30, 1e-2]
+    t = [cuda(a) for a in (ut, ys, nu)]
+    net = None if method == "NEWTON64" else trained[0]
+    m = getattr(wn, method)
+    kw = {} if net is None else {"net": net}
+    want, _ = wn.utau_solve(m, *t, **kw)
+    got, st = wn.utau_solve(m, *t, stats=False, **kw)
+    np.testing.assert_allclose(got.cpu().numpy(), want.cpu().numpy(), rtol=1.2e-7, atol=0, equal_nan=True)
+
+
 def _time(fn, reps=5):
     best = float("inf")
     for _ in range(reps):
