@@ -328,13 +328,13 @@ __device__ __forceinline__ void collide_dev_lanes(V (&g)[kQ], float tau0, float 
         const int a = 2 * p - 1;
         const float w = wgt(a);
         const V cu = dot_lane<V>(a, ux, uy, uz);
-        const V es = L::mul(L::s(w), L::fma(L::mul(r45, cu), cu, A));
-        const V ea = L::mul(L::mul(L::s(3.0f * w), rho), cu);
-        const V hs = L::mul(L::s(0.5f), s[p]), hd = L::mul(L::s(0.5f), d[p]);
-        const V sym = L::fma(L::neg(omP), L::sub(hs, es), hs);
-        const V asym = L::fma(L::neg(omM), L::sub(hd, ea), hd);
-        g[a] = L::add(sym, asym);
-        g[a + 1] = L::sub(sym, asym);
+        // Sums over the pair, twice the parts: halved (exactly) in the last step.
+        const V es = L::mul(L::s(2.0f * w), L::fma(L::mul(r45, cu), cu, A));
+        const V ea = L::mul(L::mul(L::s(6.0f * w), rho), cu);
+        const V sym = L::fma(L::neg(omP), L::sub(s[p], es), s[p]);
+        const V half = L::mul(L::s(0.5f), L::fma(L::neg(omM), L::sub(d[p], ea), d[p]));
+        g[a] = L::fma(L::s(0.5f), sym, half);
+        g[a + 1] = L::fma(L::s(0.5f), sym, L::neg(half));
     }
     rhoO = rho; uxO = ux; uyO = uy; uzO = uz;
 }
@@ -771,14 +771,18 @@ collide_tile_kernel(const typename S::T* __restrict__ src, typename S::T* __rest
 // One population array A instead of the A/B pair (Bailey, Myre, Walsh, Lilja,
 // Wilson 2009, "Accelerating lattice Boltzmann fluid flow simulations using
 // graphics processors"). Between steps the array holds one of two layouts:
-//  * swapped:  A[opp(q)][x] = f*_q(x), each cell's post-collision populations
-//    with the slots of every opposite pair exchanged;
-//  * streamed: A[q][x] = f*_q(x - c_q), the post-streaming populations.
-// An odd step reads the swapped layout from the upstream cells, f_q(x) =
-// A[opp(q)][x - c_q], collides and writes f*_q(x) to A[q][x + c_q] -- the
+//  * the A/B state: A[q][x] = f*_q(x), each cell's post-collision populations;
+//  * streamed:      A[opp(q)][x] = f*_q(x - c_q), the post-streaming
+//    populations, with the slots of every opposite pair exchanged.
+// An odd step reads the A/B state from the upstream cells, f_q(x) =
+// A[q][x - c_q], collides and writes f*_q(x) to A[opp(q)][x + c_q] -- the
 // slot it read for direction opp(q) -- leaving the streamed layout. An even
-// step reads A[q][x] of its own cell and writes f*_q(x) to A[opp(q)][x],
-// leaving the swapped layout. Every cell writes exactly the slots it read and
+// step reads A[opp(q)][x] of its own cell and writes f*_q(x) to A[q][x],
+// leaving the A/B state again, which readers want and a write leaves: no pass
+// turns one into the other around an even number of steps (with the pairs
+// exchanged in the other layout, as usual, each such read and the step after
+// it cost a pass: 0.31 ms each at 8.4 M cells in FP16, two in 40 steps of
+// 0.15 ms). Every cell writes exactly the slots it read and
 // no other cell touches them, so the update is in place without races, and
 // the non-coherent loads never see a slot another thread has written. The
 // populations entering each collision are the A/B kernel's, so the results
@@ -794,8 +798,8 @@ __device__ __forceinline__ T* byte_add(T* p, long long b) {
     return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + b);
 }
 
-/// Byte offsets from &A[0][x] of the odd-step read A[opp(q)][x - c_q] of an
-/// interior cell; its write A[q][x + c_q] is the read offset of opp(q).
+/// Byte offsets from &A[0][x] of the odd-step read A[q][x - c_q] of an
+/// interior cell; its write A[opp(q)][x + c_q] is the read offset of opp(q).
 struct AAOffsets {
     long long rd[kQ];
 };
@@ -805,50 +809,67 @@ __host__ AAOffsets aa_offsets(int nx, int ny, long long n) {
     AAOffsets o;
     const long long sx = nx, sxy = static_cast<long long>(nx) * ny;
     for (int q = 0; q < kQ; ++q)
-        o.rd[q] = (opp(q) * n - (cx(q) + sx * cy(q) + sxy * cz(q))) * static_cast<long long>(sizeof(T));
+        o.rd[q] = (q * n - (cx(q) + sx * cy(q) + sxy * cz(q))) * static_cast<long long>(sizeof(T));
     return o;
 }
 
-template <class S, bool EXACT, bool ODD>
+/// ROWS: the grid is (row blocks, y, z) over rows of whole blocks; otherwise
+/// the blocks run over the flattened lattice, so that no row end leaves lanes
+/// idle, at two divisions per cell in odd steps. 40 steps, FP16: 101x100x100
+/// 0.91 -> 0.74 ms, 333x170x149 6.11 -> 5.79, 40x300x300 4.59 -> 3.08, but
+/// 640x192x128 9.97 -> 10.39 (FP32: 1.21 -> 0.99, 8.40 -> 8.10, 6.04 -> 4.02,
+/// 14.44 -> 14.83). Tiles staged as in collide_tile_kernel measured slower
+/// than either (5.79 -> 6.30, 9.97 -> 11.45 ms): the cut chunks of each run go
+/// back element by element.
+template <class S, bool EXACT, bool ODD, bool ROWS>
 __global__ void __launch_bounds__(kCellBlockX, S::kCellMinBlocks)
-collide_aa_kernel(typename S::T* __restrict__ A, CollideArgs a, const __grid_constant__ AAOffsets off) {
+collide_aa_kernel(typename S::T* __restrict__ A, CollideArgs a, const __grid_constant__ AAOffsets off, FastDiv divX,
+                  FastDiv divY) {
     pdl_wait();
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= a.nx) return;
-    const int y = blockIdx.y, z = blockIdx.z;
-    const unsigned unx = a.nx, uny = a.ny;
-    const unsigned cell = static_cast<unsigned>(x) + unx * (static_cast<unsigned>(y) + uny * static_cast<unsigned>(z));
     const long long n = a.n;
+    const unsigned unx = a.nx, uny = a.ny;
+    unsigned cell = blockIdx.x * kCellBlockX + threadIdx.x;
+    if constexpr (ROWS) cell += unx * (blockIdx.y + uny * blockIdx.z);
+    else if (cell >= static_cast<unsigned>(n)) return;
     using P = Pop<S, !EXACT>;
     float f[kQ], r, ux, uy, uz;
-    // One collision body for every path; the wrapped neighbour indices of a
-    // face cell are formed again for the stores rather than held across it.
-    const bool inner = ODD && interior(x, y, z, a);
     typename S::T* base = A + cell;
     if constexpr (!ODD) {
 #pragma unroll
-        for (int q = 0; q < kQ; ++q) f[q] = P::ld(A + q * n, cell, wgt(q));
-    } else if (inner) {
+        for (int q = 0; q < kQ; ++q) f[q] = P::ld(A + opp(q) * n, cell, wgt(q));
+        collide_body<EXACT>(f, a, r, ux, uy, uz);
 #pragma unroll
-        for (int q = 0; q < kQ; ++q) f[q] = P::ld(byte_add(base, off.rd[q]), 0, wgt(q));
+        for (int q = 0; q < kQ; ++q) P::st(A + q * n, cell, f[q], wgt(q));
     } else {
-        const Nbr b = neighbours(x, y, z, a.nx, a.ny, a.nz);
+        int x, y, z;
+        if constexpr (ROWS) {
+            x = blockIdx.x * kCellBlockX + threadIdx.x; y = blockIdx.y; z = blockIdx.z;
+        } else {
+            const unsigned row = fdiv(cell, divX), zu = fdiv(row, divY);
+            x = static_cast<int>(cell - row * unx); y = static_cast<int>(row - zu * uny); z = static_cast<int>(zu);
+        }
+        // One collision body for both paths; the wrapped neighbour indices of
+        // a face cell are formed again for the stores rather than held across it.
+        const bool inner = interior(x, y, z, a);
+        if (inner) {
 #pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            f[q] = P::ld(A + opp(q) * n, b.sx[1 + cx(q)] + unx * (b.sy[1 + cy(q)] + uny * b.sz[1 + cz(q)]), wgt(q));
-    }
-    collide_body<EXACT>(f, a, r, ux, uy, uz);
-    if constexpr (!ODD) {
+            for (int q = 0; q < kQ; ++q) f[q] = P::ld(byte_add(base, off.rd[q]), 0, wgt(q));
+        } else {
+            const Nbr b = neighbours(x, y, z, a.nx, a.ny, a.nz);
 #pragma unroll
-        for (int q = 0; q < kQ; ++q) P::st(A + opp(q) * n, cell, f[q], wgt(q));
-    } else if (inner) {
+            for (int q = 0; q < kQ; ++q)
+                f[q] = P::ld(A + q * n, b.sx[1 + cx(q)] + unx * (b.sy[1 + cy(q)] + uny * b.sz[1 + cz(q)]), wgt(q));
+        }
+        collide_body<EXACT>(f, a, r, ux, uy, uz);
+        if (inner) {
 #pragma unroll
-        for (int q = 0; q < kQ; ++q) P::st(byte_add(base, off.rd[opp(q)]), 0, f[q], wgt(q));
-    } else {
-        const Nbr b = neighbours(x, y, z, a.nx, a.ny, a.nz);
+            for (int q = 0; q < kQ; ++q) P::st(byte_add(base, off.rd[opp(q)]), 0, f[q], wgt(q));
+        } else {
+            const Nbr b = neighbours(x, y, z, a.nx, a.ny, a.nz);
 #pragma unroll
-        for (int q = 0; q < kQ; ++q)
-            P::st(A + q * n, b.sx[1 - cx(q)] + unx * (b.sy[1 - cy(q)] + uny * b.sz[1 - cz(q)]), f[q], wgt(q));
+            for (int q = 0; q < kQ; ++q)
+                P::st(A + opp(q) * n, b.sx[1 - cx(q)] + unx * (b.sy[1 - cy(q)] + uny * b.sz[1 - cz(q)]), f[q], wgt(q));
+        }
     }
     if (a.writeMacro) { a.rho[cell] = r; a.u[cell] = ux; a.v[cell] = uy; a.w[cell] = uz; }
 }
@@ -863,12 +884,14 @@ cudaError_t launch_collide_aa_impl(void* fv, LevelDims d, const CollideParams& p
     a.writeMacro = (p.writeMacro && rho && u && v && w) ? 1 : 0;
     a.rho = rho; a.u = u; a.v = v; a.w = w;
     T* f = static_cast<T*>(fv);
-    const int bx = d.nx >= kCellBlockX ? kCellBlockX : ((d.nx + 31) / 32) * 32;
-    const dim3 grid(static_cast<unsigned>((d.nx + bx - 1) / bx), static_cast<unsigned>(d.ny),
-                    static_cast<unsigned>(d.nz));
     const AAOffsets off = aa_offsets<T>(d.nx, d.ny, a.n);
-    return launch_pdl(odd ? collide_aa_kernel<S, EXACT, true> : collide_aa_kernel<S, EXACT, false>, grid, dim3(bx), st, f,
-                      a, off);
+    const bool rows = d.nx % kCellBlockX == 0;
+    const dim3 grid = rows ? dim3(static_cast<unsigned>(d.nx / kCellBlockX), static_cast<unsigned>(d.ny),
+                                  static_cast<unsigned>(d.nz))
+                           : dim3(static_cast<unsigned>((a.n + kCellBlockX - 1) / kCellBlockX));
+    auto kern = rows ? (odd ? collide_aa_kernel<S, EXACT, true, true> : collide_aa_kernel<S, EXACT, false, true>)
+                     : (odd ? collide_aa_kernel<S, EXACT, true, false> : collide_aa_kernel<S, EXACT, false, false>);
+    return launch_pdl(kern, grid, dim3(kCellBlockX), st, f, a, off, fast_div(d.nx), fast_div(d.ny));
 }
 
 // ---- warm-restart flag edits (applyFlagEditsKernel, lbm_core.cu:644-717) -----

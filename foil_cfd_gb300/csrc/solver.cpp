@@ -202,13 +202,11 @@ struct fcfd_solver {
     int collideKernel = 0;
     bool initialized = false;
     // AA-pattern layout (fcfd_options.layout): one population array. Between
-    // steps it holds the swapped layout (next step odd) or the streamed one
-    // (next step even) -- or, after the state was read or written through the
-    // API, the A/B state (aaAB), turned back into the swapped layout before
-    // the next step. aaSlice is the one-slice scratch of the streamed
-    // layout's conversion.
+    // steps it holds the A/B state (next step odd) or the streamed layout
+    // (next step even), which a read of the state turns into the A/B state
+    // (aaToAB); a write replaces the whole array by the A/B state. aaSlice is
+    // the one-slice scratch of that conversion.
     bool aa = false;
-    bool aaAB = false;
     int aaNextOdd = 1;
     void* aaSlice = nullptr;
 
@@ -600,7 +598,7 @@ struct fcfd_solver {
             st.pending = false;
             Level* L = levelAt(level);
             if (!L || st.bytes != static_cast<size_t>(L->n) * 19 * sizeof(float)) return cudaErrorInvalidValue;
-            if (level == 0) aaAB = aa;
+            if (level == 0) aaNextOdd = 1;
             cudaError_t e;
             if (storage == Storage::F32) {
                 e = cudaMemcpyAsync(L->f[L->src], st.buf, st.bytes, cudaMemcpyDeviceToDevice, stream);
@@ -707,11 +705,10 @@ struct fcfd_solver {
     /// AA layout: leave the A/B state (post-collision f*_q(x) in slot q of
     /// cell x) in the population array for a reader; a no-op otherwise.
     cudaError_t aaToAB() {
-        if (!aa || aaAB) return cudaSuccess;
-        launches += aaNextOdd ? 1 : 18;
-        const cudaError_t e = aaNextOdd ? launch_aa_pair_swap(storage, coarse.f[0], coarse.n, stream)
-                                        : launch_aa_shift(storage, coarse.f[0], aaSlice, coarse.d, 1, stream);
-        if (e == cudaSuccess) aaAB = true;
+        if (!aa || aaNextOdd) return cudaSuccess;
+        launches += 18;
+        const cudaError_t e = launch_aa_shift(storage, coarse.f[0], aaSlice, coarse.d, stream);
+        if (e == cudaSuccess) aaNextOdd = 1;
         return e;
     }
 
@@ -720,12 +717,6 @@ struct fcfd_solver {
         if (n <= 0) return cudaSuccess;
         pollAsync();
         if (nanLatched) return cudaSuccess;
-        if (aa && aaAB) {
-            ++launches;
-            if (auto e = launch_aa_pair_swap(storage, coarse.f[0], coarse.n, stream); e != cudaSuccess) return e;
-            aaAB = false;
-            aaNextOdd = 1;
-        }
         const bool timeIt = !timingPending;
         if (timeIt) cudaEventRecord(evT0, stream);
         for (int i = 0; i < n; ++i) {
@@ -869,7 +860,7 @@ struct fcfd_solver {
             launch_speck(storage, coarse.f[i], coarse.kind, coarse.d, kSpeckAmplitudeFrac * scaling.u_lat,
                          kSpeckSeed, stream);
         }
-        aaAB = aa;
+        aaNextOdd = 1;
         seedFine();
         seedFiner();
         resetWMState();
@@ -890,7 +881,7 @@ struct fcfd_solver {
     cudaError_t importF32(Level& L, const float* host, size_t count) {
         if (count != static_cast<size_t>(L.n) * 19) return cudaErrorInvalidValue;
         const size_t bytes = count * sizeof(float);
-        if (&L == &coarse) aaAB = aa;  // a whole A/B state replaces the layout
+        if (&L == &coarse) aaNextOdd = 1;  // a whole A/B state replaces the layout
         if (storage == Storage::F32)
             return cudaMemcpy(L.f[L.src], host, bytes, cudaMemcpyHostToDevice);
         float* stage = nullptr;
@@ -1023,7 +1014,6 @@ int fcfd_init(fcfd_solver* s, const fcfd_dims* dims, const fcfd_scaling* scaling
     s->lambda = kDefaultLambda;
     s->collideKernel = 0;
     s->aa = false;
-    s->aaAB = false;
     s->aaNextOdd = 1;
     if (opts) {
         s->storage = opts->storage == FCFD_STORE_FP16 ? Storage::F16 : Storage::F32;
@@ -1356,7 +1346,7 @@ int fcfd_restore_from_macro(fcfd_solver* s, const float* r, const float* u, cons
             e != cudaSuccess)
             return e;
     }
-    s->aaAB = s->aa;
+    s->aaNextOdd = 1;
     s->notifyRestored(false);
     if (auto e = s->seedFine(); e != cudaSuccess) return e;
     if (auto e = s->seedFiner(); e != cudaSuccess) return e;

@@ -87,8 +87,8 @@ typedef struct fcfd_options {
 
 /* Streaming layouts. AB: two population arrays, each step pulls from one
  * into the other (the reference's ping-pong, lbm_solver.cpp:1156-1160). AA:
- * one array updated in place, odd and even steps alternating between a
- * swapped and a streamed slot layout (half the population memory; same
+ * one array updated in place, odd and even steps alternating between the A/B
+ * state and a streamed slot layout (half the population memory; same
  * results bit for bit). The AA layout serves all-fluid periodic lattices
  * (every flag FCFD_FLAG_FLUID, no refinement, no link fields): fcfd_init
  * refuses other flag fields with cudaErrorNotSupported, as do

@@ -1,6 +1,6 @@
 """The AA-pattern in-place layout (fcfd_options.layout = FCFD_LAYOUT_AA):
-one population array, odd and even steps alternating between the swapped and
-the streamed slot layouts. Its populations must equal the A/B ping-pong
+one population array, odd and even steps alternating between the A/B state and
+the streamed slot layout. Its populations must equal the A/B ping-pong
 step's (the reference's layout, lbm_solver.cpp:1156-1160) bit for bit after
 any number of steps, with reads of the state at either phase and stepping
 resumed after them; it holds one population array instead of two; and it
@@ -70,6 +70,22 @@ def test_aa_equals_ab_bitwise(fc, oracle_mod, storage, dims):
         total += k
         assert np.array_equal(aa.export_f32().view(np.uint32), ab.export_f32().view(np.uint32)), total
     assert not aa.nan_detected() and not ab.nan_detected()
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16"])
+@pytest.mark.parametrize("dims", [(3, 3, 1), (5, 3, 2), (127, 5, 4), (128, 5, 4), (129, 6, 3), (384, 4, 3)])
+def test_aa_blocks_of_rows_and_of_the_flat_lattice(fc, oracle_mod, storage, dims):
+    """Rows of whole blocks run one kernel shape, all others the flat one:
+    lattices of less than a block, rows around a block, both phases read."""
+    ab, aa = _pair(fc, dims, storage)
+    f0 = _state(oracle_mod, dims)
+    ab.import_f32(f0)
+    aa.import_f32(f0)
+    for k in (1, 2, 3):
+        assert ab.step_n(k) == 0 and aa.step_n(k) == 0
+        assert np.array_equal(aa.export_f32().view(np.uint32), ab.export_f32().view(np.uint32)), k
+        for x, y in zip(aa.download_macro(), ab.download_macro()):
+            assert np.array_equal(x.view(np.uint32), y.view(np.uint32)), k
 
 
 def test_aa_reset_watchdog_and_snapshot_view(fc):
