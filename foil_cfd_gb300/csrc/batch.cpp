@@ -68,6 +68,7 @@ struct fcfd_batch {
     int sms = 0;
 
     double* dPartials = nullptr;
+    std::uint32_t* dTiles = nullptr;   // tile codes of every tunnel
     int* dLatch = nullptr;    // per-tunnel watchdog verdict (0 running), then the sample count at the latch
     int* dHealth = nullptr;   // per-tunnel max speed bits, then non-finite counts
     double* dForceCur = nullptr;
@@ -95,7 +96,8 @@ struct fcfd_batch {
         }
         t.clear();
         cudaFree(dPartials); cudaFree(dForceCur); cudaFree(dHist); cudaFree(dHistCount);
-        cudaFree(dLatch); cudaFree(dHealth);
+        cudaFree(dLatch); cudaFree(dHealth); cudaFree(dTiles);
+        dTiles = nullptr;
         dPartials = dForceCur = dHist = nullptr; dHistCount = dLatch = dHealth = nullptr;
         if (ev0) { cudaEventDestroy(ev0); ev0 = nullptr; }
         if (ev1) { cudaEventDestroy(ev1); ev1 = nullptr; }
@@ -129,6 +131,7 @@ struct fcfd_batch {
         table.lambda = lambda;
         table.smagPre = smagPre();
         table.latch = dLatch;
+        table.tiles = dTiles;
         groups.clear();
         const size_t limit = static_cast<size_t>(std::max(cfg.group_mb, 0)) << 20;
         size_t groupBytes = 0;
@@ -141,7 +144,9 @@ struct fcfd_batch {
             d.links = x.links;
             d.n = x.n;
             d.nx = x.d.nx; d.ny = x.d.ny; d.nz = x.d.nz;
-            d.xChunks = 1;  // a work item spans whole rows
+            d.divX = fast_div(static_cast<unsigned>(x.d.nx));
+            d.divY = fast_div(static_cast<unsigned>(x.d.ny));
+            batch_offsets(d);
             d.tau = x.tau; d.uIn = x.uLat;
             table.begins[i] = static_cast<unsigned>(item);
             const size_t bytes = tunnelBytes(x);
@@ -149,13 +154,19 @@ struct fcfd_batch {
                 groups.push_back(Group{item, item});
                 groupBytes = 0;
             }
-            const long long rowGroups = (static_cast<long long>(x.d.ny) * x.d.nz + cfg.rows - 1) / cfg.rows;
-            item += static_cast<long long>(d.xChunks) * rowGroups;
+            item += shape().tiles() ? (x.n + 127) / 128
+                                    : (static_cast<long long>(x.d.ny) * x.d.nz + cfg.rows - 1) / cfg.rows;
             groups.back().itemEnd = item;
             groupBytes += bytes;
         }
         if (limit == 0) groups.assign(1, Group{0, item});
         nItems = item;
+        table.begins[t.size()] = static_cast<unsigned>(item);
+        while (item >> table.itemShift >= kItemBuckets) ++table.itemShift;
+        for (int k = 0, lo = 0; k < kItemBuckets; ++k) {
+            while (lo + 1 < ntun() && table.begins[lo + 1] <= static_cast<long long>(k) << table.itemShift) ++lo;
+            table.tunnelAt[k] = static_cast<std::uint8_t>(lo);
+        }
         return item < (1LL << 31) ? cudaSuccess : cudaErrorInvalidValue;
     }
 
@@ -345,7 +356,12 @@ int fcfd_batch_init(fcfd_batch* b, const fcfd_batch_tunnel* tunnels, int count, 
     const size_t esz = b->storage == Storage::F32 ? 4 : 2;
     int maxLinks = 0;
     GeomScratch scratch;   // of the flag tables; one tunnel after the other on the batch's stream
-    cudaError_t e = cudaSuccess;
+    size_t codes = 0, tile = 0;
+    for (int i = 0; i < count; ++i) {
+        const LevelDims d{tunnels[i].dims.nx, tunnels[i].dims.ny, tunnels[i].dims.nz};
+        if (d.cells() > 0 && d.cells() < (1LL << 31)) codes += tile_code_bytes(d.cells());
+    }
+    cudaError_t e = cudaMalloc(&b->dTiles, std::max<size_t>(codes, 4));
     for (int i = 0; i < count && e == cudaSuccess; ++i) {
         const fcfd_batch_tunnel& in = tunnels[i];
         Tunnel x;
@@ -362,7 +378,9 @@ int fcfd_batch_init(fcfd_batch* b, const fcfd_batch_tunnel* tunnels, int count, 
         x.chord = std::max(1, in.chord_cells);
         b->t.push_back(x);
         Tunnel& y = b->t.back();
-        for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaMalloc(&y.f[k], static_cast<size_t>(y.n) * 19 * esz);
+        // The last chunk of a staged run may reach 16 bytes past the last slice.
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+            e = cudaMalloc(&y.f[k], static_cast<size_t>(y.n) * 19 * esz + 16);
         if (e == cudaSuccess) e = cudaMalloc(&y.flags, static_cast<size_t>(y.n));
         if (e == cudaSuccess) e = cudaMalloc(&y.kind, static_cast<size_t>(y.n) + 64);
         if (e == cudaSuccess && b->storage == Storage::F32)   // the FP16 batch step does not read them
@@ -377,6 +395,8 @@ int fcfd_batch_init(fcfd_batch* b, const fcfd_batch_tunnel* tunnels, int count, 
             LevelTables t;
             t.kind = y.kind;
             t.links = y.links;
+            t.tiles = b->dTiles + tile;
+            tile += tile_code_bytes(y.n) / 4;
             e = build_level_tables(y.d, y.flags, t, scratch, b->stream);
             y.linkCells = t.linkCells;
             y.linkMasks = t.linkMasks;

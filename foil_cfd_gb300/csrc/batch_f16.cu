@@ -11,6 +11,14 @@ cudaError_t launch_batch_collide_f16(const BatchTable& tab, unsigned itemBase, u
 
 int batch_occupancy_f16(BatchShape sh) { return batch_occupancy_impl<StoreF16, false>(sh); }
 
+void batch_offsets(BatchTunnelParam& p) {
+    for (int q = 0; q < kQ; ++q) {
+        const long long shift = cx(q) + p.nx * (cy(q) + static_cast<long long>(p.ny) * cz(q));
+        p.pull[q] = static_cast<int>(q * p.n - shift);
+        p.inOff[q] = static_cast<unsigned>(q * kTileRow + 2 * (p.pull[q] & 7));
+    }
+}
+
 /// Append the current per-tunnel forces (3 doubles each) to a ring of
 /// force samples and advance its device-side count.
 __global__ void force_append_kernel(const double* __restrict__ cur, int n3, double* __restrict__ hist, int cap,

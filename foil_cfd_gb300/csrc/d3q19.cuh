@@ -9,7 +9,10 @@
 // opposite and mirror index folds away, and multiplications by 0/+-1 vanish.
 #pragma once
 
+#include "fast_div.h"
+
 #include <cstdint>
+
 #include <cuda_fp16.h>
 
 namespace fcfd {
@@ -103,21 +106,6 @@ __host__ __device__ __forceinline__ bool is_slip_z(int f) {
 constexpr float kMaxSimSpeed = 0.30f;
 constexpr float kRhoFloor = 0.05f;
 
-// ---- division by an invariant integer ----------------------------------------
-// Granlund & Montgomery 1994, "Division by invariant integers using
-// multiplication": q = (t + ((n - t) >> 1)) >> s with t = mulhi(m, n), exact
-// for every 32-bit n.
-struct FastDiv {
-    unsigned d, m;
-    int s;
-};
-/// Divisor d >= 2: m = floor(2^32 (2^l - d) / d) + 1, s = l - 1, l = ceil(log2 d).
-inline FastDiv fast_div(unsigned d) {
-    int l = 0;
-    while ((1ull << l) < d) ++l;
-    const unsigned long long m = ((1ull << 32) * ((1ull << l) - d)) / d + 1;
-    return FastDiv{d, static_cast<unsigned>(m), l - 1};
-}
 __device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv& f) {
     const unsigned t = __umulhi(n, f.m);
     return (t + ((n - t) >> 1)) >> f.s;
@@ -156,7 +144,10 @@ struct StoreF32 {
     /// per step with and without them, 3.97 M 103 with and 105 without,
     /// 7.78 M 190 and 198; 0.33 M 14.6 and 12.6.
     static constexpr long long kCodedCells = 2500000;
-    /// Resident threads per SM the batched collide is compiled for: 64
+    /// Resident 128-thread blocks per SM of the batched collide by tiles (12
+    /// tunnels: 38.3 ms per 100 steps at 12 blocks, 37.9 at 10, 40.2 at 8).
+    static constexpr int kBatchTileMinBlocks = 10;
+    /// Resident threads per SM the batched collide by rows is compiled for: 64
     /// registers (the FP16 batched polar measured 15 % slower at 1536
     /// threads, 40 registers).
     static constexpr int kBatchThreads = 1024;
@@ -198,6 +189,8 @@ struct StoreF16 {
     /// The staged tiles at 40 registers: 16 blocks (32 registers) ran 2 %
     /// slower, 10 blocks 5 %.
     static constexpr int kTileMinBlocks = 12;
+    /// 24 tunnels: 63.5 ms per 100 steps at 12 blocks, 62.1 at 10, 75 at 8.
+    static constexpr int kBatchTileMinBlocks = 10;
     /// Cells from which the collide goes by tile codes and stages its tiles:
     /// 2.62 M cells 52.1 us per step staged and 51.6 cell by cell, 3.97 M 73.6
     /// and 74.2, 7.78 M 132 and 150.

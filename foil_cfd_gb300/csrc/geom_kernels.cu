@@ -427,18 +427,10 @@ tile_codes_kernel(const std::uint8_t* __restrict__ kind, std::uint8_t* __restric
         const unsigned row = c0 / nx, z = row / ny;
         const int x = static_cast<int>(c0 - row * nx), y = static_cast<int>(row - z * ny);
         if (full && (a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) == 0) {
-            const bool inner = x > 0 && x + 31 < nx - 1 && y > 0 && y < ny - 1 && z > 0 && static_cast<int>(z) < nz - 1;
-            code = inner ? kTileBulk : kTileGeneral;
-            if (!inner) {   // the run may cross a row's end
-                bool all = true;
-                unsigned xx = x, yy = y, zz = z;
-                for (int k = 0; k < 32; ++k) {
-                    all = all && xx > 0 && static_cast<int>(xx) < nx - 1 && yy > 0 && static_cast<int>(yy) < ny - 1
-                          && zz > 0 && static_cast<int>(zz) < nz - 1;
-                    if (static_cast<int>(++xx) == nx) { xx = 0; if (static_cast<int>(++yy) == ny) { yy = 0; ++zz; } }
-                }
-                if (all) code = kTileBulk;
-            }
+            // A run across a row's end holds cells of the x faces.
+            const bool inner = x > 0 && x + 31 < nx - 1 && y > 0 && y < ny - 1 && nz > 1;
+            const int zi = static_cast<int>(z);
+            code = !inner ? kTileGeneral : zi == 0 ? kTileLowZ : zi == nz - 1 ? kTileHighZ : kTileBulk;
         } else {
             const std::uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
             for (int k = 0; k < 32 && c0 + k < n; ++k) {

@@ -65,7 +65,9 @@ enum class Storage : int { F32 = 0, F16 = 1 };
 enum : std::uint8_t {
     kTileIdle = 0,     ///< no cell that a step writes
     kTileGeneral = 1,  ///< cells to be looked at one by one
-    kTileBulk = 2      ///< all 32 bulk and off the lattice's faces
+    kTileBulk = 2,     ///< all 32 bulk and off the lattice's faces
+    kTileLowZ = 3,     ///< all 32 bulk, in plane z = 0 and off the x and y faces
+    kTileHighZ = 4     ///< the same in the last plane
 };
 /// Tile codes: one word per 128 consecutive cells, byte w the code of its
 /// cells 32 w .. 32 w + 31 (cells past the end count as idle).
@@ -196,6 +198,8 @@ cudaError_t launch_wall_harvest(Storage s, const void* f, long long cells, WallL
 /// block per work item.
 cudaError_t launch_batch_collide_f32(const BatchTable& tab, unsigned itemBase, unsigned nItems, int parity,
                                      BatchShape sh, cudaStream_t st);
+/// Pull offsets of a tunnel (nx, ny, n given).
+void batch_offsets(BatchTunnelParam& p);
 cudaError_t launch_batch_collide_f16(const BatchTable& tab, unsigned itemBase, unsigned nItems, int parity,
                                      BatchShape sh, cudaStream_t st);
 /// Resident blocks per SM of a batched collide shape (0: unknown shape).

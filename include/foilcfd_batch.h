@@ -5,9 +5,9 @@
  * (2.5-D: a few spanwise cells, periodic in z). Stepping each with its own
  * solver leaves most of the GPU idle and pays launch latency per tunnel; a
  * batch owns all of them in one device arena and advances every tunnel by
- * one step with ONE kernel launch: a grid-stride walk over work items (row
- * groups of each tunnel in x chunks) that is persistent across tunnels when
- * the grid is a few blocks per SM. Chunks of steps, with a per-tunnel
+ * one step with ONE kernel launch: a grid-stride walk over work items (tiles
+ * of 128 cells, or row groups, of each tunnel) that is persistent across
+ * tunnels when the grid is a few blocks per SM. Chunks of steps, with a per-tunnel
  * momentum-exchange force sample at their end, are captured once as CUDA
  * graphs and replayed. A project-written autotuner times the launch shapes
  * (threads per block, rows per work item, persistent vs one-item grids) on
@@ -51,7 +51,8 @@ typedef struct fcfd_batch_tunnel {
 } fcfd_batch_tunnel;
 
 /* Launch shape of the batched collide. block: 64, 128 or 256 threads (one x
- * cell each); rows: 1, 2 or 4 rows per work item; ctas_per_sm: blocks per SM
+ * cell each); rows: 1, 2 or 4 rows per work item (128 threads at one row: 128
+ * cells of the flattened lattice instead); ctas_per_sm: blocks per SM
  * of a persistent grid, 0 for one block per work item. group_mb: 0 steps all
  * tunnels with one launch per step; > 0 packs consecutive tunnels into groups
  * of at most that many MB of population buffers, and a graph-replayed chunk

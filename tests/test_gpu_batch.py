@@ -81,6 +81,37 @@ def test_shapes_and_graph_replay_are_identical(fc):
         b.close()
 
 
+def channel(dims, walls):
+    """Inlet, outlet, slip walls and a vane, or an all-fluid periodic lattice."""
+    nx, ny, nz = dims
+    f = np.zeros((nz, ny, nx), np.uint8)
+    if walls:
+        f[:, 0, :], f[:, -1, :] = 5, 4
+        f[:, :, 0] = 2
+        f[:, 1:-1, -1] = 9
+        f[:, ny // 2, nx // 2] = 1
+    return f.ravel()
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16"])
+@pytest.mark.parametrize("shape", [(128, 1, 0, 0), (128, 1, 1, 0), (128, 1, 0, 1)])
+def test_tiles_of_ragged_tunnels(fc, storage, shape):
+    """Tiles of 128 cells, one block each, looped over by a persistent grid, and
+    by groups: one, two and more planes (whose z wrap is an offset), rows below,
+    at and above a tile, cell counts that are and are not a multiple of 8."""
+    from foil_cfd_gb300.batch import PolarTunnel
+    dims = [(33, 5, 1), (64, 9, 2), (128, 8, 3), (129, 10, 3), (200, 8, 4), (333, 7, 5), (300, 40, 8), (160, 12, 16)]
+    ts = [PolarTunnel("0012", 0.0, 16, d, channel(d, w), 0.56, 0.05) for w in (True, False) for d in dims]
+    b = make_batch(ts, storage)
+    b.set_config(*shape)
+    assert b.step_n(7, use_graphs=False) == 0
+    for i, t in enumerate(ts):
+        s = single(fc, t, storage)
+        assert s.step_n(7) == 0
+        assert np.array_equal(b.export_f32(i), s.export_f32()), (t.dims, i)
+    b.close()
+
+
 def test_graph_chunks_from_odd_step_counts(fc):
     ts = small_polar()
     a = make_batch(ts, "fp32")
