@@ -67,7 +67,8 @@ struct fcfd_batch {
     long long launches = 0;
     int sms = 0;
 
-    double* dPartials = nullptr;
+    double* dPartials = nullptr;   // force scratch, partialStride per tunnel
+    size_t partialStride = 0;
     std::uint32_t* dTiles = nullptr;   // tile codes of every tunnel
     int* dLatch = nullptr;    // per-tunnel watchdog verdict (0 running), then the sample count at the latch
     int* dHealth = nullptr;   // per-tunnel max speed bits, then non-finite counts
@@ -187,15 +188,14 @@ struct fcfd_batch {
 
     /// Force of every tunnel at the current state -> dForceCur.
     cudaError_t forcesNow() {
+        ForceLists<kMaxForceLists> L;
         for (int i = 0; i < ntun(); ++i) {
             const Tunnel& x = t[i];
-            launches += 2;
-            if (auto e = launch_force(storage, x.f[parity], x.n, x.linkCells, x.linkMasks, x.linkCount, SlipField{},
-                                      dPartials, dForceCur + 3 * i, stream);
-                e != cudaSuccess)
-                return e;
+            L.list[i] = ForceList{x.f[parity], x.n, x.linkCells, x.linkMasks, x.linkCount, SlipField{},
+                                  dPartials + static_cast<size_t>(i) * partialStride, dForceCur + 3 * i};
         }
-        return cudaSuccess;
+        ++launches;
+        return launch_forces(storage, L, ntun(), stream);
     }
 
     /// Watchdog of every tunnel: a full-field scan (max |u|, non-finite
@@ -206,14 +206,10 @@ struct fcfd_batch {
     cudaError_t watchdog() {
         const int nt = ntun();
         if (auto e = cudaMemsetAsync(dHealth, 0, 2 * nt * sizeof(int), stream); e != cudaSuccess) return e;
-        for (int i = 0; i < nt; ++i) {
-            const Tunnel& x = t[i];
-            ++launches;
-            if (auto e = launch_batch_health(storage == Storage::F32, x.f[parity], x.kind, x.n, dHealth + i,
-                                             dHealth + nt + i, stream);
-                e != cudaSuccess)
-                return e;
-        }
+        ++launches;
+        if (auto e = launch_batch_health(storage == Storage::F32, table, parity, dHealth, dHealth + nt, stream);
+            e != cudaSuccess)
+            return e;
         ++launches;
         return launch_batch_latch(dHealth, dHealth + nt, nt, 0.95f * 0.3f, dHistCount, dLatch, stream);   // 0.95 x the limiter speed
     }
@@ -264,10 +260,10 @@ struct fcfd_batch {
         return e;
     }
 
-    /// Launches per replayed chunk (collides + force kernels + append).
+    /// Launches per replayed chunk (collides, forces, append, health, latch).
     long long chunkLaunches() const {
         const long long collides = cfg.group_mb > 0 ? static_cast<long long>(groups.size()) * forceEvery : forceEvery;
-        return collides + 2LL * ntun() + 1;
+        return collides + 4;
     }
 
     cudaError_t stepN(int n, bool useGraphs) {
@@ -405,7 +401,9 @@ int fcfd_batch_init(fcfd_batch* b, const fcfd_batch_tunnel* tunnels, int count, 
         }
     }
     scratch.release();
-    if (e == cudaSuccess) e = cudaMalloc(&b->dPartials, std::max(1, force_blocks(maxLinks)) * 3 * sizeof(double));
+    b->partialStride = force_scratch_bytes(maxLinks) / sizeof(double);
+    if (e == cudaSuccess) e = cudaMalloc(&b->dPartials, b->partialStride * count * sizeof(double));
+    if (e == cudaSuccess) e = cudaMemsetAsync(b->dPartials, 0, b->partialStride * count * sizeof(double), b->stream);
     if (e == cudaSuccess) e = cudaMalloc(&b->dForceCur, 3 * count * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->dHist, static_cast<size_t>(kHistCapacity) * 3 * count * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->dHistCount, sizeof(int));
@@ -566,11 +564,9 @@ int fcfd_batch_health(fcfd_batch* b, float* maxSpeed, int* nonFinite) {
     int* d = nullptr;
     if (auto e = cudaMalloc(&d, 2 * nt * sizeof(int)); e != cudaSuccess) return e;
     cudaError_t e = cudaMemsetAsync(d, 0, 2 * nt * sizeof(int), b->stream);
-    for (int i = 0; i < nt && e == cudaSuccess; ++i) {
-        const Tunnel& x = b->t[i];
-        ++b->launches;
-        e = launch_batch_health(b->storage == Storage::F32, x.f[b->parity], x.kind, x.n, d + i, d + nt + i, b->stream);
-    }
+    ++b->launches;
+    if (e == cudaSuccess)
+        e = launch_batch_health(b->storage == Storage::F32, b->table, b->parity, d, d + nt, b->stream);
     std::vector<int> h(2 * nt);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, h.size() * sizeof(int), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

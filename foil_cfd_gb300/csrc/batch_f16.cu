@@ -31,13 +31,19 @@ __global__ void force_append_kernel(const double* __restrict__ cur, int n3, doub
     if (threadIdx.x == 0) *count = c + 1;
 }
 
-/// Largest speed |j| / rho over the non-solid cells of one tunnel (float
-/// bits, atomicMax: speeds are non-negative) and the count of cells whose
-/// density is not finite.
+/// Largest speed |j| / rho over the non-solid cells of tunnel blockIdx.y
+/// (float bits, atomicMax: speeds are non-negative) and the count of cells
+/// whose density is not finite.
 template <class S>
-__global__ void health_kernel(const typename S::T* __restrict__ f, const std::uint8_t* __restrict__ kind, long long n,
-                              int* __restrict__ maxSpeedBits, int* __restrict__ nonFinite) {
+__global__ void health_kernel(const __grid_constant__ BatchTable P, int parity, int* __restrict__ maxSpeedBits,
+                              int* __restrict__ nonFinite) {
     pdl_wait();
+    const BatchTunnelParam& tp = P.t[blockIdx.y];
+    const auto* f = static_cast<const typename S::T*>(tp.f[parity]);
+    const std::uint8_t* kind = tp.kind;
+    const long long n = tp.n;
+    maxSpeedBits += blockIdx.y;
+    nonFinite += blockIdx.y;
     float best = 0.0f;
     int bad = 0;
     for (long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; c < n;
@@ -66,13 +72,13 @@ __global__ void health_kernel(const typename S::T* __restrict__ f, const std::ui
     }
 }
 
-cudaError_t launch_batch_health(bool fp32, const void* f, const std::uint8_t* kind, long long n, int* maxSpeedBits,
-                                int* nonFinite, cudaStream_t st) {
-    const unsigned nb = static_cast<unsigned>(std::min<long long>(4096, (n + 255) / 256));
-    if (fp32)
-        return launch_pdl(health_kernel<StoreF32>, nb, 256, st, static_cast<const float*>(f), kind, n, maxSpeedBits,
-                          nonFinite);
-    return launch_pdl(health_kernel<StoreF16>, nb, 256, st, static_cast<const __half*>(f), kind, n, maxSpeedBits,
+cudaError_t launch_batch_health(bool fp32, const BatchTable& tab, int parity, int* maxSpeedBits, int* nonFinite,
+                                cudaStream_t st) {
+    if (tab.ntun <= 0 || tab.ntun > kMaxBatchTunnels) return cudaErrorInvalidValue;
+    long long n = 1;
+    for (int i = 0; i < tab.ntun; ++i) n = std::max(n, tab.t[i].n);
+    const dim3 grid(static_cast<unsigned>(std::min<long long>(4096, (n + 255) / 256)), static_cast<unsigned>(tab.ntun));
+    return launch_pdl(fp32 ? health_kernel<StoreF32> : health_kernel<StoreF16>, grid, 256, st, tab, parity, maxSpeedBits,
                       nonFinite);
 }
 

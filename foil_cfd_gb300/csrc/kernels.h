@@ -135,16 +135,28 @@ cudaError_t launch_init_macro_f32(float* f, const std::uint8_t* kind, long long 
 
 // ---- force reduction (force_kernels.cu) ------------------------------------
 /// Momentum exchange over a compact wall-link list: entry i is fluid cell
-/// cells[i] with bit q of masks[i] set when the neighbour at +c_q is solid.
-/// Block partials go to `partials` (3 doubles per block, blocks =
-/// force_blocks(count)); a second single-block pass sums them in a fixed
-/// order into out[3]. Deterministic, FP64 from the per-link terms up.
-int force_blocks(int count);
-cudaError_t launch_force(Storage s, const void* f, long long cells,
-                         const std::uint32_t* linkCells,
-                         const std::uint32_t* linkMasks, int count,
-                         SlipField slip, double* partials, double* out,
-                         cudaStream_t st);
+/// cells[i] of the n cells of `f`, with bit q of masks[i] set when the
+/// neighbour at +c_q is solid. The sum goes to out[3]. Deterministic, FP64 from
+/// the per-link terms up. `scratch` (force_scratch_bytes(count), its first 8
+/// bytes zero, and zero again afterwards) serves one reduction at a time.
+struct ForceList {
+    const void* f = nullptr;
+    long long n = 0;
+    const std::uint32_t *cells = nullptr, *masks = nullptr;
+    int count = 0;
+    SlipField slip;
+    double* scratch = nullptr;
+    double* out = nullptr;
+};
+constexpr int kMaxForceLists = 64;
+template <int N>
+struct ForceLists {
+    ForceList list[N];
+};
+size_t force_scratch_bytes(int count);
+cudaError_t launch_force(Storage s, const ForceList& list, cudaStream_t st);
+/// n lists without wall models in one launch, each with a scratch of its own.
+cudaError_t launch_forces(Storage s, const ForceLists<kMaxForceLists>& lists, int n, cudaStream_t st);
 
 // ---- wall model (wall_kernels.cu) ------------------------------------------
 struct WallListDev {
@@ -206,10 +218,11 @@ cudaError_t launch_batch_collide_f16(const BatchTable& tab, unsigned itemBase, u
 int batch_occupancy_f32(BatchShape sh);
 int batch_occupancy_f16(BatchShape sh);
 cudaError_t launch_force_append(const double* cur, int n3, double* hist, int cap, int* count, cudaStream_t st);
-/// Per-tunnel health: max speed over non-solid cells (float bits into
-/// *maxSpeedBits, which must start at 0) and non-finite cell count.
-cudaError_t launch_batch_health(bool fp32, const void* f, const std::uint8_t* kind, long long n, int* maxSpeedBits,
-                                int* nonFinite, cudaStream_t st);
+/// Per-tunnel health of the tunnels of a table: max speed over non-solid cells
+/// (float bits into maxSpeedBits[t], which must start at 0) and the count of
+/// non-finite cells.
+cudaError_t launch_batch_health(bool fp32, const BatchTable& tab, int parity, int* maxSpeedBits, int* nonFinite,
+                                cudaStream_t st);
 /// Set latch[t] (1 non-finite, 2 speed >= cap) of every running tunnel from
 /// its health scan (maxSpeedBits[t], nonFinite[t]), and latch[ntun + t] to the
 /// force-sample count *samples when it does.

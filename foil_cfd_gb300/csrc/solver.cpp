@@ -393,9 +393,8 @@ struct fcfd_solver {
         if (te != cudaSuccess) return te;
         L.nReadWrite = t.classes[0]; L.nInlet = t.classes[1]; L.nUntouched = t.classes[2];
         for (int k = 0; k < 4; ++k) L.solidBox[k] = t.box[k];
-        if (auto e = dalloc(&L.dPartials, static_cast<size_t>(force_blocks(L.linkCount)) * 3 * sizeof(double));
-            e != cudaSuccess)
-            return e;
+        if (auto e = dalloc(&L.dPartials, force_scratch_bytes(L.linkCount)); e != cudaSuccess) return e;
+        if (auto e = cudaMemsetAsync(L.dPartials, 0, force_scratch_bytes(L.linkCount), stream); e != cudaSuccess) return e;
         return cudaStreamSynchronize(stream);
     }
 
@@ -688,10 +687,13 @@ struct fcfd_solver {
         return e;
     }
 
-    cudaError_t forceReduce(Level& L) {
-        launches += 2;
-        return launch_force(storage, L.f[L.src], L.n, L.dLinkCells, L.dLinkMasks, L.linkCount,
-                            L.wm.slip(), L.dPartials, dForce, stream);
+    /// Force sample of a level into out[3], device memory or pinned host memory
+    /// (the stores of one thread; a copy between two kernels waits for the copy
+    /// engine and back, some 10 us).
+    cudaError_t forceReduce(Level& L, double* out) {
+        ++launches;
+        return launch_force(storage, ForceList{L.f[L.src], L.n, L.dLinkCells, L.dLinkMasks, L.linkCount, L.wm.slip(),
+                                               L.dPartials, out}, stream);
     }
 
     cudaError_t wallUpdate(Level& L, float nu) {
@@ -820,8 +822,7 @@ struct fcfd_solver {
         }
         if (!forcePending) {
             Level& L = (fineActive && forcesFromFine) ? fine : coarse;
-            if (forceReduce(L) == cudaSuccess) {
-                cudaMemcpyAsync(hForce, dForce, 3 * sizeof(double), cudaMemcpyDeviceToHost, stream);
+            if (forceReduce(L, hForce) == cudaSuccess) {
                 cudaEventRecord(evForce, stream);
                 forcePending = true;
                 stepsAtForceLaunch = steps;
@@ -1253,7 +1254,7 @@ int fcfd_force_now(fcfd_solver* s, double out[3]) {
     cudaStreamSynchronize(s->stream);
     s->pollAsync();
     Level& L = (s->fineActive && s->forcesFromFine) ? s->fine : s->coarse;
-    if (auto e = s->forceReduce(L); e != cudaSuccess) return e;
+    if (auto e = s->forceReduce(L, s->dForce); e != cudaSuccess) return e;
     double h[3];
     if (auto e = cudaMemcpyAsync(h, s->dForce, sizeof h, cudaMemcpyDeviceToHost, s->stream); e != cudaSuccess)
         return e;

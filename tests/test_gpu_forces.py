@@ -152,3 +152,39 @@ def test_lattice_view_and_device_flags(fc):
     assert vw.uwx and vw.uwy and vw.uwz
     with pytest.raises(fc.SolverError):
         s.lattice_view(2)   # no finer level
+
+
+@pytest.mark.parametrize("dims,solid", [((12, 9, 5), None), ((12, 9, 5), (1, 1, 1)), ((40, 9, 7), (29, 1, 1)),
+                                        ((40, 9, 7), (30, 2, 3)), ((96, 40, 24), (60, 20, 12))])
+def test_force_over_lists_of_every_length(fc, oracle_mod, dims, solid):
+    """No link, less than a block, a few and many blocks, against the FP64 sum
+    over all links; a population that is not finite shows in every component."""
+    nx, ny, nz = dims
+    flags = np.zeros((nz, ny, nx), np.uint8)
+    if solid:
+        a = [(n - k) // 2 for n, k in zip(dims, solid)]
+        flags[a[2]:a[2] + solid[2], a[1]:a[1] + solid[1], a[0]:a[0] + solid[0]] = 1
+    s = fc.LBMSolver()
+    s.init(dims, fc.scaling_direct(0.56, 0.05), flags.ravel())
+    rng = np.random.default_rng(1)
+    f = (0.05 + 0.01 * rng.random((19, nz, ny, nx))).astype(np.float32)
+    s.import_f32(f)
+    c = np.array([(0, 0, 0), (1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1), (1, 1, 0), (-1, -1, 0),
+                  (1, 0, 1), (-1, 0, -1), (0, 1, 1), (0, -1, -1), (1, -1, 0), (-1, 1, 0), (1, 0, -1), (-1, 0, 1),
+                  (0, 1, -1), (0, -1, 1)])
+    want, size, last = np.zeros(3), 1e-30, None
+    for q in range(1, 19):
+        link = (np.roll(flags, -c[q][::-1], (0, 1, 2)) == 1) & (flags == 0)
+        t = 2.0 * f[q][link].astype(np.float64)
+        want += c[q] * t.sum()
+        size += t.sum()
+        if link.any():
+            last = (q, *np.argwhere(link)[-1])
+    assert np.abs(s.force_now() - want).max() <= 1e-12 * size
+    if last:
+        f[last] = np.inf
+        s.import_f32(f)
+        assert not np.isfinite(s.force_now()).any()
+        f[last] = 0.05
+        s.import_f32(f)
+        assert np.isfinite(s.force_now()).all()
