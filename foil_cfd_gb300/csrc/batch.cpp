@@ -293,16 +293,13 @@ struct fcfd_batch {
     cudaError_t reset() {
         steps = 0;
         parity = 0;
-        for (Tunnel& x : t)
-            for (int i = 0; i < 2; ++i) {
-                launches += 2;
-                if (auto e = launch_init_equilibrium(storage, x.f[i], x.kind, x.d, x.uLat, stream); e != cudaSuccess)
-                    return e;
-                if (auto e = launch_speck(storage, x.f[i], x.kind, x.d, kSpeckAmplitudeFrac * x.uLat, kSpeckSeed,
-                                          stream);
-                    e != cudaSuccess)
-                    return e;
-            }
+        for (Tunnel& x : t) {
+            ++launches;
+            if (auto e = launch_reset(storage, x.f[0], x.f[1], x.kind, x.d, x.uLat, kSpeckAmplitudeFrac * x.uLat,
+                                      kSpeckSeed, stream);
+                e != cudaSuccess)
+                return e;
+        }
         if (auto e = cudaMemsetAsync(dHistCount, 0, sizeof(int), stream); e != cudaSuccess) return e;
         if (auto e = cudaMemsetAsync(dLatch, 0, 2 * ntun() * sizeof(int), stream); e != cudaSuccess) return e;
         return cudaStreamSynchronize(stream);

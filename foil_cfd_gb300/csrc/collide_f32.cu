@@ -18,17 +18,6 @@ namespace {
 
 constexpr int kBlock1D = 256;
 
-__global__ void init_eq_f32_kernel(float* __restrict__ f, const std::uint8_t* __restrict__ kind, long long n,
-                                   float uIn) {
-    const long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    const float ux = ((kind[c] & kFlagMask) == kSolid) ? 0.0f : uIn;
-    float feq[kQ];
-    eq19(1.0f, ux, 0.0f, 0.0f, feq);
-#pragma unroll
-    for (int q = 0; q < kQ; ++q) f[q * n + c] = feq[q];
-}
-
 __global__ void init_macro_f32_kernel(float* __restrict__ f, const std::uint8_t* __restrict__ kind,
                                       long long n, const float* __restrict__ rho, const float* __restrict__ u,
                                       const float* __restrict__ v, const float* __restrict__ w) {
@@ -66,11 +55,6 @@ cudaError_t launch_collide_child_f32(const float* src, float* dst, const std::ui
 cudaError_t launch_apply_flag_edits_f32(float* fA, float* fB, const std::uint8_t* flags, const std::uint8_t* mask,
                                         LevelDims d, cudaStream_t st) {
     return launch_apply_flag_edits_impl<StoreF32>(fA, fB, flags, mask, d, st);
-}
-
-cudaError_t launch_init_eq_f32(float* f, const std::uint8_t* kind, long long n, float uIn, cudaStream_t st) {
-    init_eq_f32_kernel<<<static_cast<unsigned>((n + kBlock1D - 1) / kBlock1D), kBlock1D, 0, st>>>(f, kind, n, uIn);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_init_macro_f32(float* f, const std::uint8_t* kind, long long n, const float* rho,

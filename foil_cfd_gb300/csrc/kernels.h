@@ -76,9 +76,8 @@ cudaError_t launch_collide(Storage s, const void* src, void* dst,
                            const std::uint8_t* kind, LevelDims d,
                            const CollideParams& p, float* rho, float* u,
                            float* v, float* w, SlipField slip, cudaStream_t st);
-cudaError_t launch_init_equilibrium(Storage s, void* f, const std::uint8_t* kind,
-                                    LevelDims d, float uInlet, cudaStream_t st);
-cudaError_t launch_speck(Storage s, void* f, const std::uint8_t* kind, LevelDims d,
+/// Cold start of a level's buffers (f2 may be null): inlet equilibrium and speck.
+cudaError_t launch_reset(Storage s, void* f, void* f2, const std::uint8_t* kind, LevelDims d, float uInlet,
                          float amplitude, unsigned seed, cudaStream_t st);
 cudaError_t launch_init_from_macro(Storage s, void* f, const std::uint8_t* kind,
                                    LevelDims d, const float* rho, const float* u,
@@ -125,8 +124,6 @@ cudaError_t launch_collide_aa_f32(float* f, LevelDims d, const CollideParams& p,
                                   float* v, float* w, cudaStream_t st);
 /// Whether the staged kernel serves a level (16-byte rows, >= 2 stages fit).
 bool staged_applies(LevelDims d, Storage s);
-cudaError_t launch_init_eq_f32(float* f, const std::uint8_t* kind, long long n, float uIn,
-                               cudaStream_t st);
 cudaError_t launch_collide_child_f32(const float* src, float* dst, const std::uint8_t* kind, LevelDims d,
                                      const CollideParams& p, SlipField slip, const ChildFuse& cf, cudaStream_t st);
 cudaError_t launch_init_macro_f32(float* f, const std::uint8_t* kind, long long n,

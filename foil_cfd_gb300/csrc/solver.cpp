@@ -855,12 +855,9 @@ struct fcfd_solver {
         cudaMemsetAsync(dNan, 0, sizeof(int), stream);
         cudaMemsetAsync(dStatus, 0, sizeof(int), stream);
         const float initU = rampEnabled ? 0.0f : scaling.u_lat;
-        for (int i = 0; i < (aa ? 1 : 2); ++i) {
-            launches += 2;
-            launch_init_equilibrium(storage, coarse.f[i], coarse.kind, coarse.d, initU, stream);
-            launch_speck(storage, coarse.f[i], coarse.kind, coarse.d, kSpeckAmplitudeFrac * scaling.u_lat,
-                         kSpeckSeed, stream);
-        }
+        ++launches;
+        launch_reset(storage, coarse.f[0], aa ? nullptr : coarse.f[1], coarse.kind, coarse.d, initU,
+                     kSpeckAmplitudeFrac * scaling.u_lat, kSpeckSeed, stream);
         aaNextOdd = 1;
         seedFine();
         seedFiner();
