@@ -160,7 +160,7 @@ __device__ __forceinline__ std::uint8_t voxel_flag(const FlagBuild& b, long long
 /// A thread has one (x, y) over a run of planes: only an input field (base 2)
 /// varies along z, all else is worked out once. Cell by cell the two 64-bit
 /// divisions and the tests of three cells took 182 instructions each: 41.7
-/// million cells 184 us.
+/// million cells 184 us, 32 by columns.
 constexpr int kFlagRun = 16;
 __global__ void __launch_bounds__(256)
 build_flags_kernel(FlagBuild b, std::uint8_t* __restrict__ out, int* __restrict__ closed) {
@@ -188,6 +188,25 @@ build_flags_kernel(FlagBuild b, std::uint8_t* __restrict__ out, int* __restrict_
     }
     count = __reduce_add_sync(0xffffffffu, count);
     if (count && (threadIdx.x & 31) == 0) atomicAdd(closed, count);
+}
+
+/// Flags of a new field, in place, to the edit mask against the kind bytes of
+/// the old one (1 newly solid, 2 newly fluid), four cells a thread, and the
+/// number of edits.
+__global__ void __launch_bounds__(256)
+flag_diff_kernel(const std::uint8_t* __restrict__ kind, std::uint8_t* __restrict__ mask, unsigned n,
+                 unsigned long long* __restrict__ count) {
+    const unsigned i = 4u * (blockIdx.x * 256u + threadIdx.x);
+    int edits = 0;
+    if (i < n) {   // both arrays go on to a multiple of four
+        const std::uint32_t was = __vcmpeq4(*reinterpret_cast<const std::uint32_t*>(kind + i) & 0x0f0f0f0fu, 0x01010101u * kSolidB);
+        std::uint32_t now = __vcmpeq4(*reinterpret_cast<const std::uint32_t*>(mask + i), 0x01010101u * kSolidB);
+        if (n - i < 4) now = (now & (0xffffffffu >> (32 - 8 * (n - i)))) | (was & ~(0xffffffffu >> (32 - 8 * (n - i))));
+        edits = __popc(was ^ now) / 8;
+        *reinterpret_cast<std::uint32_t*>(mask + i) = (now & ~was & 0x01010101u) | (was & ~now & 0x02020202u);
+    }
+    edits = __reduce_add_sync(0xffffffffu, edits);
+    if (edits && (threadIdx.x & 31) == 0) atomicAdd(count, static_cast<unsigned long long>(edits));
 }
 
 // ---- bit planes -----------------------------------------------------------------
@@ -795,9 +814,20 @@ struct CallScratch {
 
 constexpr unsigned bit(Plane p) { return 1u << p; }
 
+/// Entries to allocate for a list of n that a changed field makes anew: every
+/// allocation and release idles the device.
+constexpr long long spare(long long n) { return n + n / 8 + 1; }
+
 } // namespace
 
 // ---- host entry points ---------------------------------------------------------
+
+cudaError_t launch_flag_diff(const std::uint8_t* kind, std::uint8_t* mask, long long n, long long* count, cudaStream_t st) {
+    if (!kind || !mask || !count || n <= 0 || n >= (1LL << 31)) return cudaErrorInvalidValue;
+    flag_diff_kernel<<<static_cast<unsigned>((n + 1023) / 1024), 256, 0, st>>>(kind, mask, static_cast<unsigned>(n),
+                                                                              reinterpret_cast<unsigned long long*>(count));
+    return cudaGetLastError();
+}
 
 bool is_device_pointer(const void* p) {
     cudaPointerAttributes a{};
@@ -918,13 +948,19 @@ cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTabl
     t.classes[2] = n - t.classes[0] - t.classes[1];
     for (int k = 0; k < 4; ++k) t.box[k] = h.box[k];
     t.linkCount = h.total[0];
-    t.linkCells = t.linkMasks = nullptr;
-    const size_t bytes = static_cast<size_t>(t.linkCount > 0 ? t.linkCount : 1) * 4;
-    if (auto e = cudaMalloc(&t.linkCells, bytes); e != cudaSuccess) return e;
-    if (auto e = cudaMalloc(&t.linkMasks, bytes); e != cudaSuccess) {
+    if (!t.linkCells || t.linkCount > t.linkRoom) {
         cudaFree(t.linkCells);
-        t.linkCells = nullptr;
-        return e;
+        cudaFree(t.linkMasks);
+        t.linkCells = t.linkMasks = nullptr;
+        t.linkRoom = 0;
+        const long long room = spare(t.linkCount);
+        if (auto e = cudaMalloc(&t.linkCells, static_cast<size_t>(room) * 4); e != cudaSuccess) return e;
+        if (auto e = cudaMalloc(&t.linkMasks, static_cast<size_t>(room) * 4); e != cudaSuccess) {
+            cudaFree(t.linkCells);
+            t.linkCells = nullptr;
+            return e;
+        }
+        t.linkRoom = room;
     }
     if (t.linkCount > 0) {
         const unsigned m = static_cast<unsigned>(t.linkCount);
@@ -934,10 +970,9 @@ cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTabl
     return cudaGetLastError();
 }
 
-cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, std::uint32_t** cells, long long* count,
-                             GeomScratch& scratch, cudaStream_t st) {
-    if (d.cells() <= 0 || d.cells() >= (1LL << 31) || !flags || !cells || !count) return cudaErrorInvalidValue;
-    *cells = nullptr;
+cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, std::uint32_t** cells, long long* room,
+                             long long* count, GeomScratch& scratch, cudaStream_t st) {
+    if (d.cells() <= 0 || d.cells() >= (1LL << 31) || !flags || !cells || !room || !count) return cudaErrorInvalidValue;
     *count = 0;
     const BitGrid g = bit_grid(d);
     const unsigned wanted = full ? bit(kPInter) : bit(kPInter) | bit(kPFluid) | bit(kPOutlet);
@@ -950,7 +985,13 @@ cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, 
     else select_list<kSelShell>(ts, 0, g, st);
     Readback h;
     if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
-    if (auto e = cudaMalloc(cells, static_cast<size_t>(h.total[0] > 0 ? h.total[0] : 1) * 4); e != cudaSuccess) return e;
+    if (!*cells || h.total[0] > *room) {
+        cudaFree(*cells);
+        *cells = nullptr;
+        *room = 0;
+        if (auto e = cudaMalloc(cells, static_cast<size_t>(spare(h.total[0])) * 4); e != cudaSuccess) return e;
+        *room = spare(h.total[0]);
+    }
     *count = h.total[0];
     if (h.total[0] > 0) scatter_list(ts, 0, g, *cells, st);
     return cudaGetLastError();

@@ -297,17 +297,24 @@ struct LevelTables {
     std::uint32_t* tiles = nullptr;
     long long classes[3] = {0, 0, 0};   ///< cells read and written by a step / inlet / neither
     int box[4] = {0, 0, -1, -1};        ///< solid bounding box, as device_solid_bbox
+    /// The force list: given with room for linkRoom entries (null: none), and
+    /// replaced, with an eighth to spare, by a larger pair where that is short.
     std::uint32_t *linkCells = nullptr, *linkMasks = nullptr;
-    long long linkCount = 0;
+    long long linkRoom = 0, linkCount = 0;
 };
+/// The flags of a new field in `mask` become its edits against the field whose
+/// kind bytes are given: 1 newly solid, 2 newly fluid, 0 else; *count of them is
+/// added up. mask: 4-byte aligned, with room for a multiple of four.
+cudaError_t launch_flag_diff(const std::uint8_t* kind, std::uint8_t* mask, long long n, long long* count, cudaStream_t st);
 /// Synchronises once (the list's length); the tables are ready in stream order.
 cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTables& t, GeomScratch& scratch,
                                cudaStream_t st);
 /// Interface cells of a refined level, ascending: those with a fluid or outlet
 /// cell among their 18 neighbours (the ones a stream-collide reads), or with
-/// `full` every one. Allocated here; synchronises once.
-cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, std::uint32_t** cells, long long* count,
-                             GeomScratch& scratch, cudaStream_t st);
+/// `full` every one. *cells (null: none) has room for *room entries and is
+/// replaced where that is short; synchronises once.
+cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, std::uint32_t** cells, long long* room,
+                             long long* count, GeomScratch& scratch, cudaStream_t st);
 /// The wall-model list: find counts the entries (and synchronises), emit writes
 /// them, release gives the working memory back (stream-ordered).
 struct WallListBuild {

@@ -91,9 +91,37 @@ struct WMLevel {
         l.ys = dYs; l.linkMask = dMask; l.uTau = dUTau; l.count = count;
         return l;
     }
+    // All the arrays, in one block that a rebuild of the list uses again when
+    // it is large enough (twelve allocations and the device's idling for their
+    // releases took 0.5 ms of an edit of a 3 M-cell lattice).
+    char* block = nullptr;
+    size_t blockBytes = 0;
+
+    cudaError_t lay(size_t entries, size_t cells) {
+        const size_t e4 = (entries * 4 + 255) / 256 * 256, c2 = (cells * 2 + 255) / 256 * 256;
+        const size_t need = 8 * e4 + 3 * c2 + sizeof(WallStatsDev);
+        if (need > blockBytes) {
+            free();
+            if (auto e = dalloc(&block, need); e != cudaSuccess) { block = nullptr; return e; }
+            blockBytes = need;
+        }
+        char* at = block;
+        auto take = [&](auto** q, size_t bytes) { *q = reinterpret_cast<std::remove_reference_t<decltype(*q)>>(at); at += bytes; };
+        take(&dCell, e4); take(&dSample, e4); take(&dMask, e4);
+        take(&dNx, e4); take(&dNy, e4); take(&dNz, e4); take(&dYs, e4); take(&dUTau, e4);
+        take(&dUwx, c2); take(&dUwy, c2); take(&dUwz, c2);
+        take(&dStats, sizeof(WallStatsDev));
+        return cudaSuccess;
+    }
+    /// No list; the block stays.
+    void clear() {
+        WMLevel w;
+        w.block = block;
+        w.blockBytes = blockBytes;
+        *this = w;
+    }
     void free() {
-        dfree(dCell); dfree(dSample); dfree(dMask); dfree(dNx); dfree(dNy); dfree(dNz);
-        dfree(dYs); dfree(dUTau); dfree(dUwx); dfree(dUwy); dfree(dUwz); dfree(dStats);
+        dfree(block);
         *this = WMLevel{};
     }
 };
@@ -107,9 +135,11 @@ struct Level {
     uint2* links = nullptr;   // pull-link classes of the fluid cells (8 B per cell)
     std::uint32_t* tiles = nullptr;   // tile codes (a word per 128 cells)
     int src = 0;
-    std::vector<std::uint8_t> hostFlags, surfaceRef;
+    std::vector<std::uint8_t> surfaceRef;
+    bool flagsSet = false;   // flags, kind, ... hold a field
     std::uint32_t *dLinkCells = nullptr, *dLinkMasks = nullptr;
     int linkCount = 0;
+    long long linkRoom = 0;
     double* dPartials = nullptr;
     WMLevel wm;
     // Interpolated bounce-back link field (null when the level has none).
@@ -135,8 +165,8 @@ struct Level {
         dfree(dQFrac); dfree(dFFMask);
         qLinks = qFallback = 0;
         wm.free();
-        hostFlags.clear(); surfaceRef.clear();
-        linkCount = 0; src = 0; n = 0; d = LevelDims{};
+        flagsSet = false; surfaceRef.clear();
+        linkCount = 0; linkRoom = 0; src = 0; n = 0; d = LevelDims{};
     }
 };
 
@@ -231,11 +261,13 @@ struct fcfd_solver {
     int finerFactor = 2;
     fcfd_patch_box finerBox{};
     std::uint32_t* dShellFiner = nullptr;
+    long long shellRoomFiner = 0;
     int shellCountFiner = 0;
-    std::uint64_t flagsHashCache = 0;   // FNV-1a of coarse.hostFlags
+    std::uint64_t flagsHashCache = 0;   // FNV-1a of coarse.flags
     bool flagsHashValid = false;
     float* dScratchFiner = nullptr;
     std::uint32_t* dShell = nullptr;
+    long long shellRoom = 0;
     int shellCount = 0;
     // The fine level's fill covers every interface cell while a finer box
     // reaches its outer shell layer (the finer fill gathers from there).
@@ -362,39 +394,39 @@ struct fcfd_solver {
         return cudaSuccess;
     }
 
-    /// Flags of a level from host or device memory: the device copy, the
-    /// host copy (edit diffs), the cell classes, the kind bytes and the
-    /// force-link list, the last two built on the device.
+    /// Flags of a level from host or device memory: the device copy, the cell
+    /// classes, the kind bytes and the force-link list, built on the device.
     cudaError_t uploadLevelFlags(Level& L, const std::uint8_t* flags) {
         if (&L == &coarse) flagsHashValid = false;
-        L.hostFlags.resize(static_cast<size_t>(L.n));
-        const size_t nb = static_cast<size_t>(L.n);
-        if (on_device(flags)) {
-            if (auto e = cudaMemcpyAsync(L.flags, flags, nb, cudaMemcpyDeviceToDevice, stream); e != cudaSuccess)
-                return e;
-            if (auto e = cudaMemcpyAsync(L.hostFlags.data(), flags, nb, cudaMemcpyDeviceToHost, stream);
-                e != cudaSuccess)
-                return e;
-        } else {
-            std::memcpy(L.hostFlags.data(), flags, nb);
-            if (auto e = cudaMemcpyAsync(L.flags, flags, nb, cudaMemcpyHostToDevice, stream); e != cudaSuccess)
-                return e;
-        }
-        dfree(L.dLinkCells); dfree(L.dLinkMasks); dfree(L.dPartials);
+        if (auto e = cudaMemcpyAsync(L.flags, flags, static_cast<size_t>(L.n),
+                                     on_device(flags) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream);
+            e != cudaSuccess)
+            return e;
+        L.flagsSet = true;
         LevelTables t;
         t.kind = L.kind;
         t.links = L.links;
         t.tiles = L.tiles;
+        t.linkCells = L.dLinkCells;
+        t.linkMasks = L.dLinkMasks;
+        t.linkRoom = L.linkRoom;
+        L.linkCount = 0;
         launches += 8;
         const cudaError_t te = build_level_tables(L.d, L.flags, t, geomScratch, stream);
         L.dLinkCells = t.linkCells;
         L.dLinkMasks = t.linkMasks;
-        L.linkCount = static_cast<int>(t.linkCount);
+        const bool grown = t.linkRoom != L.linkRoom;
+        L.linkRoom = t.linkRoom;
         if (te != cudaSuccess) return te;
+        L.linkCount = static_cast<int>(t.linkCount);
         L.nReadWrite = t.classes[0]; L.nInlet = t.classes[1]; L.nUntouched = t.classes[2];
         for (int k = 0; k < 4; ++k) L.solidBox[k] = t.box[k];
-        if (auto e = dalloc(&L.dPartials, force_scratch_bytes(L.linkCount)); e != cudaSuccess) return e;
-        if (auto e = cudaMemsetAsync(L.dPartials, 0, force_scratch_bytes(L.linkCount), stream); e != cudaSuccess) return e;
+        if (grown || !L.dPartials) {
+            const size_t bytes = force_scratch_bytes(static_cast<int>(L.linkRoom));
+            dfree(L.dPartials);
+            if (auto e = dalloc(&L.dPartials, bytes); e != cudaSuccess) return e;
+            if (auto e = cudaMemsetAsync(L.dPartials, 0, bytes, stream); e != cudaSuccess) return e;
+        }
         return cudaStreamSynchronize(stream);
     }
 
@@ -405,19 +437,21 @@ struct fcfd_solver {
     /// every population a step computes is the same. With `full` (the fine
     /// level while a finer level nests in it, whose fill may gather from
     /// the fine shell) every interface cell.
-    cudaError_t shellList(const Level& L, bool full, std::uint32_t** out, int* count) {
-        dfree(*out);
+    cudaError_t shellList(const Level& L, bool full, std::uint32_t** out, long long* room, int* count) {
         *count = 0;
         long long c = 0;
         launches += 4;
-        const cudaError_t e = build_shell_list(L.d, L.flags, full, out, &c, geomScratch, stream);
+        const cudaError_t e = build_shell_list(L.d, L.flags, full, out, room, &c, geomScratch, stream);
         *count = static_cast<int>(c);
         return e;
     }
 
     cudaError_t buildWM(Level& L, int sampleCells) {
-        L.wm.free();
-        if (!wmEnabled || L.hostFlags.size() != static_cast<size_t>(L.n)) return cudaSuccess;
+        L.wm.clear();
+        if (!wmEnabled || !L.flagsSet) {
+            L.wm.free();
+            return cudaSuccess;
+        }
         const size_t cells = static_cast<size_t>(L.n);
         // Normals key off the clean surface reference when one is set.
         std::uint8_t* dClean = nullptr;
@@ -439,12 +473,8 @@ struct fcfd_solver {
             return e;
         }
         WMLevel& m = L.wm;
-        auto A = [&](auto** p, size_t b) { if (e == cudaSuccess) e = dalloc(p, b); };
         const size_t nn = static_cast<size_t>(n);
-        A(&m.dCell, nn * 4); A(&m.dSample, nn * 4); A(&m.dMask, nn * 4);
-        A(&m.dNx, nn * 4); A(&m.dNy, nn * 4); A(&m.dNz, nn * 4); A(&m.dYs, nn * 4); A(&m.dUTau, nn * 4);
-        A(&m.dUwx, cells * 2); A(&m.dUwy, cells * 2); A(&m.dUwz, cells * 2);
-        A(&m.dStats, sizeof(WallStatsDev));
+        e = m.lay(nn, cells);
         if (e == cudaSuccess) {
             WallListOut o;
             o.cell = m.dCell; o.sample = m.dSample; o.mask = m.dMask;
@@ -505,6 +535,7 @@ struct fcfd_solver {
     void freeFiner() {
         finer.free_all();
         dfree(dShellFiner); dfree(dScratchFiner);
+        shellRoomFiner = 0;
         shellCountFiner = 0;
         finerActive = false;
     }
@@ -532,6 +563,7 @@ struct fcfd_solver {
         freeFiner();  // the finer level nests in the fine one
         fine.free_all();
         dfree(dShell); dfree(dScratch);
+        shellRoom = 0;
         shellCount = 0;
         fineShellFull = false;
         fineActive = false;
@@ -1089,36 +1121,30 @@ int fcfd_apply_edited_flags(fcfd_solver* s, const uint8_t* flags, size_t n, long
     if (!s || !s->initialized || !flags || n != static_cast<size_t>(s->coarse.n)) return cudaErrorInvalidValue;
     if (s->aa && !aa_flags_ok(flags, n)) return cudaErrorNotSupported;
     Level& L = s->coarse;
-    std::vector<std::uint8_t> hostNew;
-    const std::uint8_t* nf = flags;
-    if (on_device(flags)) {
-        assign_flags(hostNew, flags, n);
-        nf = hostNew.data();
-    }
-    // Diff before the host copy is replaced: 1 newly solid, 2 newly fluid.
-    std::vector<std::uint8_t> mask(static_cast<size_t>(L.n), 0);
+    // The edit mask (1 newly solid, 2 newly fluid), from the kind bytes of the
+    // field that is replaced; its count arrives with the tables below. On the
+    // host the field's copies and the comparison took 2 ms at 3 M cells.
+    const size_t cells = static_cast<size_t>(L.n), tail = (cells + 15) / 16 * 16;
+    char* work = nullptr;
+    if (auto e = cudaMallocAsync(reinterpret_cast<void**>(&work), tail + sizeof(long long), s->stream); e != cudaSuccess)
+        return e;
+    auto* mask = reinterpret_cast<std::uint8_t*>(work);
+    auto* dCount = reinterpret_cast<long long*>(work + tail);
     long long count = 0;
-    for (long long i = 0; i < L.n; ++i) {
-        const bool was = L.hostFlags[static_cast<size_t>(i)] == FCFD_FLAG_SOLID;
-        const bool now = nf[i] == FCFD_FLAG_SOLID;
-        if (was == now) continue;
-        mask[static_cast<size_t>(i)] = now ? 1 : 2;
-        ++count;
+    cudaError_t e = cudaMemcpyAsync(mask, flags, cells, on_device(flags) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                                    s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(dCount, 0, sizeof(long long), s->stream);
+    if (e == cudaSuccess) e = launch_flag_diff(L.kind, mask, L.n, dCount, s->stream);
+    ++s->launches;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&count, dCount, sizeof count, cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = s->uploadLevelFlags(L, flags);   // waits for the stream
+    if (e == cudaSuccess && count > 0) {
+        ++s->launches;
+        e = launch_apply_flag_edits(s->storage, L.f[L.src], L.f[1 - L.src], L.flags, mask, L.d, s->stream);
     }
-    if (auto e = s->uploadLevelFlags(L, flags); e != cudaSuccess) return e;
-    if (count > 0) {
-        std::uint8_t* dMaskBuf = nullptr;
-        if (auto e = cudaMalloc(&dMaskBuf, static_cast<size_t>(L.n)); e != cudaSuccess) return e;
-        cudaError_t e = cudaMemcpyAsync(dMaskBuf, mask.data(), static_cast<size_t>(L.n), cudaMemcpyHostToDevice,
-                                        s->stream);
-        if (e == cudaSuccess) {
-            ++s->launches;
-            e = launch_apply_flag_edits(s->storage, L.f[L.src], L.f[1 - L.src], L.flags, dMaskBuf, L.d, s->stream);
-        }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-        cudaFree(dMaskBuf);
-        if (e != cudaSuccess) return e;
-    }
+    cudaFreeAsync(work, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) return e;
     s->updateForcesFromFine();
     if (auto e = s->buildWM(L, kWallSampleCoarse); e != cudaSuccess) return e;
     s->rampActive = false;
@@ -1538,7 +1564,7 @@ int fcfd_init_refinement(fcfd_solver* s, const fcfd_patch_box* box, int factor, 
     };
     if (auto e = s->allocLevel(s->fine, fd); e != cudaSuccess) return fail("fine buffer allocation failed", e);
     if (auto e = s->uploadLevelFlags(s->fine, ff); e != cudaSuccess) return fail("fine flag upload failed", e);
-    if (auto e = s->shellList(s->fine, false, &s->dShell, &s->shellCount); e != cudaSuccess)
+    if (auto e = s->shellList(s->fine, false, &s->dShell, &s->shellRoom, &s->shellCount); e != cudaSuccess)
         return fail("shell list failed", e);
     s->fineActive = true;
     const long long sf = restrict_scratch_floats(s->geom());
@@ -1566,7 +1592,7 @@ int fcfd_set_refined_flags(fcfd_solver* s, const uint8_t* ff, size_t n) {
     if (!s || !s->initialized || !s->fineActive || !ff || n != static_cast<size_t>(s->fine.n))
         return cudaErrorInvalidValue;
     if (auto e = s->uploadLevelFlags(s->fine, ff); e != cudaSuccess) return e;
-    if (auto e = s->shellList(s->fine, s->fineShellFull, &s->dShell, &s->shellCount); e != cudaSuccess) return e;
+    if (auto e = s->shellList(s->fine, s->fineShellFull, &s->dShell, &s->shellRoom, &s->shellCount); e != cudaSuccess) return e;
     s->updateForcesFromFine();
     if (auto e = s->buildWM(s->fine, kWallSampleFine); e != cudaSuccess) return e;
     if (auto e = s->seedFine(); e != cudaSuccess) return e;
@@ -1849,7 +1875,7 @@ int fcfd_q_link_info(fcfd_solver* s, int level, int* active, int* links, int* fa
 
 /// Interface-shell and seed lists of the finer level (its flags uploaded).
 static int finer_lists(fcfd_solver* s) {
-    return s->shellList(s->finer, false, &s->dShellFiner, &s->shellCountFiner);
+    return s->shellList(s->finer, false, &s->dShellFiner, &s->shellRoomFiner, &s->shellCountFiner);
 }
 
 int fcfd_init_finer_refinement(fcfd_solver* s, const fcfd_patch_box* box, int factor, const uint8_t* ff,
@@ -1904,7 +1930,7 @@ int fcfd_init_finer_refinement(fcfd_solver* s, const fcfd_patch_box* box, int fa
     // the fine shell's outer layer: fill every fine interface cell from now on.
     if (box->x0 < 2 || box->y0 < 2 || box->x1 > pd.nx - 2 || box->y1 > pd.ny - 2) {
         s->fineShellFull = true;
-        if (auto e = s->shellList(s->fine, true, &s->dShell, &s->shellCount); e != cudaSuccess)
+        if (auto e = s->shellList(s->fine, true, &s->dShell, &s->shellRoom, &s->shellCount); e != cudaSuccess)
             return fail("shell list failed", e);
     }
     const long long sf = restrict_scratch_floats(s->geomFiner());
@@ -1927,7 +1953,7 @@ void fcfd_shutdown_finer_refinement(fcfd_solver* s) {
     s->freeFiner();
     if (s->fineShellFull && s->fineActive) {
         s->fineShellFull = false;
-        s->shellList(s->fine, false, &s->dShell, &s->shellCount);
+        s->shellList(s->fine, false, &s->dShell, &s->shellRoom, &s->shellCount);
     }
 }
 
@@ -1999,7 +2025,10 @@ int fcfd::solver_field_view(fcfd_solver* s, SolverFieldView* v) {
     v->stream = s->stream;
     // The flag hash is cached until the coarse flags change.
     if (!s->flagsHashValid) {
-        s->flagsHashCache = fnv1a64(s->coarse.hostFlags.data(), s->coarse.hostFlags.size());
+        std::vector<std::uint8_t> h(s->coarse.flagsSet ? static_cast<size_t>(s->coarse.n) : 0);
+        if (!h.empty())
+            if (auto e = cudaMemcpy(h.data(), s->coarse.flags, h.size(), cudaMemcpyDeviceToHost); e != cudaSuccess) return e;
+        s->flagsHashCache = fnv1a64(h.data(), h.size());
         s->flagsHashValid = true;
     }
     v->flagsHash = s->flagsHashCache;

@@ -20,7 +20,7 @@ constexpr int kBlock1D = 256;
 /// lbm_core.cu:130-160), 3 w_q c_z w'(x, z) on the fluid cells' populations,
 /// added to the value as stored. Two launches per buffer, the second over what
 /// the first had written, moved 3 x these bytes: 23.6 million cells FP32
-/// 1.10 ms, 0.56 ms in one pass over both.
+/// 1.10 ms, 0.50 ms in one pass over both.
 template <class S>
 __global__ void __launch_bounds__(kBlock1D)
 reset_kernel(typename S::T* __restrict__ f, typename S::T* __restrict__ f2, const std::uint8_t* __restrict__ kind,

@@ -42,3 +42,33 @@ def test_seeding(fc, oracle_mod, dims, box, factor):
     o.enable_refinement([x0, y0, x1, y1], factor, fine.ravel())
     keep = fine.ravel() != 1
     assert np.array_equal(s.export_fine_f32().reshape(19, -1)[:, keep], o.fine["f"].reshape(19, -1)[:, keep])
+
+
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("dims", [(5, 5, 1), (7, 5, 3), (13, 7, 2), (33, 17, 8), (40, 31, 9)])
+def test_edits_of_odd_cell_counts(fc, oracle_mod, dims, device):
+    """Cell counts with every remainder of four, edits in the first and the last
+    cell, from host and device memory (also at an odd address), back and forth."""
+    torch = pytest.importorskip("torch")
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n)
+    a = (rng.random(n) < 0.1).astype(np.uint8)
+    b = (rng.random(n) < 0.1).astype(np.uint8)
+    b[0], b[-1] = 1 - a[0], 1 - a[-1]
+    s = fc.LBMSolver()
+    s.init(dims, fc.scaling_direct(0.55, 0.05), a, les_cs=0.1)
+    f = oracle_mod.equilibrium(np.ones(n), np.full(n, 0.03), np.zeros(n), np.zeros(n))
+    s.import_f32(f)
+    s.mirror_buffers()
+    state, old = f.reshape(19, n).astype(np.float32).copy(), a
+    for new in (b, b, a):
+        arg = new
+        if device:
+            t = torch.zeros(n + 1, dtype=torch.uint8, device="cuda")
+            t[1:] = torch.from_numpy(new)
+            arg = t[1:]
+        assert s.apply_edited_flags(arg) == int(((old == 1) != (new == 1)).sum())
+        mask = np.where((new == 1) & (old != 1), 1, np.where((old == 1) & (new != 1), 2, 0))
+        oracle_mod.apply_flag_edits(dims, state, state.copy(), new, mask)
+        assert np.array_equal(s.export_f32().reshape(19, n), state)
+        old = new
