@@ -73,10 +73,11 @@ def test_aa_equals_ab_bitwise(fc, oracle_mod, storage, dims):
 
 
 @pytest.mark.parametrize("storage", ["fp32", "fp16"])
-@pytest.mark.parametrize("dims", [(3, 3, 1), (5, 3, 2), (127, 5, 4), (128, 5, 4), (129, 6, 3), (384, 4, 3)])
+@pytest.mark.parametrize("dims", [(3, 3, 1), (5, 3, 2), (127, 5, 4), (128, 5, 4), (129, 6, 3), (384, 4, 3), (129, 160, 125)])
 def test_aa_blocks_of_rows_and_of_the_flat_lattice(fc, oracle_mod, storage, dims):
     """Rows of whole blocks run one kernel shape, all others the flat one:
-    lattices of less than a block, rows around a block, both phases read."""
+    lattices of less than a block, rows around a block, one past the size up to
+    which FP32 collides in packed pairs, both phases read."""
     ab, aa = _pair(fc, dims, storage)
     f0 = _state(oracle_mod, dims)
     ab.import_f32(f0)
