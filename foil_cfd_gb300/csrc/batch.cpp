@@ -467,8 +467,13 @@ int fcfd_batch_autotune(fcfd_batch* b, int trialSteps, fcfd_batch_config* chosen
     fcfd_batch_config bestCfg = b->cfg;
     for (const fcfd_batch_config& c : list) {
         if (auto e = fcfd_batch_set_config(b, &c); e != 0) return e;
-        // One untimed step (first-launch costs), then the timed trial.
+        // One untimed step (first-launch costs), and as many as keep the force
+        // sample out of the timed trial: it fell into every fifth one and took
+        // as long as two steps.
         if (auto e = b->stepN(1, false); e != cudaSuccess) return e;
+        if (const int left = b->forceEvery - static_cast<int>(b->steps % b->forceEvery);
+            left <= trialSteps && trialSteps < b->forceEvery)
+            if (auto e = b->stepN(left, false); e != cudaSuccess) return e;
         if (auto e = b->stepN(trialSteps, false); e != cudaSuccess) return e;
         const float ms = static_cast<float>(b->lastMs) / static_cast<float>(trialSteps);
         record(c, ms);
