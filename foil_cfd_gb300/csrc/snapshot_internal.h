@@ -1,5 +1,5 @@
 // What the snapshot code (snapshot.cpp) reads from a solver: the current
-// population buffer of every active level, its storage, the host copy of the
+// population buffer of every active level, its storage, the hash of the
 // coarse flags and the scaling.
 #pragma once
 

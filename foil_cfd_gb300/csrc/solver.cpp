@@ -1873,7 +1873,7 @@ int fcfd_q_link_info(fcfd_solver* s, int level, int* active, int* links, int* fa
 
 // ---- nested finer level (initFinerRefinement & co, lbm_solver.cpp:1916-2010)
 
-/// Interface-shell and seed lists of the finer level (its flags uploaded).
+/// Interface-shell list of the finer level (its flags uploaded).
 static int finer_lists(fcfd_solver* s) {
     return s->shellList(s->finer, false, &s->dShellFiner, &s->shellRoomFiner, &s->shellCountFiner);
 }

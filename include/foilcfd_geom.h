@@ -15,7 +15,7 @@
  * fcfd_apply_edited_flags, fcfd_init_refinement, fcfd_set_refined_flags,
  * fcfd_init_finer_refinement, fcfd_set_refined_finer_flags) accept a flag
  * field in device memory as well: the solver then copies it on the device and
- * builds its force-link, wall-model, shell and seed lists with these kernels.
+ * builds its force-link, wall-model and shell lists with these kernels.
  *
  * Return convention: 0 or a cudaError_t value. The list builders and the
  * patch box synchronise the stream before they return; the flag builder
