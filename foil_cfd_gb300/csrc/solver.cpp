@@ -101,7 +101,8 @@ struct WMLevel {
         const size_t e4 = (entries * 4 + 255) / 256 * 256, c2 = (cells * 2 + 255) / 256 * 256;
         const size_t need = 8 * e4 + 3 * c2 + sizeof(WallStatsDev);
         if (need > blockBytes) {
-            free();
+            dfree(block);   // the block only: the counts of this build are already noted
+            blockBytes = 0;
             if (auto e = dalloc(&block, need); e != cudaSuccess) { block = nullptr; return e; }
             blockBytes = need;
         }
