@@ -83,6 +83,8 @@ def test_counts_of_a_refined_level(fc):
         return g.ravel()
 
     fa, fcl = fine(active), fine(clean)
-    s.init_refinement(fc.Box(x0, y0, x1, y1), 2, fa)
+    s.init_refinement(fc.Box(x0, y0, x1, y1), 2, fa)      # first build, no reference yet
+    st = fc.build_wall_list(fd, fa, None, 3)["stats"]
+    assert st["degenerate"] > 0 and counts(s) == (1, 0, st["degenerate"])
     assert s.set_refined_surface_reference(fcl) == 0
     assert counts(s) == (1, *expected(fc, fd, fa, fcl, 3))
