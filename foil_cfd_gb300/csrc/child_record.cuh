@@ -30,7 +30,10 @@ __device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, 
 
 // Terms whose lattice coefficient is 0 are left out of the sums below, and
 // sums start from their first term: the same value for finite populations
-// (the sign of a zero aside).
+// (the sign of a zero aside). What such terms do for an infinity or a NaN,
+// which 0 times it passes on to every sum, is kept by one term 0 times the sum
+// of all: a bad population, the rest one too, spoils the whole cell, and so
+// travels on to where the watchdog looks.
 
 /// Moments of fi with the density floor and the |u| <= 0.3 limiter.
 __device__ __forceinline__ void limited_moments(const float (&fi)[kQ], float& rho, float& ux, float& uy,
@@ -43,6 +46,7 @@ __device__ __forceinline__ void limited_moments(const float (&fi)[kQ], float& rh
         if (cy(q) != 0 && q != 3) jy = cy(q) > 0 ? rn_add(jy, fi[q]) : rn_sub(jy, fi[q]);
         if (cz(q) != 0 && q != 5) jz = cz(q) > 0 ? rn_add(jz, fi[q]) : rn_sub(jz, fi[q]);
     }
+    jx = __fmaf_rn(0.0f, r, jx); jy = __fmaf_rn(0.0f, r, jy); jz = __fmaf_rn(0.0f, r, jz);
     r = fmaxf(r, kRhoFloor);
     const float inv = 1.0f / r;
     ux = rn_mul(jx, inv); uy = rn_mul(jy, inv); uz = rn_mul(jz, inv);

@@ -59,7 +59,8 @@ __device__ __forceinline__ void regularize(float (&fneq)[kQ]) {
         if (cx(q) * cz(q) != 0 && q != 9) pxz = cx(q) * cz(q) > 0 ? pxz + v : pxz - v;
         if (cy(q) * cz(q) != 0 && q != 11) pyz = cy(q) * cz(q) > 0 ? pyz + v : pyz - v;
     }
-    const float trace = (1.0f / 3.0f) * (pxx + pyy + pzz);
+    const float sum = pxx + pyy + pzz;   // has every population but the rest one
+    const float trace = __fmaf_rn(0.0f, sum + fneq[0], (1.0f / 3.0f) * sum);
     fneq[0] = 4.5f * wgt(0) * (0.0f - trace);
 #pragma unroll
     for (int p = 1; p <= 9; ++p) {   // c and -c project alike
@@ -383,6 +384,7 @@ restrict_kernel(typename S::T* __restrict__ fc, const std::uint8_t* __restrict__
             if (cy(q) != 0 && q != 3) bjy = cy(q) > 0 ? bjy + b[q] : bjy - b[q];
             if (cz(q) != 0 && q != 5) bjz = cz(q) > 0 ? bjz + b[q] : bjz - b[q];
         }
+        bjx = __fmaf_rn(0.0f, br, bjx); bjy = __fmaf_rn(0.0f, br, bjy); bjz = __fmaf_rn(0.0f, br, bjz);
         br = fmaxf(br, kRhoFloor);
         const float bi = 1.0f / br;
         mRho[cell] = br; mU[cell] = bjx * bi; mV[cell] = bjy * bi; mW[cell] = bjz * bi;
