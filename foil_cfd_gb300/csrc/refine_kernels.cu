@@ -46,7 +46,9 @@ constexpr int kRestrictBlend = 3;  // edge-blend ramp width (coarse cells)
 __device__ __forceinline__ int wrap1(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 
 /// Latt-Chopard projection of fneq onto the second-order Hermite space
-/// (zero-coefficient terms left out, as in child_record.cuh).
+/// (zero-coefficient terms left out, as in child_record.cuh; the rest part, all
+/// of whose coefficients are 0, is then not read: limited_moments has made every
+/// part of a cell with a bad population NaN).
 __device__ __forceinline__ void regularize(float (&fneq)[kQ]) {
     float pxx = fneq[1], pyy = fneq[3], pzz = fneq[5], pxy = fneq[7], pxz = fneq[9], pyz = fneq[11];
 #pragma unroll
@@ -59,8 +61,7 @@ __device__ __forceinline__ void regularize(float (&fneq)[kQ]) {
         if (cx(q) * cz(q) != 0 && q != 9) pxz = cx(q) * cz(q) > 0 ? pxz + v : pxz - v;
         if (cy(q) * cz(q) != 0 && q != 11) pyz = cy(q) * cz(q) > 0 ? pyz + v : pyz - v;
     }
-    const float sum = pxx + pyy + pzz;   // has every population but the rest one
-    const float trace = __fmaf_rn(0.0f, sum + fneq[0], (1.0f / 3.0f) * sum);
+    const float trace = (1.0f / 3.0f) * (pxx + pyy + pzz);
     fneq[0] = 4.5f * wgt(0) * (0.0f - trace);
 #pragma unroll
     for (int p = 1; p <= 9; ++p) {   // c and -c project alike
