@@ -23,7 +23,7 @@ void batch_offsets(BatchTunnelParam& p) {
 /// force samples and advance its device-side count.
 __global__ void force_append_kernel(const double* __restrict__ cur, int n3, double* __restrict__ hist, int cap,
                                     int* __restrict__ count) {
-    pdl_wait();
+    pdl_wait(cur, count);
     const int c = *count;
     double* slot = hist + static_cast<long long>(c % cap) * n3;
     for (int i = threadIdx.x; i < n3; i += blockDim.x) slot[i] = cur[i];
@@ -87,7 +87,7 @@ cudaError_t launch_batch_health(bool fp32, const BatchTable& tab, int parity, in
 /// + t] records the force-sample count at that moment.
 __global__ void batch_latch_kernel(const int* __restrict__ maxSpeedBits, const int* __restrict__ nonFinite, int ntun,
                                    float cap, const int* __restrict__ samples, int* __restrict__ latch) {
-    pdl_wait();
+    pdl_wait(maxSpeedBits, nonFinite, samples);
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntun || latch[t] != 0) return;
     const int v = nonFinite[t] > 0 ? 1 : (__int_as_float(maxSpeedBits[t]) >= cap ? 2 : 0);

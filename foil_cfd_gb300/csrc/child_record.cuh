@@ -96,6 +96,19 @@ struct RecordGrid {
     __host__ __device__ long long count(int nz) const { return static_cast<long long>(w + 2) * (h + 2) * nz; }
 };
 
+/// Parts of a record, which the launch before wrote: ordinary loads, free to be
+/// scheduled (the kernel had t back from its wait).
+__device__ __forceinline__ float4 ld_rec(const float4* p) {
+    float4 v;
+    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_rec(const uint4* p) {
+    uint4 v;
+    asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 /// The planes of the scratch (four or six of them), float4 k of record t at p[k][t].
 struct RecordPlanes {
     const float4* p[kScratchVals / 4];
@@ -139,7 +152,7 @@ template <> struct ChildRecord<StoreF32> {
     __device__ __forceinline__ static void add(const RecordPlanes& r, unsigned t, float (&acc)[kQ], float& count) {
         float4 a[5];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) a[k] = __ldg(r.p[k] + t);
+        for (int k = 0; k < 5; ++k) a[k] = ld_rec(r.p[k] + t);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
             const float v[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
@@ -152,7 +165,7 @@ template <> struct ChildRecord<StoreF32> {
         }
     }
     __device__ __forceinline__ static float4 moments(const RecordPlanes& r, unsigned t) {
-        return __ldg(r.p[kScratchRho / 4] + t);
+        return ld_rec(r.p[kScratchRho / 4] + t);
     }
 };
 
@@ -187,7 +200,7 @@ template <> struct ChildRecord<StoreF16> {
     __device__ __forceinline__ static void add(const RecordPlanes& r, unsigned t, float (&acc)[kQ], float& count) {
         uint4 c[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) c[k] = __ldg(reinterpret_cast<const uint4*>(r.p[k]) + t);
+        for (int k = 0; k < 3; ++k) c[k] = ld_rec(reinterpret_cast<const uint4*>(r.p[k]) + t);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const unsigned w[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
@@ -202,7 +215,7 @@ template <> struct ChildRecord<StoreF16> {
         }
         count = SET ? __uint_as_float(c[2].z) : count + __uint_as_float(c[2].z);
     }
-    __device__ __forceinline__ static float4 moments(const RecordPlanes& r, unsigned t) { return __ldg(r.p[3] + t); }
+    __device__ __forceinline__ static float4 moments(const RecordPlanes& r, unsigned t) { return ld_rec(r.p[3] + t); }
 };
 
 /// Record of a coarse cell from the sum fi of its nFluid fluid children

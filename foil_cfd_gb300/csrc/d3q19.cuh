@@ -116,18 +116,37 @@ __device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv& f) {
 // widened to FP32 on load (deviation storage keeps the O(1) weight out of the
 // 11-bit mantissa). All arithmetic is FP32 in both cases.
 //
-// Population loads go through the read-only path with a 256-byte L2
-// prefetch hint: a warp's pull along a direction slice reads one or two
-// 128-byte lines, and the next warp of the row reads the lines after them
-// (measured 0.7 % faster on the FP32 collide launch than plain __ldg).
+// Population loads carry a 256-byte L2 prefetch hint: a warp's pull along a
+// direction slice reads one or two 128-byte lines, and the next warp of the
+// row reads the lines after them (measured 0.7 % faster on the FP32 collide
+// launch than plain __ldg).
+//
+// Most kernels read what the launch before theirs wrote, after a wait
+// (pdl.cuh), so the load is an ordinary one, not one of the read-only path, and
+// must not move up past the wait. In the collides both cost nothing (768x320x96
+// tunnel 5.48 ms per 10 steps either way); in the fill, the seeding and the
+// restriction volatile loads cost 4-8 % of a refined step, as did the
+// restriction's own cells by ordinary loads, which its stores hold back
+// (640-cell tunnel 30.7 -> 32.6 ms per 10 steps).
+enum Read {
+    kOrdered,   ///< volatile: stays behind the wait, whatever its address
+    kIndexed,   ///< free to be scheduled: the kernel had its indices back from the wait
+    kEarlier    ///< also past stores and the wait: what it reads was written before the launch before this one
+};
+template <int R>
 __device__ __forceinline__ float ld_pf(const float* p) {
     float v;
-    asm("ld.global.nc.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    if constexpr (R == kOrdered) asm volatile("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    else if constexpr (R == kIndexed) asm("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    else asm("ld.global.nc.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
+template <int R>
 __device__ __forceinline__ float ld_pf(const __half* p) {
     unsigned short h;
-    asm("ld.global.nc.L2::256B.b16 %0, [%1];" : "=h"(h) : "l"(p));
+    if constexpr (R == kOrdered) asm volatile("ld.global.L2::256B.b16 %0, [%1];" : "=h"(h) : "l"(p));
+    else if constexpr (R == kIndexed) asm("ld.global.L2::256B.b16 %0, [%1];" : "=h"(h) : "l"(p));
+    else asm("ld.global.nc.L2::256B.b16 %0, [%1];" : "=h"(h) : "l"(p));
     return __half2float(__ushort_as_half(h));
 }
 struct StoreF32 {
@@ -156,8 +175,9 @@ struct StoreF32 {
     /// which spill 108 B).
     static constexpr int kChildMinBlocks = 8;
     /// Load population q (weight w_q) at element i of its direction slice.
+    template <int R = kOrdered>
     __device__ __forceinline__ static float ld(const T* __restrict__ p, long long i, float) {
-        return ld_pf(p + i);
+        return ld_pf<R>(p + i);
     }
     __device__ __forceinline__ static void st(T* __restrict__ p, long long i, float v, float) {
         p[i] = v;
@@ -171,8 +191,9 @@ struct StoreF32 {
         return v;
     }
     /// Deviation forms g = f - w_q of ld / st / lds.
+    template <int R = kOrdered>
     __device__ __forceinline__ static float ld_dev(const T* __restrict__ p, long long i, float w) {
-        return ld_pf(p + i) - w;
+        return ld_pf<R>(p + i) - w;
     }
     __device__ __forceinline__ static void st_dev(T* __restrict__ p, long long i, float g, float w) {
         p[i] = g + w;
@@ -197,8 +218,9 @@ struct StoreF16 {
     static constexpr long long kCodedCells = 4000000;
     static constexpr int kBatchThreads = 1024;
     static constexpr int kChildMinBlocks = 8;
+    template <int R = kOrdered>
     __device__ __forceinline__ static float ld(const T* __restrict__ p, long long i, float w) {
-        return w + ld_pf(p + i);
+        return w + ld_pf<R>(p + i);
     }
     __device__ __forceinline__ static void st(T* __restrict__ p, long long i, float v, float w) {
         p[i] = __float2half_rn(v - w);
@@ -208,8 +230,9 @@ struct StoreF16 {
         return w + lds_dev(row, i, w);
     }
     /// The stored deviation itself: no weight add on load or subtract on store.
+    template <int R = kOrdered>
     __device__ __forceinline__ static float ld_dev(const T* __restrict__ p, long long i, float) {
-        return ld_pf(p + i);
+        return ld_pf<R>(p + i);
     }
     __device__ __forceinline__ static void st_dev(T* __restrict__ p, long long i, float g, float) {
         p[i] = __float2half_rn(g);

@@ -1,8 +1,8 @@
 // Programmatic dependent launch of the step's kernels. A kernel launched this
 // way is set up while its predecessor in the stream still runs, and its
 // blocks wait in pdl_wait() until that one has completed and its writes are
-// visible; pdl_wait() is the first statement of every kernel so launched, so
-// no memory is touched earlier and the order of the stream's work is kept
+// visible; every kernel so launched calls pdl_wait() before it touches memory
+// that an earlier launch writes, and the order of the stream's work is kept
 // (after a copy, a memset or an event the launch is an ordinary one).
 //
 // Back-to-back ordinary launches on a GB300 complete on a grid of about
@@ -17,7 +17,24 @@
 
 namespace fcfd {
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class V>
+__device__ __forceinline__ void after_wait(V& v) {
+    if constexpr (sizeof(V) == 8) asm volatile("" : "+l"(v)::"memory");
+    else asm volatile("" : "+r"(v)::"memory");
+}
+
+/// The wait. Volatile loads and those through pointers that may alias stay
+/// behind it by its memory clobber. A load that is to the compiler a function
+/// of its address alone does not: through a const restrict pointer, __ldg, or
+/// an assembler statement that is not volatile. A kernel that reads what
+/// earlier launches wrote in such a way hands the indices or pointers over from
+/// which the addresses are formed; they come back as values that the compiler
+/// cannot have had before.
+template <class... V>
+__device__ __forceinline__ void pdl_wait(V&... v) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    (after_wait(v), ...);
+}
 
 template <class... P, class... A>
 cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {

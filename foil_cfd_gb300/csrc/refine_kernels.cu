@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(kRefineBlock)
 fill_kernel(const __grid_constant__ FillPtrs<typename S::T> fp, const std::uint8_t* __restrict__ ckind,
             const std::uint32_t* __restrict__ targets, unsigned count, RefineGeom g, float invFactor, float tw,
             float neqScale, FastDiv divX, FastDiv divXY) {
-    pdl_wait();
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(i);
     if (i >= count) return;
     const std::uint32_t t = targets[i];
     const unsigned zu = fdiv(t, divXY);
@@ -173,11 +173,11 @@ fill_kernel(const __grid_constant__ FillPtrs<typename S::T> fp, const std::uint8
         for (int c = 0; c < 8; ++c) {
             const unsigned e = row[c >> 1];
             if constexpr (kDev) {
-                s0 += w8[c] * S::ld_dev(fp.t0[q] + e, c & 1, wgt(q));
-                if constexpr (BLEND) s1 += w8[c] * S::ld_dev(fp.t1[q] + e, c & 1, wgt(q));
+                s0 += w8[c] * S::template ld_dev<kIndexed>(fp.t0[q] + e, c & 1, wgt(q));
+                if constexpr (BLEND) s1 += w8[c] * S::template ld_dev<kIndexed>(fp.t1[q] + e, c & 1, wgt(q));
             } else {
-                s0 += w8[c] * S::ld(fp.t0[q] + e, c & 1, wgt(q));
-                if constexpr (BLEND) s1 += w8[c] * S::ld(fp.t1[q] + e, c & 1, wgt(q));
+                s0 += w8[c] * S::template ld<kIndexed>(fp.t0[q] + e, c & 1, wgt(q));
+                if constexpr (BLEND) s1 += w8[c] * S::template ld<kIndexed>(fp.t1[q] + e, c & 1, wgt(q));
             }
         }
         if constexpr (kDev) {
@@ -187,7 +187,7 @@ fill_kernel(const __grid_constant__ FillPtrs<typename S::T> fp, const std::uint8
         } else {
             if (s0 == 0.0f) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c) s1 += w8[c] * S::ld(fp.t1[q] + row[c >> 1], c & 1, wgt(q));
+                for (int c = 0; c < 8; ++c) s1 += w8[c] * S::template ld<kIndexed>(fp.t1[q] + row[c >> 1], c & 1, wgt(q));
                 s0 = s0 + tw * (s1 - s0);
             }
             fi[q] = s0;
@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(kRefineBlock, G == 2 ? 6 : 10)
 seed_kernel(const __grid_constant__ FillPtrs<typename S::T> fp, const std::uint8_t* __restrict__ ckind,
             const std::uint8_t* __restrict__ fkind, unsigned count, RefineGeom g, float invFactor, float neqScale,
             FastDiv divX, FastDiv divXY, long long twin) {
-    pdl_wait();
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(i);
     if (i >= count) return;
     const unsigned zu = fdiv(i, divXY);
     const unsigned rem = i - zu * divXY.d;
@@ -265,7 +265,7 @@ seed_kernel(const __grid_constant__ FillPtrs<typename S::T> fp, const std::uint8
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const auto* p = fp.t0[q] + row[c >> 1];
-            v[c] = kDev ? S::ld_dev(p, c & 1, wgt(q)) : S::ld(p, c & 1, wgt(q));
+            v[c] = kDev ? S::template ld_dev<kIndexed>(p, c & 1, wgt(q)) : S::template ld<kIndexed>(p, c & 1, wgt(q));
         }
 #pragma unroll
         for (int k = 0; k < G; ++k) {
@@ -294,8 +294,8 @@ template <class S>
 __global__ void __launch_bounds__(kRefineBlock)
 child_avg_kernel(const typename S::T* __restrict__ ff, const std::uint8_t* __restrict__ fkind,
                  RefineGeom g, int rx0, int ry0, RecordGrid rg, float* __restrict__ scratch) {
-    pdl_wait();
-    const int lx = blockIdx.x * blockDim.x + threadIdx.x;
+    int lx = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait(lx);
     if (lx >= rg.w) return;
     const int ly = blockIdx.y, zc = blockIdx.z;
     const int m = g.factor;
@@ -314,7 +314,7 @@ child_avg_kernel(const typename S::T* __restrict__ ff, const std::uint8_t* __res
                 if ((fkind[c] & kFlagMask) == kSolid) continue;
                 ++nFluid;
 #pragma unroll
-                for (int q = 0; q < kQ; ++q) fi[q] += S::ld(ff + q * fn, c, wgt(q));
+                for (int q = 0; q < kQ; ++q) fi[q] += S::template ld<kIndexed>(ff + q * fn, c, wgt(q));
             }
     write_child_record<S>(fi, nFluid, reinterpret_cast<float4*>(scratch) + rg.index(lx, ly, zc),
                           rg.count(g.coarse.nz));
@@ -335,8 +335,8 @@ restrict_kernel(typename S::T* __restrict__ fc, const std::uint8_t* __restrict__
                 RefineGeom g, int rx0, int ry0, RecordGrid rg, float neqScaleInv,
                 const __grid_constant__ RecordPlanes rec, float* __restrict__ mRho,
                 float* __restrict__ mU, float* __restrict__ mV, float* __restrict__ mW) {
-    pdl_wait();
-    const int lx = blockIdx.x * kRestrictTX + threadIdx.x;
+    int lx = blockIdx.x * kRestrictTX + threadIdx.x;
+    pdl_wait(lx);
     const int ly = blockIdx.y * kRestrictTY + threadIdx.y;
     const int zc = blockIdx.z * kRestrictTZ + threadIdx.z;
     const int nz = g.coarse.nz;
@@ -368,11 +368,13 @@ restrict_kernel(typename S::T* __restrict__ fc, const std::uint8_t* __restrict__
     const float4 m4 = ChildRecord<S>::moments(rec, t);
     float feq[kQ];
     feq_rn(m4.x, m4.y, m4.z, m4.w, feq);
+    // The coarse collide, whose result this replaces, ran before the fine
+    // sub-steps: earlier than the launch before this one.
     float b[kQ];
 #pragma unroll
     for (int q = 0; q < kQ; ++q) {
         const float restricted = feq[q] + neqScaleInv * fneq[q];
-        const float existing = S::ld(fc + q * cn, cell, wgt(q));
+        const float existing = S::template ld<kEarlier>(fc + q * cn, cell, wgt(q));
         b[q] = existing + blend * (restricted - existing);
         S::st(fc + q * cn, cell, b[q], wgt(q));
     }

@@ -88,7 +88,7 @@ adam_kernel(const float* __restrict__ partials, int nb, AdamStep a, float invCou
     // launch in between began its work.
     const float m = own ? __ldcg(a.m + p) : 0.0f, v = own ? __ldcg(a.v + p) : 0.0f;
     const float w0 = own ? __ldcg(a.master + p) : 0.0f;
-    pdl_wait();
+    pdl_wait(partials);
     asm volatile("griddepcontrol.launch_dependents;");
     if (p > kParams) return;
     float g = 0.0f;
@@ -152,7 +152,7 @@ grad_kernel(const std::uint16_t* __restrict__ wbf, Norm nm, SampleView S, unsign
         tns[s] = tn;
     };
     if (early && u0 == 0) load_sample();
-    pdl_wait();
+    pdl_wait(wbf);   // and the samples, where they are not read early: the launch is then an ordinary one
     // The next launch may come up now, on the SMs this one leaves idle.
     asm volatile("griddepcontrol.launch_dependents;");
     if (!early && u0 == 0) load_sample();
