@@ -398,11 +398,24 @@ struct fcfd_solver {
     /// Flags of a level from host or device memory: the device copy, the cell
     /// classes, the kind bytes and the force-link list, built on the device.
     cudaError_t uploadLevelFlags(Level& L, const std::uint8_t* flags) {
+        if (auto e = copyLevelFlags(L, flags); e != cudaSuccess) return e;
+        return buildLevelTables(L);
+    }
+
+    /// The device copy alone. A field in device memory may still be under way
+    /// in the legacy default stream, for which a solver on a non-blocking
+    /// stream would not wait by itself.
+    cudaError_t copyLevelFlags(Level& L, const std::uint8_t* flags) {
+        const bool dev = on_device(flags);
+        if (dev)
+            if (auto e = cudaStreamSynchronize(nullptr); e != cudaSuccess) return e;
         if (&L == &coarse) flagsHashValid = false;
-        if (auto e = cudaMemcpyAsync(L.flags, flags, static_cast<size_t>(L.n),
-                                     on_device(flags) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream);
-            e != cudaSuccess)
-            return e;
+        return cudaMemcpyAsync(L.flags, flags, static_cast<size_t>(L.n),
+                               dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream);
+    }
+
+    /// What a level derives from L.flags; waits for the stream.
+    cudaError_t buildLevelTables(Level& L) {
         L.flagsSet = true;
         LevelTables t;
         t.kind = L.kind;
@@ -1132,13 +1145,14 @@ int fcfd_apply_edited_flags(fcfd_solver* s, const uint8_t* flags, size_t n, long
     auto* mask = reinterpret_cast<std::uint8_t*>(work);
     auto* dCount = reinterpret_cast<long long*>(work + tail);
     long long count = 0;
-    cudaError_t e = cudaMemcpyAsync(mask, flags, cells, on_device(flags) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                                    s->stream);
+    // The caller's field is read once: mask and tables come from the same copy.
+    cudaError_t e = s->copyLevelFlags(L, flags);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(mask, L.flags, cells, cudaMemcpyDeviceToDevice, s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(dCount, 0, sizeof(long long), s->stream);
     if (e == cudaSuccess) e = launch_flag_diff(L.kind, mask, L.n, dCount, s->stream);
     ++s->launches;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&count, dCount, sizeof count, cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess) e = s->uploadLevelFlags(L, flags);   // waits for the stream
+    if (e == cudaSuccess) e = s->buildLevelTables(L);   // waits for the stream
     if (e == cudaSuccess && count > 0) {
         ++s->launches;
         e = launch_apply_flag_edits(s->storage, L.f[L.src], L.f[1 - L.src], L.flags, mask, L.d, s->stream);

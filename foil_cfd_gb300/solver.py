@@ -19,7 +19,9 @@ from .capi import ptr
 def _flags_arg(flags):
     """(void* pointer, byte count, keep-alive) of a flag field given as host
     bytes (anything numpy takes) or as a contiguous uint8 CUDA tensor (a
-    field built on the device; the C ABI detects device memory)."""
+    field built on the device; the C ABI detects device memory). The tensor
+    may still be under way in the default stream or the solver's own; one that
+    another stream writes must be complete."""
     if getattr(flags, "is_cuda", False):
         if flags.element_size() != 1 or not flags.is_contiguous():
             raise SolverError("device flag field must be a contiguous uint8 tensor")

@@ -164,7 +164,10 @@ fcfd_solver* fcfd_create(void);
 /* LBMSolver::~LBMSolver + shutdown (lbm_solver.cpp:890, 868). */
 void fcfd_destroy(fcfd_solver* s);
 /* LBMSolver::init (lbm_solver.h:151-154, lbm_solver.cpp:803-887): allocates,
- * uploads flags (n == nx*ny*nz bytes), resets. opts may be NULL. */
+ * uploads flags (n == nx*ny*nz bytes), resets. opts may be NULL.
+ * A flag field in device memory, here and in the other calls that take flags,
+ * is read after all work queued before the call in the solver's stream and in
+ * the legacy default stream; one written in another stream must be complete. */
 int fcfd_init(fcfd_solver* s, const fcfd_dims* dims,
               const fcfd_scaling* scaling, const uint8_t* flags, size_t n,
               void* stream, const fcfd_options* opts, char* err,
