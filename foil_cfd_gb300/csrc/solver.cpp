@@ -141,7 +141,8 @@ struct Level {
     std::uint32_t *dLinkCells = nullptr, *dLinkMasks = nullptr;
     int linkCount = 0;
     long long linkRoom = 0;
-    double* dPartials = nullptr;
+    double* dPartials = nullptr;   // force scratch of partialBytes, its ticket zero between launches
+    size_t partialBytes = 0;
     WMLevel wm;
     // Interpolated bounce-back link field (null when the level has none).
     std::uint8_t* dQFrac = nullptr;
@@ -167,7 +168,7 @@ struct Level {
         qLinks = qFallback = 0;
         wm.free();
         flagsSet = false; surfaceRef.clear();
-        linkCount = 0; linkRoom = 0; src = 0; n = 0; d = LevelDims{};
+        linkCount = 0; linkRoom = 0; partialBytes = 0; src = 0; n = 0; d = LevelDims{};
     }
 };
 
@@ -429,17 +430,18 @@ struct fcfd_solver {
         const cudaError_t te = build_level_tables(L.d, L.flags, t, geomScratch, stream);
         L.dLinkCells = t.linkCells;
         L.dLinkMasks = t.linkMasks;
-        const bool grown = t.linkRoom != L.linkRoom;
         L.linkRoom = t.linkRoom;
         if (te != cudaSuccess) return te;
         L.linkCount = static_cast<int>(t.linkCount);
         L.nReadWrite = t.classes[0]; L.nInlet = t.classes[1]; L.nUntouched = t.classes[2];
         for (int k = 0; k < 4; ++k) L.solidBox[k] = t.box[k];
-        if (grown || !L.dPartials) {
-            const size_t bytes = force_scratch_bytes(static_cast<int>(L.linkRoom));
+        // By its own size, whatever became of the calls that grew the list.
+        if (const size_t bytes = force_scratch_bytes(static_cast<int>(L.linkRoom)); bytes > L.partialBytes) {
             dfree(L.dPartials);
+            L.partialBytes = 0;
             if (auto e = dalloc(&L.dPartials, bytes); e != cudaSuccess) return e;
             if (auto e = cudaMemsetAsync(L.dPartials, 0, bytes, stream); e != cudaSuccess) return e;
+            L.partialBytes = bytes;
         }
         return cudaStreamSynchronize(stream);
     }
