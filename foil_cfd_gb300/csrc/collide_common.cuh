@@ -982,11 +982,13 @@ cudaError_t launch_collide_aa_impl(void* fv, LevelDims d, const CollideParams& p
         return rows ? (odd ? collide_aa_kernel<S, EXACT, true, true, P> : collide_aa_kernel<S, EXACT, false, true, P>)
                     : (odd ? collide_aa_kernel<S, EXACT, true, false, P> : collide_aa_kernel<S, EXACT, false, false, P>);
     };
-    // FP32 in pairs while the lattice is in L2: 40 steps of 1.01 M cells 0.99 ->
-    // 0.88 ms, of 8.4 M cells, from HBM, 8.07 -> 8.30.
+    // FP32 in pairs while the lattice is mostly in L2. 40 steps, ms without and
+    // with: 1.01 M cells 0.99 and 0.88, 1.33 M 1.34 and 1.28, 1.60 M 1.65 and
+    // 1.62, 2.16 M (rows) 2.25 and 2.25, 2.20 M 2.28 and 2.30, 2.74 M 2.78 and
+    // 2.82, 4.49 M 4.46 and 4.57, 8.4 M 8.07 and 8.30.
     auto kern = pick(std::false_type{});
     if constexpr (EXACT)
-        if (a.n < S::kCodedCells) kern = pick(std::true_type{});
+        if (a.n < S::kPairCells) kern = pick(std::true_type{});
     return launch_pdl(kern, grid, dim3(kCellBlockX), st, f, a, off, fast_div(d.nx), fast_div(d.ny));
 }
 

@@ -163,6 +163,8 @@ struct StoreF32 {
     /// per step with and without them, 3.97 M 103 with and 105 without,
     /// 7.78 M 190 and 198; 0.33 M 14.6 and 12.6.
     static constexpr long long kCodedCells = 2500000;
+    /// Cells below which the in-place collide runs in packed pairs (launch_collide_aa_impl).
+    static constexpr long long kPairCells = 1900000;
     /// Resident 128-thread blocks per SM of the batched collide by tiles (12
     /// tunnels: 38.3 ms per 100 steps at 12 blocks, 37.9 at 10, 40.2 at 8).
     static constexpr int kBatchTileMinBlocks = 10;
