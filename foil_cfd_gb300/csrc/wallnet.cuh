@@ -248,33 +248,37 @@ __device__ __forceinline__ double newton64(double ut, double ys, double nu, doub
 }
 
 /// newton64's root without its iteration count: FP32 Newton (accurate
-/// functions) down to its rounding, then steps with the residual in FP64 and
-/// the last FP32 slope, to the same stop. FP32 forms 1 - e11 - (yp / 11) e3 with
-/// an absolute error of some 6e-8, so its root and slope are good to 4e-5 at
-/// y+ = 0.01, 5e-7 from y+ = 1 on (largest of 2e5 samples per decade), and a step
-/// leaves that share of the error before it: the first residual puts the root
-/// within 2e-9, the second meets the 1e-8 stop. Below y+ = 0.01 it would take
-/// three and more (at 1e-5 the FP32 root is off by 3 %, and a tenth of the samples
-/// never stop), and a stop there let one result in 4000 round the other way: that
-/// range is newton64's, and so is a sample that FP32 lost. Bound by FP64, which
-/// has 1/64 of the FP32 rate here: two residuals instead of the four full steps,
-/// 3 M samples in 1.01 ms (newton64: 3.80 ms).
+/// functions) down to its rounding (a step of 2e-6, below y+ = 0.25 of
+/// 5e-7 / y+), then steps with the residual in FP64 and the last FP32 slope, to
+/// the same stop. FP32 forms 1 - e11 - (yp / 11) e3 with an absolute error of some
+/// 6e-8, so its root and slope are good to 4e-5 at y+ = 0.01, 5e-7 from y+ = 1 on
+/// (largest of 2e5 samples per decade), and a step leaves that share of the error
+/// before it: the first residual puts the root within 2e-9, the second meets the
+/// 1e-8 stop. Below y+ = 0.01 it would take three and more (at 1e-5 the FP32 root
+/// is off by 3 %, and a tenth of the samples never stop), and a stop there let one
+/// result in 4000 round the other way: that range is newton64's, and so is a
+/// sample that FP32 lost, or that twelve steps from a poor seed do not settle
+/// (its slope is off by more). Bound by FP64, which has 1/64 of the FP32 rate
+/// here: two residuals instead of the four full steps, 3 M samples in 1.01 ms
+/// (newton64: 3.80 ms).
 constexpr float kShortYplus = 0.01f;
 __device__ __forceinline__ double newton64_short(double ut, double ys, double nu, float seed) {
     const float utf = static_cast<float>(ut), ysf = static_cast<float>(ys), nuf = static_cast<float>(nu);
+    const float rounding = 5e-7f * nuf / ysf;   // 5e-7 / y+ of u
     float u = fmaxf(seed, 1e-30f), dg = 1.0f, yp = 0.0f;
-    for (int it = 0; it < 12; ++it) {
+    bool settled = false;
+    for (int it = 0; it < 12 && !settled; ++it) {
         yp = ysf * u / nuf;
         float up, dup;
         reichardt_acc(yp, up, dup);
         dg = up + yp * dup;
         const float step = (u * up - utf) / dg;
         u = fmaxf(u - step, 0.0f);
-        if (!(fabsf(step) > 2e-6f * u)) break;
+        settled = fabsf(step) <= fmaxf(2e-6f * u, rounding);
     }
     double ud = u;
     const double inv = 1.0 / static_cast<double>(dg);
-    for (int it = 0; it < 4 && yp >= kShortYplus; ++it) {
+    for (int it = 0; it < 4 && settled && yp >= kShortYplus; ++it) {
         const double ypd = ys * ud / nu;
         const double e11 = exp(ypd * (-1.0 / 11.0)), e3 = exp(ypd * (-1.0 / 3.0));
         const double up = log(1.0 + kKappaD * ypd) * (1.0 / kKappaD) + kCD * (1.0 - e11 - ypd * (1.0 / 11.0) * e3);
