@@ -1407,17 +1407,6 @@ StagedPlan staged_plan(LevelDims d) {
     return p;
 }
 
-inline int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 template <class S, bool EXACT>
 cudaError_t launch_collide_impl(const void* srcv, void* dstv, const std::uint8_t* kind, LevelDims d,
                                 const CollideParams& p, float* rho, float* u, float* v, float* w, SlipField slip,

@@ -739,7 +739,7 @@ inline unsigned blocks_of(unsigned long long n, unsigned b) { return static_cast
 /// What the host reads back of a build: one copy.
 struct Readback {
     unsigned long long counts[2];
-    long long total[2];    // of the force-link (or wall candidate) and the shell list
+    long long total[2];    // of the list, and of the wall list among its candidates
     int stats[4];
     int box[4];
 };
@@ -758,19 +758,19 @@ struct Carver {
 struct TableScratch {
     Readback* rb;
     Planes planes{}, clean{};
-    std::uint32_t* sel[2] = {};
-    int* tiles[2] = {};
+    std::uint32_t* sel = nullptr;   // null: no list wanted
+    int* tiles = nullptr;
     /// Lays the parts out at `base` (null: only counts the bytes).
-    size_t lay(char* base, const BitGrid& g, unsigned wanted, bool cleanSolid, int lists) {
+    size_t lay(char* base, const BitGrid& g, unsigned wanted, bool cleanSolid, bool list) {
         Carver c{base};
         rb = c.take<Readback>(1);
         const size_t words = g.total();
         for (int k = 0; k < kPlanes; ++k) planes.p[k] = (wanted >> k & 1u) ? c.take<std::uint32_t>(words) : nullptr;
         clean = Planes{};
         clean.p[kPSolid] = cleanSolid ? c.take<std::uint32_t>(words) : planes.p[kPSolid];
-        for (int k = 0; k < lists; ++k) {
-            sel[k] = c.take<std::uint32_t>(words);
-            tiles[k] = c.take<int>(words / kSelTile + 1);
+        if (list) {
+            sel = c.take<std::uint32_t>(words);
+            tiles = c.take<int>(words / kSelTile + 1);
         }
         return c.used;
     }
@@ -792,15 +792,20 @@ cudaError_t reset_readback(Readback* rb, const BitGrid& g, cudaStream_t st) {
     return cudaMemcpyAsync(rb, &init, sizeof init, cudaMemcpyHostToDevice, st);
 }
 
-template <int OP>
-void select_list(const TableScratch& ts, int list, const BitGrid& g, cudaStream_t st) {
-    const unsigned tiles = blocks_of(g.total(), kSelTile);
-    select_kernel<OP><<<tiles, kSelTile, 0, st>>>(ts.planes, ts.clean, g, ts.sel[list], ts.tiles[list], ts.rb->stats);
-    tile_scan_kernel<<<1, 1024, 0, st>>>(ts.tiles[list], static_cast<int>(tiles), &ts.rb->total[list]);
+void launch_classes(const TableScratch& ts, const BitGrid& g, unsigned long long* counts, cudaStream_t st) {
+    const unsigned nb = min(blocks_of(g.total(), 256), 8u * static_cast<unsigned>(sm_count()));
+    classes_kernel<<<nb, 256, 0, st>>>(ts.planes, g, counts, ts.rb->box);
 }
 
-void scatter_list(const TableScratch& ts, int list, const BitGrid& g, std::uint32_t* cells, cudaStream_t st) {
-    scatter_kernel<<<blocks_of(g.total(), kSelTile), kSelTile, 0, st>>>(ts.sel[list], g, ts.tiles[list], cells);
+template <int OP>
+void select_list(const TableScratch& ts, const BitGrid& g, cudaStream_t st) {
+    const unsigned tiles = blocks_of(g.total(), kSelTile);
+    select_kernel<OP><<<tiles, kSelTile, 0, st>>>(ts.planes, ts.clean, g, ts.sel, ts.tiles, ts.rb->stats);
+    tile_scan_kernel<<<1, 1024, 0, st>>>(ts.tiles, static_cast<int>(tiles), &ts.rb->total[0]);
+}
+
+void scatter_list(const TableScratch& ts, const BitGrid& g, std::uint32_t* cells, cudaStream_t st) {
+    scatter_kernel<<<blocks_of(g.total(), kSelTile), kSelTile, 0, st>>>(ts.sel, g, ts.tiles, cells);
 }
 
 cudaError_t read_back(const TableScratch& ts, Readback& h, cudaStream_t st) {
@@ -914,11 +919,11 @@ cudaError_t device_solid_bbox(LevelDims d, const std::uint8_t* flags, cudaStream
     const BitGrid g = bit_grid(d);
     TableScratch ts;
     CallScratch cs(st);
-    if (auto e = cs.alloc(ts.lay(nullptr, g, bit(kPSolid), false, 0)); e != cudaSuccess) return e;
-    ts.lay(static_cast<char*>(cs.p), g, bit(kPSolid), false, 0);
+    if (auto e = cs.alloc(ts.lay(nullptr, g, bit(kPSolid), false, false)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(cs.p), g, bit(kPSolid), false, false);
     if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
     if (auto e = build_planes(flags, g, ts.planes, st); e != cudaSuccess) return e;
-    classes_kernel<<<min(blocks_of(g.total(), 256), 152u * 8u), 256, 0, st>>>(ts.planes, g, nullptr, ts.rb->box);
+    launch_classes(ts, g, nullptr, st);
     Readback h;
     if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
     for (int k = 0; k < 4; ++k) box[k] = h.box[k];
@@ -932,11 +937,11 @@ cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTabl
     const BitGrid g = bit_grid(d);
     const unsigned wanted = bit(kPSolid) | bit(kPFluid) | bit(kPSlip) | bit(kPInlet) | bit(kPOutlet);
     TableScratch ts;
-    if (auto e = scratch.ensure(ts.lay(nullptr, g, wanted, false, 1)); e != cudaSuccess) return e;
-    ts.lay(static_cast<char*>(scratch.p), g, wanted, false, 1);
+    if (auto e = scratch.ensure(ts.lay(nullptr, g, wanted, false, true)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(scratch.p), g, wanted, false, true);
     if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
     if (auto e = build_planes(flags, g, ts.planes, st, 0x0f0f0f0fu); e != cudaSuccess) return e;
-    classes_kernel<<<min(blocks_of(g.total(), 256), 152u * 8u), 256, 0, st>>>(ts.planes, g, ts.rb->counts, ts.rb->box);
+    launch_classes(ts, g, ts.rb->counts, st);
     const unsigned nb = blocks_of(g.total(), 256);
     const auto a = reinterpret_cast<std::uintptr_t>(flags) | reinterpret_cast<std::uintptr_t>(t.kind);
     if (d.nx % 4 == 0 && a % 4 == 0) classify_kernel<4><<<nb, 256, 0, st>>>(flags, ts.planes, g, t.kind, t.links);
@@ -946,7 +951,7 @@ cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTabl
         tile_codes_kernel<<<blocks_of(nc, 256), 256, 0, st>>>(t.kind, reinterpret_cast<std::uint8_t*>(t.tiles), d.nx,
                                                              d.ny, d.nz, static_cast<unsigned>(n), nc);
     }
-    select_list<kSelForce>(ts, 0, g, st);
+    select_list<kSelForce>(ts, g, st);
     Readback h;
     if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
     t.classes[0] = static_cast<long long>(h.counts[0]);
@@ -970,7 +975,7 @@ cudaError_t build_level_tables(LevelDims d, const std::uint8_t* flags, LevelTabl
     }
     if (t.linkCount > 0) {
         const unsigned m = static_cast<unsigned>(t.linkCount);
-        scatter_list(ts, 0, g, t.linkCells, st);
+        scatter_list(ts, g, t.linkCells, st);
         link_mask_kernel<true><<<blocks_of(m, 128), 128, 0, st>>>(flags, g, t.linkCells, m, t.linkMasks);
     }
     return cudaGetLastError();
@@ -983,12 +988,12 @@ cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, 
     const BitGrid g = bit_grid(d);
     const unsigned wanted = full ? bit(kPInter) : bit(kPInter) | bit(kPFluid) | bit(kPOutlet);
     TableScratch ts;
-    if (auto e = scratch.ensure(ts.lay(nullptr, g, wanted, false, 1)); e != cudaSuccess) return e;
-    ts.lay(static_cast<char*>(scratch.p), g, wanted, false, 1);
+    if (auto e = scratch.ensure(ts.lay(nullptr, g, wanted, false, true)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(scratch.p), g, wanted, false, true);
     if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
     if (auto e = build_planes(flags, g, ts.planes, st); e != cudaSuccess) return e;
-    if (full) select_list<kSelInter>(ts, 0, g, st);
-    else select_list<kSelShell>(ts, 0, g, st);
+    if (full) select_list<kSelInter>(ts, g, st);
+    else select_list<kSelShell>(ts, g, st);
     Readback h;
     if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
     if (!*cells || h.total[0] > *room) {
@@ -999,7 +1004,7 @@ cudaError_t build_shell_list(LevelDims d, const std::uint8_t* flags, bool full, 
         *room = spare(h.total[0]);
     }
     *count = h.total[0];
-    if (h.total[0] > 0) scatter_list(ts, 0, g, *cells, st);
+    if (h.total[0] > 0) scatter_list(ts, g, *cells, st);
     return cudaGetLastError();
 }
 
@@ -1010,17 +1015,17 @@ cudaError_t device_force_links(LevelDims d, const std::uint8_t* flags, std::uint
     const unsigned wanted = bit(kPSolid) | bit(kPFluid);
     TableScratch ts;
     CallScratch cs(st);
-    if (auto e = cs.alloc(ts.lay(nullptr, g, wanted, false, 1)); e != cudaSuccess) return e;
-    ts.lay(static_cast<char*>(cs.p), g, wanted, false, 1);
+    if (auto e = cs.alloc(ts.lay(nullptr, g, wanted, false, true)); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(cs.p), g, wanted, false, true);
     if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
     if (auto e = build_planes(flags, g, ts.planes, st); e != cudaSuccess) return e;
-    select_list<kSelForce>(ts, 0, g, st);
+    select_list<kSelForce>(ts, g, st);
     Readback h;
     if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
     *count = h.total[0];
     if (*count <= 0 || *count > cap) return cudaSuccess;
     const unsigned m = static_cast<unsigned>(*count);
-    scatter_list(ts, 0, g, cells, st);
+    scatter_list(ts, g, cells, st);
     link_mask_kernel<true><<<blocks_of(m, 128), 128, 0, st>>>(flags, g, cells, m, masks);
     if (auto e = cudaGetLastError(); e != cudaSuccess) return e;
     return cudaStreamSynchronize(st);
@@ -1039,13 +1044,13 @@ cudaError_t WallListBuild::find(LevelDims dims, const std::uint8_t* activeF, con
     const bool own = clean && clean != activeF;
     const unsigned wanted = bit(kPSolid) | bit(kPFluid);
     TableScratch ts;
-    if (auto e = cudaMallocAsync(&block, ts.lay(nullptr, g, wanted, own, 1), st); e != cudaSuccess) return e;
-    ts.lay(static_cast<char*>(block), g, wanted, own, 1);
+    if (auto e = cudaMallocAsync(&block, ts.lay(nullptr, g, wanted, own, true), st); e != cudaSuccess) return e;
+    ts.lay(static_cast<char*>(block), g, wanted, own, true);
     if (auto e = reset_readback(ts.rb, g, st); e != cudaSuccess) return e;
     if (auto e = build_planes(activeF, g, ts.planes, st); e != cudaSuccess) return e;
     if (own)
         if (auto e = build_planes(clean, g, ts.clean, st); e != cudaSuccess) return e;
-    select_list<kSelWall>(ts, 0, g, st);
+    select_list<kSelWall>(ts, g, st);
     Readback h;
     if (auto e = read_back(ts, h, st); e != cudaSuccess) return e;
     if (stats) stats[1] = h.stats[1];
@@ -1065,7 +1070,7 @@ cudaError_t WallListBuild::find(LevelDims dims, const std::uint8_t* activeF, con
         }
     }
     solid = ts.clean.p[kPSolid];
-    scatter_list(ts, 0, g, cand, st);
+    scatter_list(ts, g, cand, st);
     link_mask_kernel<false><<<blocks_of(nc, 128), 128, 0, st>>>(activeF, g, cand, nc, masks);
     normal_count_kernel<<<tiles, kSelTile, 0, st>>>(solid, g, cand, nc, offsets, ts.rb->stats);
     tile_scan_kernel<<<1, 1024, 0, st>>>(offsets, static_cast<int>(tiles), &ts.rb->total[1]);

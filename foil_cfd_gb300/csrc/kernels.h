@@ -20,6 +20,18 @@ struct fcfd_wallnet;
 
 namespace fcfd {
 
+/// Multiprocessors of the device, for grids that are persistent or stride.
+inline int sm_count() {
+    static int n = 0;
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 1;
+    }
+    return n;
+}
+
 /// Geometry of one lattice level: unpadded SoA, cell = x + nx*(y + ny*z).
 struct LevelDims {
     int nx = 0, ny = 0, nz = 0;
