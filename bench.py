@@ -38,10 +38,9 @@ DIST = None   # torch.distributed when launched as replicas under torchrun
 # Measured DRAM traffic of the collide kernel over its algorithmic bytes
 # (dram__bytes_read.sum + dram__bytes_write.sum of one coarse and one fine
 # launch without macro output, divided by the class-based algorithmic bytes
-# of those launches): FP32 from the one-pass capture of the full 640x192x192
-# tunnel (profiles/launches_airfoil_640x192x192.md), FP16 from the capture of
-# the 320x96x96 tunnel (profiles/collide_fp16_airfoil.md).
-NCU_TRAFFIC_OVER_ALG = {"fp32": 1.0321, "fp16": 1.0886}
+# of those launches, with FP16 storage two fine ones): one-pass captures of the
+# full 640x192x192 tunnel (profiles/launches_airfoil_640x192x192.md).
+NCU_TRAFFIC_OVER_ALG = {"fp32": 1.0335, "fp16": 1.0675}
 
 
 def peaks():
