@@ -96,16 +96,16 @@ struct RecordGrid {
     __host__ __device__ long long count(int nz) const { return static_cast<long long>(w + 2) * (h + 2) * nz; }
 };
 
-/// Parts of a record, which the launch before wrote: ordinary loads, free to be
-/// scheduled (the kernel had t back from its wait).
+/// Parts of a record, which the launch before wrote: ordinary loads behind the
+/// wait, in the order of the source.
 __device__ __forceinline__ float4 ld_rec(const float4* p) {
     float4 v;
-    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint4 ld_rec(const uint4* p) {
     uint4 v;
-    asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 
@@ -147,12 +147,16 @@ template <> struct ChildRecord<StoreF32> {
         for (int k = 0; k < 4; ++k) rec[k * st] = make_float4(-0.0f, -0.0f, -0.0f, -0.0f);
         rec[4 * st] = make_float4(-0.0f, -0.0f, -0.0f, 0.0f);
     }
+    /// A record's fneq and valid flag as stored.
+    struct Raw { float4 a[5]; };
+    __device__ __forceinline__ static void fetch(const RecordPlanes& r, unsigned t, Raw& w) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) w.a[k] = ld_rec(r.p[k] + t);
+    }
     /// acc[q] += fneq[q], count += valid flag; SET: the record's own values.
     template <bool SET>
-    __device__ __forceinline__ static void add(const RecordPlanes& r, unsigned t, float (&acc)[kQ], float& count) {
-        float4 a[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) a[k] = ld_rec(r.p[k] + t);
+    __device__ __forceinline__ static void add(const Raw& w, float (&acc)[kQ], float& count) {
+        const float4 (&a)[5] = w.a;
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
             const float v[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
@@ -196,11 +200,14 @@ template <> struct ChildRecord<StoreF16> {
         r[st] = make_uint4(z, z, z, z);
         r[2 * st] = make_uint4(z, z, 0u, 0u);
     }
-    template <bool SET>
-    __device__ __forceinline__ static void add(const RecordPlanes& r, unsigned t, float (&acc)[kQ], float& count) {
-        uint4 c[3];
+    struct Raw { uint4 c[3]; };
+    __device__ __forceinline__ static void fetch(const RecordPlanes& r, unsigned t, Raw& w) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) c[k] = ld_rec(reinterpret_cast<const uint4*>(r.p[k]) + t);
+        for (int k = 0; k < 3; ++k) w.c[k] = ld_rec(reinterpret_cast<const uint4*>(r.p[k]) + t);
+    }
+    template <bool SET>
+    __device__ __forceinline__ static void add(const Raw& raw, float (&acc)[kQ], float& count) {
+        const uint4 (&c)[3] = raw.c;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const unsigned w[4] = {c[k].x, c[k].y, c[k].z, c[k].w};
